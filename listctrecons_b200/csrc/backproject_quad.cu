@@ -15,11 +15,11 @@
 // for the sample column (phat/dso, theta*dso/ds) and the texture unit's 8-bit weight rules.
 // EXACT also: floor, fraction and index of a sample from one round-down add (no conversions)
 // and one wide multiply-add for its address; per-view terms staged in shared memory 128 views
-// at a time; a warp-uniform path without out tests, selects or row clamps when a chunk's first
-// and last slices project inside the detector rows, where the view and its conjugate run as
-// packed FP32 pairs (FFMA2 / FADD2: half the instructions for the row, floor, fraction and first
-// two bilinear FMAs of the two samples, each lane rounded as in the scalar form); an L1 prefetch
-// of the next view's tile footprint; a polynomial asin on tiles within dso / 2 of the axis.
+// at a time; the view and its conjugate as packed FP32 pairs (FFMA2 / FADD2: half the
+// instructions for the row, floor, fraction and first two bilinear FMAs of the two samples, each
+// lane rounded as in the scalar form), in a warp-uniform path without out tests, selects or row
+// clamps when a chunk's first and last slices project inside the detector rows; loads that bring
+// the next view's tile footprint into L1; a polynomial asin on tiles within dso / 2 of the axis.
 #include <climits>
 #include <cmath>
 #include <mutex>
@@ -34,6 +34,10 @@ namespace lct {
 // tile 16 x 16 voxel columns (warps of 16 x 2): its footprint on the detector, |16 cos| + |16 sin|
 // voxels wide, averages 20% narrower over the views than a 32 x 8 tile's; kQVB views staged per batch
 constexpr int kQTX = 16, kQTY = 16, kQVB = 128;
+// slices per group on a partly filled window (EXACT): a view that only some of the thread's
+// slices use runs the groups that hold one of them.  512^2 x 256 from 736 x 64 views, where 37% of
+// the view iterations are partial: 2 slices 64.5 ms, 4 70.0, 8 74.1, 1 92.8.
+constexpr int kQGroup = 2;
 
 // cos/sin of a view angle in FP64 rounded to float (sincospi: no large-argument reduction)
 __device__ __forceinline__ void view_trig_pi(const float* __restrict__ betas, int v, float& c,
@@ -372,17 +376,22 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
     for (int k = 0; k < nv; ++k) {
       const int ia = vb + k;
       if (INTERP == LCT_INTERP_EXACT && k + 1 < nv) {
-        // the next view's footprint into L1 while this one is sampled (a hint: no result depends
-        // on it, and every address lies inside that view's quads)
-        const int pf_conj = tid >> 7, pf_row = (tid >> 3) & 15, pf_line = tid & 7;
+        // the next view's footprint into L1 while this one is sampled (no result depends on it,
+        // and every address lies inside that view's quads).  One 4-byte load per 32-byte sector,
+        // its value unused: a load brings in the sector it touches, and a prefetch instruction
+        // does no better per sector and costs more (512^2 x 256 from 736 x 64 views: 64.5 ms so,
+        // 70.8 ms with one prefetch.global.L1 per 128-byte line, slower with one per sector).
+        const int pf_conj = tid >> 7, pf_col = 2 * (tid & 15);
         const int4 sz = s_pfs[k + 1];
         const int rows = pf_conj ? sz.z : sz.x, cspan = pf_conj ? sz.w : sz.y;
-        if (pf_row < rows && 8 * pf_line <= cspan + 7) {
+        if (pf_col <= cspan + 1) {
           const ulonglong2 bs = s_pfb[k + 1];
-          const unsigned long long a = (pf_conj ? bs.y : bs.x) +
-                                       (unsigned long long)pf_row * A.qrow_bytes +
-                                       16ull * (unsigned)min(8 * pf_line, cspan);
-          asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
+          unsigned long long a = (pf_conj ? bs.y : bs.x) + 16ull * (unsigned)min(pf_col, cspan) +
+                                 (unsigned long long)((tid >> 4) & 7) * A.qrow_bytes;
+          for (int r = (tid >> 4) & 7; r < rows; r += 8, a += 8ull * A.qrow_bytes) {
+            unsigned unused;
+            asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(unused) : "l"(a));
+          }
         }
       }
       const int2 jr = s_jr[k];
@@ -426,61 +435,70 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         float a1, a2;
         const unsigned long long q1 = quad_col_exact(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
         const unsigned long long q2 = quad_col_exact(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
-        // INSIDE: both samples of every slice lie within the detector rows (no tests, no selects)
-        auto slice_x = [&](int j, auto inside) {
-          const float fj = (float)j;
-          const float qh1 = fmaf(fj, kd1, h1), qh2 = fmaf(fj, kd2, h2);
+        const float2 KD = make_float2(kd1, kd2), H = make_float2(h1, h2), U = make_float2(u1, u2);
+        const float2 A1 = f2(a1), A2 = f2(a2);
+        // one slice of the pair, the view and its conjugate as one packed FP32 pair; INSIDE: both
+        // samples lie within the detector rows (no tests, no selects, no row clamps).  A slice
+        // whose window does not hold the view is evaluated with its group and not added.
+        auto slice_x = [&](int j, auto inside, bool add) {
+          const float2 J = f2((float)j);
+          const float2 qh = __ffma2_rn(J, KD, H);
           // the pair weights sum to one in every case -- (-qh2, qh1) / (qh1 - qh2), (0, 1),
           // (1, 0), (1/2, 1/2) -- so w1 s1 + w2 s2 = s2 + w1 (s1 - s2)
-          const float in1 = -qh2 * __fdividef(1.0f, qh1 - qh2);
+          const float in1 = -qh.y * __fdividef(1.0f, qh.x - qh.y);
           float w1 = in1;
+          const float2 u = __ffma2_rn(J, KD, U);
+          const float2 t = __fadd2_rd(u, f2(kMagic));
+          const float2 b = f2sub(u, __fadd2_rn(t, f2(-kMagic)));
+          int r1 = __float_as_int(t.x), r2 = __float_as_int(t.y);
           if constexpr (!decltype(inside)::value) {
-            const bool out1 = fabsf(qh1) > wt, out2 = fabsf(qh2) > wt;
+            const bool out1 = fabsf(qh.x) > wt, out2 = fabsf(qh.y) > wt;
             w1 = out1 ? (out2 ? 0.5f : 0.0f) : (out2 ? 1.0f : in1);
+            r1 = min(max(r1, kMagicBits), kMagicBits + A.nt + 2);
+            r2 = min(max(r2, kMagicBits), kMagicBits + A.nt + 2);
           }
-          constexpr bool kClamp = !decltype(inside)::value;
-          const float s1 = quad_sample_exact<kClamp>(q1, A.qrow_bytes, A.nt, a1, fmaf(fj, kd1, u1));
-          const float s2 = quad_sample_exact<kClamp>(q2, A.qrow_bytes, A.nt, a2, fmaf(fj, kd2, u2));
-          acc[j] = fmaf(w1, s1 - s2, acc[j] + s2);
+          const float4 v0 = __ldg(reinterpret_cast<const float4*>(
+              q1 + (unsigned long long)(unsigned)r1 * A.qrow_bytes));  // T00, dy, dx, dxy
+          const float4 v1 = __ldg(reinterpret_cast<const float4*>(
+              q2 + (unsigned long long)(unsigned)r2 * A.qrow_bytes));
+          const float2 p0 = __ffma2_rn(A1, make_float2(v0.z, v0.w), make_float2(v0.x, v0.y));
+          const float2 p1 = __ffma2_rn(A2, make_float2(v1.z, v1.w), make_float2(v1.x, v1.y));
+          const float s1 = fmaf(b.x, p0.y, p0.x), s2 = fmaf(b.y, p1.y, p1.x);
+          const float sum = fmaf(w1, s1 - s2, acc[j] + s2);
+          if (add) acc[j] = sum;
         };
-        // qhat(j) = fmaf(j, kd, h) is monotone in j (monotone rounding of a linear function),
-        // so the chunk's first and last slices bound every |qhat|: when both are inside for both
-        // views in every lane of the warp, every out test of the chunk is false and the selects
-        // are skipped with no change to any result.  The row coordinate u = qhat + wt + 2 (equal
-        // to within a few ulps, far below half a row) then lies in (1.5, 2 wt + 2.5), inside the
-        // quad rows when rows_inside_ok.  Plain comparisons: a NaN fails them.
-        bool inside = false;
-        if (jlo == 0 && jhi == NZ) {
-          const float e1 = fmaf((float)(NZ - 1), kd1, h1), e2 = fmaf((float)(NZ - 1), kd2, h2);
-          inside = A.rows_inside_ok && fabsf(h1) <= wt && fabsf(e1) <= wt &&
-                   fabsf(h2) <= wt && fabsf(e2) <= wt;
-        }
+        // qhat(j) = fmaf(j, kd, h) is monotone in j (monotone rounding of a linear function), so
+        // the first and last slices of the groups that run bound every |qhat|: when both are
+        // inside for both views in every lane of the warp, every out test is false and the tests,
+        // selects and clamps are skipped with no change to any result.  The row coordinate
+        // u = qhat + wt + 2 (equal to within a few ulps, far below half a row) then lies in
+        // (1.5, 2 wt + 2.5), inside the quad rows when rows_inside_ok.  A NaN fails the test.
+        // (69.4 ms with scalar code and no inside path on partial windows, 64.5 ms so.)
+        const float jf = (float)(jlo & ~(kQGroup - 1));
+        const float jl = (float)(((jhi + kQGroup - 1) & ~(kQGroup - 1)) - 1);
+        const bool inside = A.rows_inside_ok && fabsf(fmaf(jf, kd1, h1)) <= wt &&
+                            fabsf(fmaf(jl, kd1, h1)) <= wt && fabsf(fmaf(jf, kd2, h2)) <= wt &&
+                            fabsf(fmaf(jl, kd2, h2)) <= wt;
         if (__all_sync(0xffffffffu, inside)) {
-          // the two views of the pair as one packed FP32 pair per slice: each lane is
-          // slice_x(j, inside) rounded the same way
-          const float2 KD = make_float2(kd1, kd2), H = make_float2(h1, h2), U = make_float2(u1, u2);
-          const float2 A1 = f2(a1), A2 = f2(a2);
+          if (jlo == 0 && jhi == NZ) {  // straight code: every load of the chunk may be in flight
 #pragma unroll
-          for (int j = 0; j < NZ; ++j) {
-            const float2 J = f2((float)j);
-            const float2 qh = __ffma2_rn(J, KD, H);
-            const float w1 = -qh.y * __fdividef(1.0f, qh.x - qh.y);
-            const float2 u = __ffma2_rn(J, KD, U);
-            const float2 t = __fadd2_rd(u, f2(kMagic));
-            const float2 b = f2sub(u, __fadd2_rn(t, f2(-kMagic)));
-            const float4 v0 = __ldg(reinterpret_cast<const float4*>(
-                q1 + (unsigned long long)(unsigned)__float_as_int(t.x) * A.qrow_bytes));
-            const float4 v1 = __ldg(reinterpret_cast<const float4*>(
-                q2 + (unsigned long long)(unsigned)__float_as_int(t.y) * A.qrow_bytes));
-            const float2 p0 = __ffma2_rn(A1, make_float2(v0.z, v0.w), make_float2(v0.x, v0.y));
-            const float2 p1 = __ffma2_rn(A2, make_float2(v1.z, v1.w), make_float2(v1.x, v1.y));
-            const float s1 = fmaf(b.x, p0.y, p0.x), s2 = fmaf(b.y, p1.y, p1.x);
-            acc[j] = fmaf(w1, s1 - s2, acc[j] + s2);
+            for (int j = 0; j < NZ; ++j) slice_x(j, std::true_type{}, true);
+          } else
+#pragma unroll
+          for (int g = 0; g < NZ; g += kQGroup) {
+            if (jlo < g + kQGroup && jhi > g) {
+#pragma unroll
+              for (int j = g; j < g + kQGroup; ++j) slice_x(j, std::true_type{}, j >= jlo && j < jhi);
+            }
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < NZ; ++j)
-            if (j >= jlo && j < jhi) slice_x(j, std::false_type{});
+          for (int g = 0; g < NZ; g += kQGroup) {
+            if (jlo < g + kQGroup && jhi > g) {
+#pragma unroll
+              for (int j = g; j < g + kQGroup; ++j) slice_x(j, std::false_type{}, j >= jlo && j < jhi);
+            }
+          }
         }
         continue;
       }
