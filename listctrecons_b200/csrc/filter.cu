@@ -3,13 +3,13 @@
 // The reference convolves each detector row with 2*ns taps, out[is] = sum_{k<ns}
 // h[is-k+ns] * row[k] (CUDA/Filter.cu:42-46), i.e. out = row * T with the Toeplitz matrix
 // T[k][is] = h[is-k+ns].  LCT_FILTER_FP32 keeps that sum's order (FP32 FMA, k increasing) so
-// results are bit-exact with the reference kernel; it tiles R rows per CTA so each tap read
-// from shared memory feeds R FMAs.  LCT_FILTER_BF16X3 runs the same product as a GEMM on the
+// results are bit-exact with the reference kernel.  LCT_FILTER_BF16X3 runs the same product as a GEMM on the
 // tensor cores (filter_tc.cu).
 #include <cmath>
-#include <vector>
+#include <mutex>
 
 #include "lct_internal.h"
+#include "tc_ptx.cuh"
 
 namespace lct {
 
@@ -85,79 +85,164 @@ LCT_API int lct_filter_taps(int kind, int window, int ns, float ds, float* h) {
 namespace lct {
 
 // ---------------------------------------------------------------------------------------
-// FP32 convolution in the reference's order.  CTA = R rows x all ns outputs; thread `is`
-// keeps R accumulators; taps and rows staged in shared memory (rows read as float4
-// broadcasts).
+// FP32 convolution in the reference's order.  Bound: the FP32 FMA pipe, so the operands have to
+// come cheaply: shared memory returns 128 bytes per clock and SM, a quarter of what 128 FMA lanes
+// would ask for if every FMA loaded one operand.  A thread therefore makes a tile of 8 rows x 8
+// consecutive outputs: per k it loads the 8 rows' samples (two 16-byte broadcasts of the rows
+// interleaved [k][row]) and ONE tap -- output j at k + 1 uses output j - 1's tap at k, so the
+// other seven stay in registers (a ring of eight, its positions fixed by unrolling k by 8) -- for
+// 64 FMAs, issued as 32 packed FP32 pairs of two rows (each lane rounded as a scalar fmaf, k
+// increasing: bit-exact with the reference's sum).
+// Taps are padded by one word in nine so that lanes 8 outputs apart fall on different banks.
+// 56,128 rows of 672 (with their rebin): 1.03 ms, 2.18 ms with 16 rows x 1 output per thread, which
+// asked shared memory for 17 words per 16 FMAs (23 of the chip's 74 TFLOP/s).
 // ---------------------------------------------------------------------------------------
-constexpr int kFiltRows = 16;
-constexpr int kFiltThreads = 256;
+constexpr int kFiltR = 8;         // rows per thread, and per row group in shared memory
+constexpr int kFiltC = 8;         // outputs per thread
+constexpr int kFiltBlk = 8 * kFiltR + 4;  // words of 8 k: padded, so that staging stores spread over the banks
+constexpr int kFiltThreads = 256; // most threads of a CTA
 
-__host__ __device__ __forceinline__ int filt_rows_offset(int ns) { return (2 * ns + 8 + 3) / 4 * 4; }
+// front padding that puts tap index ns on a multiple of 8, and the padded taps' words
+__host__ __device__ __forceinline__ int filt_front(int ns) { return 8 + (8 - (ns & 7)) % 8; }
+__host__ __device__ __forceinline__ int filt_tap_words(int ns) {
+  return ((filt_front(ns) + 2 * ns + 8) * 9 / 8 + 8) / 4 * 4;
+}
 
-__global__ void __launch_bounds__(kFiltThreads) filter_fp32_kernel(const float* __restrict__ h,
-                                                                   float* __restrict__ rows,
-                                                                   long long nrows, int ns,
-                                                                   int nsp) {
+// grid ceil(row groups / rg); CTA: rg groups of 8 rows x all ns outputs, thread items
+// (row group, 8 outputs) flattened so that a warp may hold two row groups' ends
+__global__ void __launch_bounds__(kFiltThreads, 2)
+    filter_fp32_kernel(const float* __restrict__ h, float* __restrict__ rows, long long nrows, int ns,
+                       int rg) {
   extern __shared__ __align__(16) float sm[];
-  float* s_h = sm;  // 2*ns taps with 4 zero pads either side (indices down to -3)
-  // rows start on a 16-byte boundary (float4 reads): offset rounded up to 4 floats
-  float* s_r = sm + filt_rows_offset(ns);  // kFiltRows x nsp, zero padded to nsp (multiple of 4)
-  const long long r0 = (long long)blockIdx.x * kFiltRows;
-  for (int i = threadIdx.x; i < 2 * ns + 8; i += blockDim.x) {
-    int k = i - 4;
-    s_h[i] = (k >= 0 && k < 2 * ns) ? h[k] : 0.0f;
+  const int front = filt_front(ns);
+  float* s_h = sm;                        // tap i at (i + front) * 9 / 8
+  float* s_r = sm + filt_tap_words(ns);   // [rg][ns / 8][8 k][8 rows] + 4 words per 8 k
+  const long long r0 = (long long)blockIdx.x * rg * kFiltR;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < front + 2 * ns + 8; i += blockDim.x) {
+    const int k = i - front;
+    s_h[i + (i >> 3)] = (k >= 0 && k < 2 * ns) ? h[k] : 0.0f;
   }
-  for (int r = 0; r < kFiltRows; ++r) {
-    const bool ok = r0 + r < nrows;
-    for (int k = threadIdx.x; k < nsp; k += blockDim.x)
-      s_r[r * nsp + k] = (ok && k < ns) ? rows[(r0 + r) * ns + k] : 0.0f;
+  // asynchronous 4-byte copies (transposing, all in flight at once: a small CTA would otherwise
+  // wait for its loads in turn); rows past the end are zero-filled
+  const int nsb = (ns + 7) / 8;
+  for (int r = 0; r < rg * kFiltR; ++r) {
+    const unsigned bytes = r0 + r < nrows ? 4u : 0u;
+    const float* src = rows + (bytes ? r0 + r : r0) * ns;
+    const uint32_t dst = smem_u32(s_r + (r / kFiltR) * nsb * kFiltBlk + r % kFiltR);
+#pragma unroll 4
+    for (int k = threadIdx.x; k < ns; k += blockDim.x)
+      cp_async4(dst + 4u * ((k >> 3) * kFiltBlk + (k & 7) * kFiltR), src + k, bytes);
   }
+  cp_async_wait_all();
   __syncthreads();
-  const float* hs = s_h + 4;
-  for (int is = threadIdx.x; is < ns; is += blockDim.x) {
-    float acc[kFiltRows];
+  const int groups = (ns + kFiltC - 1) / kFiltC;
+  const bool vec = (ns & 3) == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
+  for (int item = threadIdx.x; item < groups * rg; item += blockDim.x) {
+    const int gr = item / groups, cg = item - gr * groups;
+    const float* x = s_r + gr * nsb * kFiltBlk;
+    const float* t = s_h + cg * 9 + (ns + front) / 8 * 9;  // tap of output 0 at k = 0
+    float2 acc[kFiltC][kFiltR / 2];
 #pragma unroll
-    for (int r = 0; r < kFiltRows; ++r) acc[r] = 0.0f;
-    for (int k = 0; k < nsp; k += 4) {
-      // padded columns k >= ns carry row value 0 and leave acc unchanged
-      const float h0 = hs[is - k + ns], h1 = hs[is - k - 1 + ns];
-      const float h2 = hs[is - k - 2 + ns], h3 = hs[is - k - 3 + ns];
+    for (int j = 0; j < kFiltC; ++j)
 #pragma unroll
-      for (int r = 0; r < kFiltRows; ++r) {
-        const float4 v = *reinterpret_cast<const float4*>(s_r + r * nsp + k);
-        acc[r] = fmaf(h0, v.x, acc[r]);
-        acc[r] = fmaf(h1, v.y, acc[r]);
-        acc[r] = fmaf(h2, v.z, acc[r]);
-        acc[r] = fmaf(h3, v.w, acc[r]);
-      }
+      for (int q = 0; q < kFiltR / 2; ++q) acc[j][q] = make_float2(0.0f, 0.0f);
+    float2 ring[8];  // (tap, tap): output j at k = k0 + u in ring[(j - u) & 7]
+#pragma unroll
+    for (int j = 1; j < 8; ++j) ring[j] = make_float2(t[j], t[j]);
+    auto step = [&](int u) {  // u = k mod 8, a constant after unrolling
+      const float tap = u == 0 ? t[0] : t[-u - 1];
+      ring[(8 - u) & 7] = make_float2(tap, tap);
+      const float4 a = *reinterpret_cast<const float4*>(x + u * kFiltR);
+      const float4 b = *reinterpret_cast<const float4*>(x + u * kFiltR + 4);
+      const float2 v[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y),
+                           make_float2(b.z, b.w)};
+#pragma unroll
+      for (int j = 0; j < kFiltC; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[j][q] = __ffma2_rn(ring[(j - u) & 7], v[q], acc[j][q]);
+    };
+    int k = 0;
+    for (; k + 8 <= ns; k += 8) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) step(u);
+      t -= 9;
+      x += kFiltBlk;
     }
 #pragma unroll
-    for (int r = 0; r < kFiltRows; ++r)
-      if (r0 + r < nrows) rows[(r0 + r) * ns + is] = acc[r];
+    for (int u = 0; u < 7; ++u)
+      if (k + u < ns) step(u);
+    const int is0 = cg * kFiltC;
+#pragma unroll
+    for (int r = 0; r < kFiltR; ++r) {
+      const long long row = r0 + gr * kFiltR + r;
+      if (row >= nrows) break;
+      float* o = rows + row * ns + is0;
+      float y[kFiltC];
+#pragma unroll
+      for (int j = 0; j < kFiltC; ++j) y[j] = (r & 1) ? acc[j][r / 2].y : acc[j][r / 2].x;
+      if (vec && is0 + kFiltC <= ns) {
+        *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
+        *reinterpret_cast<float4*>(o + 4) = make_float4(y[4], y[5], y[6], y[7]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kFiltC; ++j)
+          if (is0 + j < ns) o[j] = y[j];
+      }
+    }
   }
 }
 
+// Row groups per CTA: the fewest warps on the busiest SM, counting the lanes that the last warp of
+// a CTA leaves idle; ties to the smaller CTA.
+static int filt_row_groups(long long row_groups, int ns, int sms, size_t* smem) {
+  const int groups = (ns + kFiltC - 1) / kFiltC;
+  int best = 1;
+  long long best_cost = 0;
+  for (int rg = 1; rg == 1 || (groups * rg <= kFiltThreads && rg <= 32); ++rg) {
+    const size_t b = sizeof(float) * (filt_tap_words(ns) + (size_t)rg * ((ns + 7) / 8) * kFiltBlk);
+    if (rg > 1 && b > 96 * 1024) break;
+    const long long ctas = (row_groups + rg - 1) / rg;
+    const long long cost = (ctas + sms - 1) / sms * ((groups * rg + 31) / 32);
+    if (rg == 1 || cost < best_cost) {
+      best = rg;
+      best_cost = cost;
+      *smem = b;
+    }
+  }
+  return best;
+}
 
 int launch_filter_rows(int ns, const float* d_h, float* d_rows, long long nrows, int mode,
                        cudaStream_t s) {
   if (nrows <= 0) return LCT_OK;
   if (mode == LCT_FILTER_BF16X3 || mode == LCT_FILTER_BF16X6)
     return launch_filter_tc(ns, d_h, d_rows, nrows, mode, s);
-  const int nsp = (ns + 3) / 4 * 4;
-  const size_t smem = sizeof(float) * (filt_rows_offset(ns) + (size_t)kFiltRows * nsp);
-  static bool attr_set[64] = {false};
-  int dev = 0;
+  static std::mutex mu;
+  static int sms_of[64] = {0};  // 0: attribute not set yet on that device
+  int dev = 0, sms = 148;
   cudaGetDevice(&dev);
-  if (smem > 48 * 1024 && dev < 64 && !attr_set[dev]) {
-    int st = cuda_status(cudaFuncSetAttribute(filter_fp32_kernel,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              227 * 1024));
-    if (st) return st;
-    attr_set[dev] = true;
+  {
+    std::lock_guard<std::mutex> lock(mu);  // host threads may share a device
+    if (dev >= 64 || !sms_of[dev]) {
+      int st = cuda_status(cudaFuncSetAttribute(filter_fp32_kernel,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                200 * 1024));
+      if (!st) st = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      if (st) return st;
+      if (dev < 64) sms_of[dev] = sms;
+    } else {
+      sms = sms_of[dev];
+    }
   }
-  const long long nblk = (nrows + kFiltRows - 1) / kFiltRows;
+  const long long row_groups = (nrows + kFiltR - 1) / kFiltR;
+  size_t smem = 0;
+  const int rg = filt_row_groups(row_groups, ns, sms, &smem);
+  const long long nblk = (row_groups + rg - 1) / rg;
   if (nblk > 0x7fffffffLL) return LCT_ERR_ARG;
-  filter_fp32_kernel<<<(unsigned)nblk, kFiltThreads, smem, s>>>(d_h, d_rows, nrows, ns, nsp);
+  const int items = (ns + kFiltC - 1) / kFiltC * rg;
+  const int threads = std::min(kFiltThreads, (items + 31) / 32 * 32);
+  filter_fp32_kernel<<<(unsigned)nblk, threads, smem, s>>>(d_h, d_rows, nrows, ns, rg);
   return launch_status();
 }
 
