@@ -605,7 +605,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
     float4* q = nullptr;
     const size_t bytes = sizeof(float4) * (size_t)g->n_angle * quad_view_elems(g->ns, g->nt);
     if ((st = cuda_status(cudaMallocAsync((void**)&q, bytes, s)))) return LCT_ERR_ALLOC;
-    st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, q, s);
+    st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, interp, q, s);
     if (!st) {
       BpLaunch L;
       L.proj = d_proj;
@@ -619,7 +619,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
       L.slab_z0[0] = 0;
       L.interp = interp;
       L.addr = addr;
-      L.nz_thread = 8;
+      L.nz_thread = bp_nz_default(*g, *ig);
       st = launch_bp_par_quads(*g, *ig, L, q, s);
     }
     int st2 = cuda_status(cudaFreeAsync(q, s));

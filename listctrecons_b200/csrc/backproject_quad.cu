@@ -12,8 +12,11 @@
 //   * the pair weights are branch-free selects around one reciprocal;
 //   * views whose window covers every slice of the thread's chunk run an unpredicated loop.
 // EXACT keeps FP64 view trigonometry and full FP32 weights; TEX8 keeps the reference's order
-// for the sample column (phat/dso, theta*dso/ds) and the texture unit's 8-bit weight rules.
-// EXACT also: floor, fraction and index of a sample from one round-down add (no conversions)
+// for the sample column (phat/dso, theta*dso/ds) and the texture unit's 8-bit weight rules, bit
+// for bit, in the same packed path: divisions by launch constants as three FMAs, 8-bit weights as
+// whole numbers from round-down adds (256^2 x 32 from 672 x 16 views: 4.17 ms, 5.13 ms in scalar
+// code with IEEE divisions, FRND and F2I).
+// Both: floor, fraction and index of a sample from one round-down add (no conversions)
 // and one wide multiply-add for its address; per-view terms staged in shared memory 128 views
 // at a time; the view and its conjugate as packed FP32 pairs (FFMA2 / FADD2: half the
 // instructions for the row, floor, fraction and first two bilinear FMAs of the two samples, each
@@ -37,7 +40,8 @@ constexpr int kQTX = 16, kQTY = 16, kQVB = 128;
 // slices per group on a partly filled window (EXACT): a view that only some of the thread's
 // slices use runs the groups that hold one of them.  512^2 x 256 from 736 x 64 views, where 37% of
 // the view iterations are partial: 2 slices 64.5 ms, 4 70.0, 8 74.1, 1 92.8.
-constexpr int kQGroup = 2;
+template <int NZ>
+constexpr int kQGroupOf = NZ < 2 ? NZ : 2;
 
 // cos/sin of a view angle in FP64 rounded to float (sincospi: no large-argument reduction)
 __device__ __forceinline__ void view_trig_pi(const float* __restrict__ betas, int v, float& c,
@@ -70,7 +74,7 @@ struct BpQuadArgs {
   long long qstride;    // float4 per view
   int qcols;            // ns + 3
   int ns, nt, n_angle, nx, ny, nz;
-  float ws, wt, ds, dso, dso2, inv_dso, dso_over_ds, orbit, inv_orbit, z0, dzv, kq;
+  float ws, wt, ds, inv_ds, dso, dso2, inv_dso, dso_over_ds, orbit, inv_orbit, z0, dzv, kq;
   float wx, wy, wz, dx, dy, dz;
   int half;
   int zchunks;
@@ -86,7 +90,9 @@ struct BpQuadArgs {
 
 // quad pack: grid (views, nt + 3), block 256 over the ns + 3 quad columns; view v goes to slot
 // (vbase + v) mod ring of a ring of quads (ring > 0), else to view v
-template <int ADDR>
+// TEX8: the row differences carry a factor 2^-8 (exact), so the samples' 8-bit row weights stay
+// whole numbers
+template <int ADDR, int INTERP>
 __global__ void __launch_bounds__(256) quad_pack_kernel(const float* __restrict__ rows, int ns,
                                                         int nt, float4* __restrict__ quads,
                                                         long long vbase, long long ring) {
@@ -110,20 +116,26 @@ __global__ void __launch_bounds__(256) quad_pack_kernel(const float* __restrict_
                 t11 = texel(j + 1, i + 1);
     // differences {T00, dy, dx, dxy}: a bilinear sample is then T00 + a dx + b (dy + a dxy), the
     // pair (T00, dy) + a (dx, dxy) one packed FMA
-    out[q] = make_float4(t00, t10 - t00, t01 - t00, (t11 - t10) - (t01 - t00));
+    constexpr float kRow = INTERP == LCT_INTERP_TEX8 ? 1.0f / 256.0f : 1.0f;
+    out[q] = make_float4(t00, kRow * (t10 - t00), t01 - t00, kRow * ((t11 - t10) - (t01 - t00)));
   }
 }
 
-int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, float4* quads,
-                     cudaStream_t s, long long vbase, long long ring) {
+int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, int interp,
+                     float4* quads, cudaStream_t s, long long vbase, long long ring) {
   if (views <= 0) return LCT_OK;
   if (views > 0x7fffffffLL || nt + 3 > 65535 || vbase < 0 || ring < 0) return LCT_ERR_ARG;
   if (ring > 0 && views > ring) return LCT_ERR_ARG;  // a piece would overwrite itself
   dim3 grid((unsigned)views, nt + 3);
-  if (addr == LCT_ADDR_CLAMP)
-    quad_pack_kernel<LCT_ADDR_CLAMP><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
+  const bool tex = interp == LCT_INTERP_TEX8, clamp = addr == LCT_ADDR_CLAMP;
+  if (tex && clamp)
+    quad_pack_kernel<LCT_ADDR_CLAMP, LCT_INTERP_TEX8><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
+  else if (tex)
+    quad_pack_kernel<LCT_ADDR_BORDER, LCT_INTERP_TEX8><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
+  else if (clamp)
+    quad_pack_kernel<LCT_ADDR_CLAMP, LCT_INTERP_EXACT><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
   else
-    quad_pack_kernel<LCT_ADDR_BORDER><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
+    quad_pack_kernel<LCT_ADDR_BORDER, LCT_INTERP_EXACT><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
   return launch_status();
 }
 
@@ -134,31 +146,6 @@ __device__ __forceinline__ const float4* quad_view_ptr(const BpQuadArgs& A, int 
   return A.quads + v * A.qstride;
 }
 
-// Bilinear sample at origin column already applied to qb (qb = view base + clamped column);
-// q_idx is the row coordinate in texel units (texel centres at integers).
-template <int INTERP>
-__device__ __forceinline__ float quad_sample(const float4* __restrict__ qb, int qcols, int nt,
-                                             float a, float q_idx) {
-  float yb;
-  if (INTERP == LCT_INTERP_TEX8)
-    yb = __fsub_rn(__fadd_rn(q_idx, 0.5f), 0.5f);  // the reference's texture coordinate
-  else
-    yb = q_idx;
-  const float fy = floorf(yb);
-  float b = yb - fy;
-  int j = (int)fy;
-  j = min(max(j, -2), nt);
-  const float4 v = __ldg(qb + (j + 2) * qcols);  // T00, dy, dx, dxy
-  if (INTERP == LCT_INTERP_TEX8) {
-    // texture unit: w01 = a - w11, w10 = b - w11, w00 = 1 - a - b + w11, so the sample is
-    // T00 + a dx + b dy + w11 dxy with w11 = round-half-up(a b) on the 1/256 grid
-    b = q8(b);
-    const float w11 = floorf(a * b * 256.0f + 0.5f) * (1.0f / 256.0f);
-    return fmaf(w11, v.w, fmaf(b, v.y, fmaf(a, v.z, v.x)));
-  }
-  return fmaf(b, fmaf(a, v.w, v.y), fmaf(a, v.z, v.x));
-}
-
 // EXACT floor without conversions: for |x| < 2^22, x + 1.5 * 2^23 rounded toward -inf is
 // 1.5 * 2^23 + floor(x) exactly, so its bit pattern is kMagicBits + floor(x) and subtracting the
 // constant back (exact: both operands lie within a factor of two) gives floor(x).  Outside that
@@ -167,26 +154,14 @@ constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
 
 // view base biased so that a column bit pattern (clamped to kMagicBits + [-2, ns]) times 16 and a
-// row bit pattern (clamped to kMagicBits + [0, nt + 2]) times the row pitch add up to the quad's
-// address: one wide multiply-add per sample
+// row bit pattern times the row pitch add up to the quad's address, one wide multiply-add per
+// sample; rows are clamped to kMagicBits + [0, nt + 2]
+// (EXACT, whose row coordinate carries + 2) or kMagicBits + [-2, nt] (TEX8)
+template <int INTERP>
 __device__ __forceinline__ unsigned long long quad_view_bias(const float4* view, unsigned qrow_bytes) {
+  constexpr int kRow0 = INTERP == LCT_INTERP_TEX8 ? kMagicBits - 2 : kMagicBits;
   return reinterpret_cast<unsigned long long>(view) - (unsigned long long)(kMagicBits - 2) * 16ull -
-         (unsigned long long)kMagicBits * qrow_bytes;
-}
-
-// EXACT sample: u = row coordinate + 2 (texel centres at integers), so floor(u) is the quad row;
-// col = quad_view_bias(view) + 16 * (column bit pattern).  CLAMP false: the caller has shown
-// that 1 <= u < nt + 3 (rows inside the detector), so the row needs no clamp.
-template <bool CLAMP>
-__device__ __forceinline__ float quad_sample_exact(unsigned long long col, unsigned qrow_bytes,
-                                                   int nt, float a, float u) {
-  const float t = __fadd_rd(u, kMagic);
-  const float b = u - (t - kMagic);
-  int rb = __float_as_int(t);
-  if (CLAMP) rb = min(max(rb, kMagicBits), kMagicBits + nt + 2);
-  const float4 v = __ldg(reinterpret_cast<const float4*>(
-      col + (unsigned long long)(unsigned)rb * qrow_bytes));  // T00, dy, dx, dxy
-  return fmaf(b, fmaf(a, v.w, v.y), fmaf(a, v.z, v.x));
+         (unsigned long long)kRow0 * qrow_bytes;
 }
 
 // Blackwell's packed FP32 pairs (FFMA2, FADD2, FMUL2): one instruction for two lanes, each lane
@@ -197,8 +172,8 @@ __device__ __forceinline__ float2 f2sub(float2 x, float2 y) {
   return __ffma2_rn(y, make_float2(-1.0f, -1.0f), x);
 }
 
-// EXACT column: weight a and 16 * (clamped column bit pattern) added to the biased view base
-__device__ __forceinline__ unsigned long long quad_col_exact(unsigned long long vbias, float p,
+// column p: weight a (the fraction) and 16 * (clamped column bit pattern) added to the biased view base
+__device__ __forceinline__ unsigned long long quad_col(unsigned long long vbias, float p,
                                                              int ns, float& a) {
   const float t = __fadd_rd(p, kMagic);
   a = p - (t - kMagic);
@@ -261,19 +236,15 @@ __device__ __forceinline__ float asin_half(float x) {
   return fmaf(__fmul_rn(x, t), p, x);
 }
 
-// Column of a sample: clamped origin offset and weight
-template <int INTERP>
-__device__ __forceinline__ void quad_col(float p_idx, int ns, int& off, float& a) {
-  float xb;
-  if (INTERP == LCT_INTERP_TEX8)
-    xb = __fsub_rn(__fadd_rn(p_idx, 0.5f), 0.5f);
-  else
-    xb = p_idx;
-  const float fx = floorf(xb);
-  a = xb - fx;
-  if (INTERP == LCT_INTERP_TEX8) a = q8(a);
-  int i = (int)fx;
-  off = min(max(i, -2), ns) + 2;
+// x / d rounded to nearest for a launch-constant d with r = RN(1 / d): the quotient estimate's
+// remainder is exact in an FMA and one more FMA rounds correctly (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34(1), 1990), except
+// that a divisor whose fraction bits are all ones may leave a power of two one ulp off; 3
+// operations where a division by a variable is a subroutine.  tests/test_div_by.py compares every
+// fraction of x with the division.
+__device__ __forceinline__ float div_by(float x, float d, float r) {
+  const float q = __fmul_rn(x, r);
+  return fmaf(fmaf(-q, d, x), r, q);
 }
 
 // One tile: voxel columns [bx*kQTX, +kQTX) x [by*kQTY, +kQTY), slab/slice chunk bz.  Called with
@@ -283,9 +254,9 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
   __shared__ float4 s_cs[kQVB];      // cos, sin of view ia and of its conjugate ia + half
   __shared__ int2 s_jr[kQVB];        // slices [jlo, jhi) of the chunk whose window holds ia
   __shared__ float2 s_zb[kQVB];      // EXACT: source z of both views without the fan-angle term
-  __shared__ ulonglong2 s_qv[kQVB];  // bases of both views (EXACT: biased, quad_view_bias)
-  __shared__ ulonglong2 s_pfb[kQVB]; // EXACT: prefetch box origins of both views
-  __shared__ int4 s_pfs[kQVB];       // EXACT: prefetch box rows and column spans
+  __shared__ ulonglong2 s_qv[kQVB];  // biased bases of both views (quad_view_bias)
+  __shared__ ulonglong2 s_pfb[kQVB]; // prefetch box origins of both views
+  __shared__ int4 s_pfs[kQVB];       // prefetch box rows and column spans
 
   const int tid = threadIdx.y * kQTX + threadIdx.x;
   const int ix = bx * kQTX + threadIdx.x;
@@ -301,7 +272,7 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
   const float yc = __fmul_rn((float)iy - A.wy, A.dy);
   const float zc0 = __fmul_rn((float)z0 - A.wz, A.dz);
   const float wt2 = A.wt + 2.0f;
-  // EXACT prefetch: the tile's corner coordinates and last slice
+  // prefetch: the tile's corner coordinates and last slice
   const float xr0 = __fmul_rn((float)(bx * kQTX) - A.wx, A.dx);
   const float xr1 = __fmul_rn((float)(min(bx * kQTX + kQTX, A.nx) - 1) - A.wx, A.dx);
   const float yr0 = __fmul_rn((float)(by * kQTY) - A.wy, A.dy);
@@ -311,9 +282,6 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
   // when that is below dso / 2 every view of the tile takes the polynomial asin
   const float rx = fmaxf(fabsf(xr0), fabsf(xr1)), ry = fmaxf(fabsf(yr0), fabsf(yr1));
   const bool asin_poly = sqrtf(fmaf(rx, rx, ry * ry)) * A.inv_dso < 0.49f;
-  float zc[NZ];
-#pragma unroll
-  for (int j = 0; j < NZ; ++j) zc[j] = ((float)(z0 + j) - A.wz) * A.dz;
 
   int vlo = INT_MAX, vhi = INT_MIN;
   for (int j = 0; j < nzc; ++j) {
@@ -350,19 +318,16 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
       const float4* v1 = RING ? quad_view_ptr(A, sv, ia) : quads + (long long)ia * A.qstride;
       const float4* v2 = RING ? quad_view_ptr(A, sv, ia + A.half)
                               : quads + (long long)(ia + A.half) * A.qstride;
-      if (INTERP != LCT_INTERP_EXACT)
-        s_qv[tid] = make_ulonglong2(reinterpret_cast<unsigned long long>(v1),
-                                    reinterpret_cast<unsigned long long>(v2));
-      if (INTERP == LCT_INTERP_EXACT) {
+      if (INTERP == LCT_INTERP_EXACT)
         s_zb[tid] = make_float2(fmaf((float)ia, A.dzv, A.z0), fmaf((float)(ia + A.half), A.dzv, A.z0));
-        s_qv[tid] = make_ulonglong2(quad_view_bias(v1, A.qrow_bytes), quad_view_bias(v2, A.qrow_bytes));
-        int4 b1, b2;
-        prefetch_boxes(A, c1, s1, c2, s2, ia, xr0, xr1, yr0, yr1, zc0, zcl, b1, b2);
-        s_pfb[tid] = make_ulonglong2(
-            reinterpret_cast<unsigned long long>(v1) + (unsigned long long)b1.x * A.qrow_bytes + 16ull * b1.z,
-            reinterpret_cast<unsigned long long>(v2) + (unsigned long long)b2.x * A.qrow_bytes + 16ull * b2.z);
-        s_pfs[tid] = make_int4(b1.y - b1.x + 1, b1.w - b1.z, b2.y - b2.x + 1, b2.w - b2.z);
-      }
+      s_qv[tid] = make_ulonglong2(quad_view_bias<INTERP>(v1, A.qrow_bytes),
+                                  quad_view_bias<INTERP>(v2, A.qrow_bytes));
+      int4 b1, b2;
+      prefetch_boxes(A, c1, s1, c2, s2, ia, xr0, xr1, yr0, yr1, zc0, zcl, b1, b2);
+      s_pfb[tid] = make_ulonglong2(
+          reinterpret_cast<unsigned long long>(v1) + (unsigned long long)b1.x * A.qrow_bytes + 16ull * b1.z,
+          reinterpret_cast<unsigned long long>(v2) + (unsigned long long)b2.x * A.qrow_bytes + 16ull * b2.z);
+      s_pfs[tid] = make_int4(b1.y - b1.x + 1, b1.w - b1.z, b2.y - b2.x + 1, b2.w - b2.z);
       int jlo = nzc, jhi = 0;
       for (int j = 0; j < nzc; ++j)
         if (ia >= A.a_min[z0 + j] && ia < A.a_mid[z0 + j]) {
@@ -375,7 +340,7 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
     const int nv = min(kQVB, vhi - vb);
     for (int k = 0; k < nv; ++k) {
       const int ia = vb + k;
-      if (INTERP == LCT_INTERP_EXACT && k + 1 < nv) {
+      if (k + 1 < nv) {
         // the next view's footprint into L1 while this one is sampled (no result depends on it,
         // and every address lies inside that view's quads).  One 4-byte load per 32-byte sector,
         // its value unused: a load brings in the sector it touches, and a prefetch instruction
@@ -400,137 +365,146 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
       const float cb = cs.x, sb = cs.y, cb2 = cs.z, sb2 = cs.w;
       // CUDA/Backprojector.cu:53-64, z-invariant part
       const float phat = fmaf(-xc, cb, -__fmul_rn(yc, sb));
-      float theta, delta_p, tho, sq;
-      if (INTERP == LCT_INTERP_TEX8) {
-        theta = asinf(__fdiv_rn(phat, A.dso));
-        delta_p = __fdiv_rn(__fmul_rn(theta, A.dso), A.ds);
-        tho = __fdiv_rn(theta, A.orbit);
-        sq = sqrtf(fmaf(-phat, phat, A.dso2));
-      } else {
+      const ulonglong2 qv = s_qv[k];
+      // slice j's row coordinate in both views is one packed FMA: EXACT h + j kd, TEX8 zc k + m
+      // (the reference's expression, CUDA/Backprojector.cu:66-67)
+      float2 K, M;
+      float a1, a2;
+      unsigned long long q1, q2;
+      float2 U = make_float2(0.f, 0.f);  // EXACT: M + wt + 2
+      if constexpr (INTERP == LCT_INTERP_EXACT) {
         const float sx = __fmul_rn(phat, A.inv_dso);
+        float theta;
         if (asin_poly)
           theta = asin_half(sx);
         else
           theta = asinf(sx);
-        delta_p = 0.0f;  // EXACT: the columns are fmaf(+-theta, dso/ds, ws)
-        tho = __fmul_rn(theta, A.inv_orbit);
+        const float tho = __fmul_rn(theta, A.inv_orbit);
         const float t = fmaf(-phat, phat, A.dso2);
-        sq = __fmul_rn(t, rsqrtf(t));
-      }
-      const float l1 = fmaf(xc, sb, fmaf(-yc, cb, sq));
-      const float l2 = fmaf(xc, sb2, fmaf(-yc, cb2, sq));
-      if constexpr (INTERP == LCT_INTERP_EXACT) {
+        const float sq = __fmul_rn(t, rsqrtf(t));
+        const float l1 = fmaf(xc, sb, fmaf(-yc, cb, sq));
+        const float l2 = fmaf(xc, sb2, fmaf(-yc, cb2, sq));
         // source z from the staged per-view term: zr = (ia + tho) dzv + z0
         const float2 zb = s_zb[k];
-        const ulonglong2 qv = s_qv[k];
         const float zr1 = fmaf(tho, A.dzv, zb.x), zr2 = fmaf(-tho, A.dzv, zb.y);
-        // slice j: qhat = h + j kd with k = kq / l, kd = k dz (one FMA with a constant j, no
-        // per-slice z register); weights halved around one reciprocal -- the factor 2 is
-        // restored, exactly, at the output
+        // k = kq / l, kd = k dz (no per-slice z register); weights halved around one reciprocal --
+        // the factor 2 is restored, exactly, at the output
         const float r1 = __fdividef(1.0f, l1), r2 = __fdividef(1.0f, l2);
-        const float kd1 = __fmul_rn(A.kqdz, r1), kd2 = __fmul_rn(A.kqdz, r2);
-        const float h1 = __fmul_rn(__fsub_rn(zc0, zr1), __fmul_rn(A.kq, r1));
-        const float h2 = __fmul_rn(__fsub_rn(zc0, zr2), __fmul_rn(A.kq, r2));
-        const float u1 = __fadd_rn(h1, wt2), u2 = __fadd_rn(h2, wt2);
-        float a1, a2;
-        const unsigned long long q1 = quad_col_exact(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
-        const unsigned long long q2 = quad_col_exact(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
-        const float2 KD = make_float2(kd1, kd2), H = make_float2(h1, h2), U = make_float2(u1, u2);
-        const float2 A1 = f2(a1), A2 = f2(a2);
-        // one slice of the pair, the view and its conjugate as one packed FP32 pair; INSIDE: both
-        // samples lie within the detector rows (no tests, no selects, no row clamps).  A slice
-        // whose window does not hold the view is evaluated with its group and not added.
-        auto slice_x = [&](int j, auto inside, bool add) {
-          const float2 J = f2((float)j);
-          const float2 qh = __ffma2_rn(J, KD, H);
+        K = make_float2(__fmul_rn(A.kqdz, r1), __fmul_rn(A.kqdz, r2));
+        M = make_float2(__fmul_rn(__fsub_rn(zc0, zr1), __fmul_rn(A.kq, r1)),
+                        __fmul_rn(__fsub_rn(zc0, zr2), __fmul_rn(A.kq, r2)));
+        U = make_float2(__fadd_rn(M.x, wt2), __fadd_rn(M.y, wt2));
+        q1 = quad_col(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
+        q2 = quad_col(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
+      } else {
+        const float theta = asinf(div_by(phat, A.dso, A.inv_dso));
+        const float delta_p = div_by(__fmul_rn(theta, A.dso), A.ds, A.inv_ds);
+        const float tho = div_by(theta, A.orbit, A.inv_orbit);
+        const float sq = sqrtf(fmaf(-phat, phat, A.dso2));
+        const float l1 = fmaf(xc, sb, fmaf(-yc, cb, sq));
+        const float l2 = fmaf(xc, sb2, fmaf(-yc, cb2, sq));
+        const float zr1 = fmaf(__fadd_rn((float)ia, tho), A.dzv, A.z0);
+        const float zr2 = fmaf(__fsub_rn((float)(ia + A.half), tho), A.dzv, A.z0);
+        K = make_float2(__fdividef(A.kq, l1), __fdividef(A.kq, l2));
+        M = make_float2(__fmul_rn(-zr1, K.x), __fmul_rn(-zr2, K.y));
+        // the reference's texture coordinate carries + 0.5
+        q1 = quad_col(qv.x, __fsub_rn(__fadd_rn(__fadd_rn(delta_p, A.ws), 0.5f), 0.5f), A.ns, a1);
+        q2 = quad_col(qv.y, __fsub_rn(__fadd_rn(__fsub_rn(A.ws, delta_p), 0.5f), 0.5f), A.ns, a2);
+        a1 = q8(a1);
+        a2 = q8(a2);
+      }
+      const float2 A1 = f2(a1), A2 = f2(a2);
+      // J of slice j: EXACT its number (a constant), TEX8 its z
+      auto slice_j = [&](int j) {
+        return INTERP == LCT_INTERP_EXACT ? (float)j : __fmul_rn(__fsub_rn((float)(z0 + j), A.wz), A.dz);
+      };
+      // one slice of the pair, the view and its conjugate as one packed FP32 pair; INSIDE: both
+      // samples lie within the detector rows (no tests, no selects, no row clamps).  A slice
+      // whose window does not hold the view is evaluated with its group and not added.
+      auto slice = [&](int j, auto inside, bool add) {
+        constexpr bool kIn = decltype(inside)::value;
+        const float2 J = f2(slice_j(j));
+        const float2 qh = __ffma2_rn(J, K, M);
+        const bool out1 = !kIn && fabsf(qh.x) > wt, out2 = !kIn && fabsf(qh.y) > wt;
+        float2 y;  // row coordinate (EXACT: + 2), texel centres at whole numbers
+        if constexpr (INTERP == LCT_INTERP_EXACT)
+          y = __ffma2_rn(J, K, U);
+        else
+          y = __fadd2_rn(__fadd2_rn(__fadd2_rn(qh, f2(wt)), f2(0.5f)), f2(-0.5f));
+        const float2 t = __fadd2_rd(y, f2(kMagic));
+        const float2 b = f2sub(y, __fadd2_rn(t, f2(-kMagic)));
+        int r1 = __float_as_int(t.x), r2 = __float_as_int(t.y);
+        if constexpr (!kIn) {
+          constexpr int kRow0 = INTERP == LCT_INTERP_TEX8 ? kMagicBits - 2 : kMagicBits;
+          r1 = min(max(r1, kRow0), kRow0 + A.nt + 2);
+          r2 = min(max(r2, kRow0), kRow0 + A.nt + 2);
+        }
+        const float4 v0 = __ldg(reinterpret_cast<const float4*>(
+            q1 + (unsigned long long)(unsigned)r1 * A.qrow_bytes));  // T00, dy, dx, dxy
+        const float4 v1 = __ldg(reinterpret_cast<const float4*>(
+            q2 + (unsigned long long)(unsigned)r2 * A.qrow_bytes));
+        float sum;
+        if constexpr (INTERP == LCT_INTERP_EXACT) {
           // the pair weights sum to one in every case -- (-qh2, qh1) / (qh1 - qh2), (0, 1),
           // (1, 0), (1/2, 1/2) -- so w1 s1 + w2 s2 = s2 + w1 (s1 - s2)
-          const float in1 = -qh.y * __fdividef(1.0f, qh.x - qh.y);
-          float w1 = in1;
-          const float2 u = __ffma2_rn(J, KD, U);
-          const float2 t = __fadd2_rd(u, f2(kMagic));
-          const float2 b = f2sub(u, __fadd2_rn(t, f2(-kMagic)));
-          int r1 = __float_as_int(t.x), r2 = __float_as_int(t.y);
-          if constexpr (!decltype(inside)::value) {
-            const bool out1 = fabsf(qh.x) > wt, out2 = fabsf(qh.y) > wt;
-            w1 = out1 ? (out2 ? 0.5f : 0.0f) : (out2 ? 1.0f : in1);
-            r1 = min(max(r1, kMagicBits), kMagicBits + A.nt + 2);
-            r2 = min(max(r2, kMagicBits), kMagicBits + A.nt + 2);
-          }
-          const float4 v0 = __ldg(reinterpret_cast<const float4*>(
-              q1 + (unsigned long long)(unsigned)r1 * A.qrow_bytes));  // T00, dy, dx, dxy
-          const float4 v1 = __ldg(reinterpret_cast<const float4*>(
-              q2 + (unsigned long long)(unsigned)r2 * A.qrow_bytes));
+          float w1 = -qh.y * __fdividef(1.0f, qh.x - qh.y);
+          if constexpr (!kIn) w1 = out1 ? (out2 ? 0.5f : 0.0f) : (out2 ? 1.0f : w1);
           const float2 p0 = __ffma2_rn(A1, make_float2(v0.z, v0.w), make_float2(v0.x, v0.y));
           const float2 p1 = __ffma2_rn(A2, make_float2(v1.z, v1.w), make_float2(v1.x, v1.y));
           const float s1 = fmaf(b.x, p0.y, p0.x), s2 = fmaf(b.y, p1.y, p1.x);
-          const float sum = fmaf(w1, s1 - s2, acc[j] + s2);
-          if (add) acc[j] = sum;
-        };
-        // qhat(j) = fmaf(j, kd, h) is monotone in j (monotone rounding of a linear function), so
-        // the first and last slices of the groups that run bound every |qhat|: when both are
-        // inside for both views in every lane of the warp, every out test is false and the tests,
-        // selects and clamps are skipped with no change to any result.  The row coordinate
-        // u = qhat + wt + 2 (equal to within a few ulps, far below half a row) then lies in
-        // (1.5, 2 wt + 2.5), inside the quad rows when rows_inside_ok.  A NaN fails the test.
-        // (69.4 ms with scalar code and no inside path on partial windows, 64.5 ms so.)
-        const float jf = (float)(jlo & ~(kQGroup - 1));
-        const float jl = (float)(((jhi + kQGroup - 1) & ~(kQGroup - 1)) - 1);
-        const bool inside = A.rows_inside_ok && fabsf(fmaf(jf, kd1, h1)) <= wt &&
-                            fabsf(fmaf(jl, kd1, h1)) <= wt && fabsf(fmaf(jf, kd2, h2)) <= wt &&
-                            fabsf(fmaf(jl, kd2, h2)) <= wt;
-        if (__all_sync(0xffffffffu, inside)) {
-          if (jlo == 0 && jhi == NZ) {  // straight code: every load of the chunk may be in flight
-#pragma unroll
-            for (int j = 0; j < NZ; ++j) slice_x(j, std::true_type{}, true);
-          } else
-#pragma unroll
-          for (int g = 0; g < NZ; g += kQGroup) {
-            if (jlo < g + kQGroup && jhi > g) {
-#pragma unroll
-              for (int j = g; j < g + kQGroup; ++j) slice_x(j, std::true_type{}, j >= jlo && j < jhi);
-            }
-          }
+          sum = fmaf(w1, s1 - s2, acc[j] + s2);
         } else {
+          const float r = __fdividef(2.0f, qh.x - qh.y);
+          float w1 = -qh.y * r, w2 = qh.x * r;
+          if constexpr (!kIn) {
+            w1 = out1 ? (out2 ? 1.0f : 0.0f) : (out2 ? 2.0f : w1);
+            w2 = out1 ? (out2 ? 1.0f : 2.0f) : (out2 ? 0.0f : w2);
+          }
+          // texture unit: w01 = a - w11, w10 = b - w11, w00 = 1 - a - b + w11, so the sample is
+          // T00 + a dx + b dy + w11 dxy with b = round-half-up of the fraction and w11 =
+          // round-half-up(a b), both on the 1/256 grid: B = 256 b and W = 256 w11 are the whole
+          // parts of exact sums (the quads' row differences carry the 1/256)
+          const float2 B = __fadd2_rn(__fadd2_rd(__ffma2_rn(b, f2(256.0f), f2(0.5f)), f2(kMagic)), f2(-kMagic));
+          const float2 W = __fadd2_rn(__fadd2_rd(__ffma2_rn(make_float2(a1, a2), B, f2(0.5f)), f2(kMagic)), f2(-kMagic));
+          const float s1 = fmaf(W.x, v0.w, fmaf(B.x, v0.y, fmaf(a1, v0.z, v0.x)));
+          const float s2 = fmaf(W.y, v1.w, fmaf(B.y, v1.y, fmaf(a2, v1.z, v1.x)));
+          sum = fmaf(w1, s1, fmaf(w2, s2, acc[j]));
+        }
+        if (add) acc[j] = sum;
+      };
+      constexpr int kQGroup = kQGroupOf<NZ>;
+      // qhat is monotone in j (a monotone rounding of a linear function), so the first and last
+      // slices of the groups that run bound every |qhat|: when both are inside for both views in
+      // every lane of the warp, every out test is false and the tests, selects and clamps are
+      // skipped with no change to any result.  The row coordinate (equal to qhat + wt within a
+      // few ulps, far below half a row) then lies inside the quad rows when rows_inside_ok.  A
+      // NaN fails the test.  (EXACT, 512^2 x 256 from 736 x 64 views: 69.4 ms with scalar code and
+      // no inside path on partial windows, 64.5 ms so.)
+      const float jf = slice_j(jlo & ~(kQGroup - 1));
+      const float jl = slice_j(((jhi + kQGroup - 1) & ~(kQGroup - 1)) - 1);
+      const bool inside = A.rows_inside_ok && fabsf(fmaf(jf, K.x, M.x)) <= wt &&
+                          fabsf(fmaf(jl, K.x, M.x)) <= wt && fabsf(fmaf(jf, K.y, M.y)) <= wt &&
+                          fabsf(fmaf(jl, K.y, M.y)) <= wt;
+      if (__all_sync(0xffffffffu, inside)) {
+        if (jlo == 0 && jhi == NZ) {  // straight code: every load of the chunk may be in flight
+#pragma unroll
+          for (int j = 0; j < NZ; ++j) slice(j, std::true_type{}, true);
+        } else
 #pragma unroll
           for (int g = 0; g < NZ; g += kQGroup) {
             if (jlo < g + kQGroup && jhi > g) {
 #pragma unroll
-              for (int j = g; j < g + kQGroup; ++j) slice_x(j, std::false_type{}, j >= jlo && j < jhi);
+              for (int j = g; j < g + kQGroup; ++j) slice(j, std::true_type{}, j >= jlo && j < jhi);
             }
           }
-        }
-        continue;
-      }
-      const float zr1 = fmaf((float)ia + tho, A.dzv, A.z0);
-      const float zr2 = fmaf((float)(ia + A.half) - tho, A.dzv, A.z0);
-      const float k1 = __fdividef(A.kq, l1), k2 = __fdividef(A.kq, l2);
-      const float m1 = -zr1 * k1, m2 = -zr2 * k2;
-      int o1, o2;
-      float a1, a2;
-      quad_col<INTERP>(delta_p + A.ws, A.ns, o1, a1);
-      quad_col<INTERP>(-delta_p + A.ws, A.ns, o2, a2);
-      const ulonglong2 qb = s_qv[k];
-      const float4* q1 = reinterpret_cast<const float4*>(qb.x) + o1;
-      const float4* q2 = reinterpret_cast<const float4*>(qb.y) + o2;
-      auto slice = [&](int j) {
-        const float qh1 = fmaf(zc[j], k1, m1), qh2 = fmaf(zc[j], k2, m2);
-        const bool out1 = fabsf(qh1) > wt, out2 = fabsf(qh2) > wt;
-        const float r = __fdividef(2.0f, qh1 - qh2);
-        float w1 = -qh2 * r, w2 = qh1 * r;
-        w1 = out1 ? (out2 ? 1.0f : 0.0f) : (out2 ? 2.0f : w1);
-        w2 = out1 ? (out2 ? 1.0f : 2.0f) : (out2 ? 0.0f : w2);
-        const float s1 = quad_sample<INTERP>(q1, A.qcols, A.nt, a1, qh1 + wt);
-        const float s2 = quad_sample<INTERP>(q2, A.qcols, A.nt, a2, qh2 + wt);
-        acc[j] = fmaf(w1, s1, fmaf(w2, s2, acc[j]));
-      };
-      if (jlo == 0 && jhi == NZ) {
-#pragma unroll
-        for (int j = 0; j < NZ; ++j) slice(j);
       } else {
 #pragma unroll
-        for (int j = 0; j < NZ; ++j)
-          if (j >= jlo && j < jhi) slice(j);
+        for (int g = 0; g < NZ; g += kQGroup) {
+          if (jlo < g + kQGroup && jhi > g) {
+#pragma unroll
+            for (int j = g; j < g + kQGroup; ++j) slice(j, std::false_type{}, j >= jlo && j < jhi);
+          }
+        }
       }
     }
   }
@@ -656,7 +630,8 @@ __device__ __forceinline__ void bp_tma_tile(const BpQuadArgs& A, const CUtensorM
       const float4* v1 = quad_view_ptr(A, sv, ia);
       const float4* v2 = quad_view_ptr(A, sv, ia + A.half);
       s_zb[tid] = make_float2(fmaf((float)ia, A.dzv, A.z0), fmaf((float)(ia + A.half), A.dzv, A.z0));
-      s_qv[tid] = make_ulonglong2(quad_view_bias(v1, A.qrow_bytes), quad_view_bias(v2, A.qrow_bytes));
+      s_qv[tid] = make_ulonglong2(quad_view_bias<LCT_INTERP_EXACT>(v1, A.qrow_bytes),
+                                  quad_view_bias<LCT_INTERP_EXACT>(v2, A.qrow_bytes));
       int4 b1, b2;
       prefetch_boxes(A, c1, s1, c2, s2, ia, xr0, xr1, yr0, yr1, zc0, zcl, b1, b2);
       const bool fits = b1.y - b1.x + 1 <= kTmaBH && b1.w - b1.z + 1 <= kTmaBW &&
@@ -710,8 +685,8 @@ __device__ __forceinline__ void bp_tma_tile(const BpQuadArgs& A, const CUtensorM
       const float h2 = __fmul_rn(__fsub_rn(zc0, zr2), __fmul_rn(A.kq, r2));
       const float u1 = __fadd_rn(h1, wt2), u2 = __fadd_rn(h2, wt2);
       float a1, a2;
-      const unsigned long long q1 = quad_col_exact(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
-      const unsigned long long q2 = quad_col_exact(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
+      const unsigned long long q1 = quad_col(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
+      const unsigned long long q2 = quad_col(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
       // the thread's quad columns (0 .. ns + 2) and its first / last slice's quad rows
       const int qc1 = (int)((q1 - qv.x) >> 4) - (kMagicBits - 2);
       const int qc2 = (int)((q2 - qv.y) >> 4) - (kMagicBits - 2);
@@ -1047,6 +1022,7 @@ static int build_bp_quad_args(const lct_geom& g, const lct_img& ig, const BpLaun
   a.ws = g.ws;
   a.wt = g.wt;
   a.ds = g.ds;
+  a.inv_ds = 1.0f / g.ds;
   a.dso = g.dso;
   a.dso2 = g.dso * g.dso;
   a.inv_dso = 1.0f / g.dso;
@@ -1077,7 +1053,7 @@ static int build_bp_quad_args(const lct_geom& g, const lct_img& ig, const BpLaun
     a.slab_z0[i] = L.slab_z0[i];
   }
   nzt = L.nz_thread;
-  if (nzt != 4 && nzt != 8 && nzt != 16) nzt = 8;
+  if (nzt != 1 && nzt != 2 && nzt != 4 && nzt != 8 && nzt != 16) nzt = 8;
   a.zchunks = (L.nz + nzt - 1) / nzt;
   a.gx = (ig.nx + kQTX - 1) / kQTX;
   a.gy = (ig.ny + kQTY - 1) / kQTY;
@@ -1119,6 +1095,8 @@ int launch_bp_par_quads(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
   } while (0)
   if (a.qring > 0) {
     switch (nzt) {
+      case 1: LCT_BPQR(1); break;
+      case 2: LCT_BPQR(2); break;
       case 4: LCT_BPQR(4); break;
       case 16: LCT_BPQR(16); break;
       default: LCT_BPQR(8);
@@ -1136,6 +1114,8 @@ int launch_bp_par_quads(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
     }                              \
   } while (0)
   switch (nzt) {
+    case 1: LCT_BPQ(1, 4); break;
+    case 2: LCT_BPQ(2, 4); break;
     case 4: LCT_BPQ_NZ(4); break;
     case 16: LCT_BPQ_NZ(16); break;
     default: LCT_BPQ_NZ(8);
@@ -1213,6 +1193,8 @@ int launch_bp_par_texture(const lct_geom& g, const lct_img& ig, const BpLaunch& 
     }                                    \
   } while (0)
   switch (nzt) {
+    case 1: LCT_BPT(1, 4); break;
+    case 2: LCT_BPT(2, 4); break;
     case 4: LCT_BPT_NZ(4); break;
     case 16: LCT_BPT_NZ(16); break;
     default: LCT_BPT_NZ(8);
@@ -1259,6 +1241,8 @@ int launch_bp_quad_worklist(const void* d_args, const int* d_prefix, int n_scans
     }                                    \
   } while (0)
   switch (nz_thread) {
+    case 1: LCT_BPW(1, 4); break;
+    case 2: LCT_BPW(2, 4); break;
     case 4: LCT_BPW_NZ(4); break;
     case 16: LCT_BPW_NZ(16); break;
     default: LCT_BPW_NZ(8);

@@ -63,7 +63,7 @@ struct BpLaunch {
   int slab_view[kBpMaxSlabs];
   int slab_z0[kBpMaxSlabs];
   int interp, addr;
-  int nz_thread;       // slices per thread (8, 16, 32; 0 = choose)
+  int nz_thread;       // slices per thread (quads: 1, 2, 4, 8, 16; else 8, 16, 32; 0 = choose)
   int minb = 0;        // quad kernel: resident CTAs per SM the register budget targets (0 = 4)
   // quad kernel only: a part of the slabs' views, [view_lo, view_hi) in slab-local indices,
   // carried between parts as raw FP32 sums in img (part kBpWhole / First / Middle / Last); the
@@ -89,8 +89,23 @@ LCT_HD inline long long quad_cols(int ns) { return (long long)ns + 3; }
 LCT_HD inline long long quad_view_elems(int ns, int nt) { return (long long)(nt + 3) * (ns + 3); }
 // ring > 0: quads is a ring of `ring` views and rows view v is packed into slot
 // (vbase + v) mod ring; 0: into view v.
-int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, float4* quads,
-                     cudaStream_t s, long long vbase = 0, long long ring = 0);
+// interp: TEX8 quads hold their row differences (dy, dxy) times 2^-8.
+int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, int interp,
+                     float4* quads, cudaStream_t s, long long vbase = 0, long long ring = 0);
+// Slices per thread of the quad kernel by default: 8, which shares a view's terms among most slices;
+// 4 when a view stays active for fewer than 6 slices ((feed / 2) / dz); and fewer where one slab's
+// 16 x 16 tiles would leave most of the chip's 592 CTA slots empty and the views' latency in series
+// is what counts.  The line by tiles, on 736 x 64 views (ms at 1 / 2 / 4 / 8 slices): 32^2
+// 0.41 / 0.47 / 0.80 / 1.39, 64^2 0.48 / 0.47 / 0.77 / 1.25, 128^2 1.48 / 0.98 / 0.83 / 1.16, 192^2
+// 3.16 / 2.08 / 1.60 / 1.34, 256^2 5.41 / 3.54 / 2.70 / 2.32.  One slab's tiles, whatever the launch
+// holds: streamed, bounded and whole runs then sum alike.
+inline int bp_nz_default(const lct_geom& g, const lct_img& ig) {
+  const long long tiles = (long long)((ig.nx + 15) / 16) * ((ig.ny + 15) / 16);
+  if (tiles * 16 < 200) return 1;
+  if (tiles * 8 < 500) return 2;
+  if (tiles * 4 < 500) return 4;
+  return 0.5 * (double)g.pitch / (double)ig.dz < 6.0 ? 4 : 8;
+}
 // Backprojection from quad-layout views (full windows only; L.proj is ignored, L.quads used).
 int launch_bp_par_quads(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
                         const float4* quads, cudaStream_t s);
