@@ -279,8 +279,9 @@ typedef struct lct_recon_opts {
   int backprojector; /* LCT_BP_* */
   int interp;        /* LCT_INTERP_* */
   int addr;          /* LCT_ADDR_* */
-  int bp_nz;         /* backprojection slices per thread: 4, 8, 16; 0 = default (8, or 4 when a
-                        view stays active for few slices); -1 = autotune at create */
+  int bp_nz;         /* backprojection slices per thread: 4, 8, 16; 0 = default (8; fewer when a
+                        view stays active for few slices or the image is small); -1 = autotune at
+                        create */
   int bp_minb;       /* backprojection CTAs per SM the register budget targets: 1-4 (0 = 4) */
   int bp_sampler;    /* LCT_BP_SAMPLER_*: how the backprojector samples the filtered views */
 } lct_recon_opts;

@@ -104,12 +104,9 @@ struct lct_recon {
 };
 
 namespace lct {
-// backprojection slices per thread: the requested 4 / 8 / 16, else the measured default (8,
-// or 4 when a view stays active for fewer than 6 slices: (feed / 2) / dz)
+// backprojection slices per thread: the requested 4 / 8 / 16, else bp_nz_default
 inline int pick_bp_nz(const lct_geom& g, const lct_img& ig, int requested) {
-  if (requested == 4 || requested == 8 || requested == 16) return requested;
-  const double act = 0.5 * (double)g.pitch / (double)ig.dz;
-  return act < 6.0 ? 4 : 8;
+  return requested == 4 || requested == 8 || requested == 16 ? requested : bp_nz_default(g, ig);
 }
 // kernels one filter call launches
 inline int filter_launches(int mode) { return mode == LCT_FILTER_FP32 ? 1 : 2; }
