@@ -82,6 +82,11 @@ int lct_last_cuda_error(void); /* cudaError_t of the last LCT_ERR_CUDA, per thre
    (no trap, no assert).  Synchronous. */
 int lct_device_status(int* code_out);
 int lct_version(void);
+/* Gives back the device memory that the current device's scratch pool keeps between calls of the
+   stage entry points (lct_filter_rows in the BF16 modes, lct_backproject_par): at most 4 GiB or
+   1/32 of the device, whichever is less; the driver also takes it when another allocation of the
+   process needs it.  Calls in flight are not disturbed.  No effect where nothing is kept. */
+int lct_scratch_release(void);
 
 /* ---------------------------------------------------------------------------------------
  * Stage 1 -- rebinning.  fan [n_angle_add][nt][ns] -> par [n_angle][nt][ns] (both device).

@@ -131,6 +131,7 @@ SIGNATURES: dict[str, tuple] = {
     "lct_last_cuda_error": (I32, []),
     "lct_device_status": (I32, [C.POINTER(I32)]),
     "lct_version": (I32, []),
+    "lct_scratch_release": (I32, []),
     "lct_rebin_fan2par": (I32, [GP, P, P, I32, I32, P]),
     "lct_rebin_fan2par_index": (I32, [GP, I32, P, P, P]),
     "lct_rebin_fan2par_scan": (I32, [GP, P, I64, I64, P, I64, I64, I32, I32, I32, P]),

@@ -604,7 +604,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
   if (ig->nz <= kBpMaxZ && bp_windows_full(*g, *ig, ig->nz)) {
     float4* q = nullptr;
     const size_t bytes = sizeof(float4) * (size_t)g->n_angle * quad_view_elems(g->ns, g->nt);
-    if ((st = cuda_status(cudaMallocAsync((void**)&q, bytes, s)))) return LCT_ERR_ALLOC;
+    if ((st = scratch_alloc((void**)&q, bytes, s))) return LCT_ERR_ALLOC;
     st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, interp, q, s);
     if (!st) {
       BpLaunch L;
@@ -622,7 +622,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
       L.nz_thread = bp_nz_default(*g, *ig);
       st = launch_bp_par_quads(*g, *ig, L, q, s);
     }
-    int st2 = cuda_status(cudaFreeAsync(q, s));
+    int st2 = scratch_free(q, s);
     return st ? st : st2;
   }
   // slices in chunks of 32 (each chunk has its own window table; the voxel z coordinate is

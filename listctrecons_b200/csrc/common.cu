@@ -1,4 +1,5 @@
 // Status codes, CUDA error bookkeeping, the device status word and geometry checks.
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -34,6 +35,54 @@ int* device_status_ptr() {
   }
   return ptrs[dev];
 }
+
+// Scratch of the stage entry points.  The default pool unmaps what is freed at every
+// synchronisation, so a call that takes a gigabyte of scratch after each one paid for mapping it
+// again (a 3,600-view block of 735 x 31: 15-160 ms a call for a 5 ms kernel).  One pool per device
+// keeps up to kScratchKeep bytes (1/32 of the device's memory if that is less) mapped between calls.
+// The pool is stream-ordered and thread-safe like the default one; what exceeds the bound goes back
+// at the next synchronisation, the rest when the driver needs it for another allocation of the
+// process or lct_scratch_release asks.
+constexpr size_t kScratchKeep = 4ull << 30;
+static std::mutex g_scratch_mu;
+static cudaMemPool_t g_scratch_pool[64] = {nullptr};
+
+static cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  if (!g_scratch_pool[dev]) {
+    cudaMemPoolProps p = {};
+    p.allocType = cudaMemAllocationTypePinned;
+    p.handleTypes = cudaMemHandleTypeNone;
+    p.location.type = cudaMemLocationTypeDevice;
+    p.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    size_t free_b = 0, total = 0;
+    uint64_t keep = kScratchKeep;
+    if (cudaMemGetInfo(&free_b, &total) == cudaSuccess) keep = std::min<uint64_t>(keep, total / 32);
+    if (cudaMemPoolCreate(&pool, &p) != cudaSuccess) {
+      cudaGetLastError();  // no pools on this device: the default one
+      return nullptr;
+    }
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
+      cudaGetLastError();
+    g_scratch_pool[dev] = pool;
+  }
+  return g_scratch_pool[dev];
+}
+
+int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  *p = nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaMemPool_t pool = nullptr;
+  // a captured call's scratch belongs to its graph
+  if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+    pool = scratch_pool();
+  return cuda_status(pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s));
+}
+
+int scratch_free(void* p, cudaStream_t s) { return cuda_status(cudaFreeAsync(p, s)); }
 
 int check_geom(const lct_geom* g) {
   if (!g) return LCT_ERR_ARG;
@@ -86,6 +135,15 @@ LCT_API const char* lct_status_string(int status) {
 }
 
 LCT_API int lct_last_cuda_error(void) { return t_last_cuda_error; }
+
+LCT_API int lct_scratch_release(void) {
+  int dev = 0;
+  int st = cuda_status(cudaGetDevice(&dev));
+  if (st) return st;
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  if (dev < 0 || dev >= 64 || !g_scratch_pool[dev]) return LCT_OK;
+  return cuda_status(cudaMemPoolTrimTo(g_scratch_pool[dev], 0));
+}
 
 LCT_API int lct_version(void) { return 100; }
 

@@ -374,11 +374,11 @@ int launch_filter_tc(int ns, const float* d_h, float* d_rows, long long nrows, i
                      cudaStream_t s) {
   if (nrows <= 0) return LCT_OK;
   void* scratch = nullptr;
-  if (cuda_status(cudaMallocAsync(&scratch, tc_scratch_bytes(ns, nrows, mode), s)))
+  if (scratch_alloc(&scratch, tc_scratch_bytes(ns, nrows, mode), s))
     return LCT_ERR_ALLOC;
   int st = tc_build_toeplitz(ns, d_h, scratch, mode, s);
   if (!st) st = tc_filter(ns, d_rows, nrows, scratch, nrows, mode, s);
-  int st2 = cuda_status(cudaFreeAsync(scratch, s));
+  int st2 = scratch_free(scratch, s);
   return st ? st : st2;
 }
 

@@ -28,6 +28,10 @@ void set_cuda_error(cudaError_t e);
 int cuda_status(cudaError_t e);  // LCT_OK or LCT_ERR_CUDA (records e)
 int launch_status();             // cudaGetLastError() -> status
 
+// Stream-ordered scratch of a stage entry point (common.cu), from a bounded pool of the library's own.
+int scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+int scratch_free(void* p, cudaStream_t s);
+
 // Device status word (file-scope __device__ int in common.cu).  Kernels raise it on a work
 // item they refuse (an index outside its buffer) instead of trapping.
 int* device_status_ptr();  // per current device, resolved with cudaGetSymbolAddress
