@@ -25,6 +25,7 @@
 #include <cmath>
 
 #include "lct_internal.h"
+#include "fp32_pair.cuh"
 #include "tex_emul.cuh"
 
 namespace lct {
@@ -44,7 +45,9 @@ struct BpArgsDev {
   int slab_view[kBpMaxSlabs];
   int slab_z0[kBpMaxSlabs];
   int a_min[kBpMaxZ], a_mid[kBpMaxZ], a_max[kBpMaxZ];
-  float pitch;     // PI-window kernel only
+  float pitch, inv_pitch, inv_dso, inv_ds;  // PI-window kernel only (rounded reciprocals)
+  float row_scale;   // 2 (nt - 1) / pitch
+  int rows_centred;  // wt == (nt - 1) / 2 and pitch > 0
   int trig_table;  // PI-window kernel: 1 = every view's cos / sin staged in dynamic shared memory
 };
 
@@ -70,6 +73,20 @@ __device__ __forceinline__ ColSetup col_setup(float p_idx, int ns) {
     c.ok1 = (unsigned)(i + 1) < (unsigned)ns;
   }
   return c;
+}
+
+// Bilinear blend of a 2 x 2 texel block with weights a (columns) and b (rows; TEX8: before the
+// texture unit's rounding).
+template <int INTERP>
+__device__ __forceinline__ float blend(float a, float b, float v00, float v01, float v10, float v11) {
+  if (INTERP == LCT_INTERP_TEX8) {
+    float w00, w01, w10, w11;
+    tex_bilinear_weights(a, q8(b), w00, w01, w10, w11);
+    return fmaf(w11, v11, fmaf(w10, v10, fmaf(w01, v01, w00 * v00)));
+  }
+  const float top = fmaf(a, v01, (1.0f - a) * v00);
+  const float bot = fmaf(a, v11, (1.0f - a) * v10);
+  return fmaf(b, bot, (1.0f - b) * top);
 }
 
 // Bilinear sample of one view at column setup c and row coordinate q_idx (texel index).
@@ -371,28 +388,37 @@ __global__ void __launch_bounds__(kBpTX* kBpTY) bp_par_general_kernel(const __gr
 // own a_middle, its own stop of the backward walk (|t| > pitch / 4) and its own forward range, and
 // sums its views in the reference's order (backward from a_middle, then forward from
 // a_middle + 1), with the reference's expression for t (CUDA/Backprojector.cu:200-245).
+// Bound: instruction issue (114 instructions per sample with IEEE divisions, conversions and per-tap
+// border tests, one slice at a time).  Two slices run as one packed FP32 pair; the divisions by the
+// view's in-plane distance and by the pitch are remainder-corrected products with the rounded
+// reciprocal (div_by: the same quotients); floors come from round-down adds; a pair whose texels
+// all lie on the detector in every lane of the warp loads them without tests; a pair that no lane
+// of the warp needs in this view is skipped.  256^2 x 32 voxels x 577 views: 4.05 ms, 6.02 ms
+// before.
 constexpr int kPiNZ = 8;
+constexpr int kPiTX = 16, kPiTY = 16;
 constexpr int kPiTrigMaxViews = 12288;  // 96 KB of staged view trigonometry per CTA
 template <int INTERP, int ADDR>
-__global__ void __launch_bounds__(256) bp_pi_ori_z_kernel(const __grid_constant__ BpArgsDev A) {
+__global__ void __launch_bounds__(kPiTX* kPiTY, 4) bp_pi_ori_z_kernel(const __grid_constant__ BpArgsDev A) {
   extern __shared__ float2 s_trig[];  // trig_table: cos, sin of view v at s_trig[v]
-  const int ix = blockIdx.x * kBpTX + threadIdx.x;
-  const int iy = blockIdx.y * kBpTY + threadIdx.y;
+  const int ix = blockIdx.x * kPiTX + threadIdx.x;
+  const int iy = blockIdx.y * kPiTY + threadIdx.y;
   const int z0 = blockIdx.z * kPiNZ;
   if (A.trig_table) {  // once per CTA instead of once per thread and view; the same values
-    for (int v = threadIdx.y * kBpTX + threadIdx.x; v < A.n_angle; v += kBpTX * kBpTY) {
+    for (int v = threadIdx.y * kPiTX + threadIdx.x; v < A.n_angle; v += kPiTX * kPiTY) {
       float c, sn;
       view_trig_mode<INTERP>(A.betas, v, c, sn);
       s_trig[v] = make_float2(c, sn);
     }
     __syncthreads();
   }
-  if (ix >= A.nx || iy >= A.ny) return;
+  const bool present = ix < A.nx && iy < A.ny;  // absent threads walk along for the warp's votes
   const int nzc = min(kPiNZ, A.nz - z0);
   const float xc = ((float)ix - A.wx) * A.dx;
   const float yc = ((float)iy - A.wy) * A.dy;
   const float pitch = A.pitch;
   const float t2 = (float)((double)pitch / (2 * kRefPi));  // :209, double through PI
+  const float rows2 = (float)(2 * (A.nt - 1));  // t * 2 * (nt - 1): the doubling is exact
   float zc[kPiNZ], sum[kPiNZ];
   int amid[kPiNZ], amin[kPiNZ];
   unsigned walking = 0;  // bit j: slice j's backward walk has not stopped
@@ -407,15 +433,17 @@ __global__ void __launch_bounds__(256) bp_pi_ori_z_kernel(const __grid_constant_
     amin[j] = -1;
     sum[j] = 0.0f;
     if (j < nzc) {
-      walking |= 1u << j;
+      if (present) walking |= 1u << j;
       vtop = max(vtop, a);
     }
   }
   // the slice-invariant terms of view v
   struct ViewTerms {
-    float temp1, gt2, den;
+    float temp1, gt2, gz, den, rden, zv;  // temp1 and gz = gt2 carry the table direction's sign
     ColSetup c;
     const float* view;
+    const float* p0;  // column c0 of row 0
+    bool cols;        // both columns on the detector, in every lane of the warp
   };
   auto terms = [&](int v) {
     ViewTerms w;
@@ -428,54 +456,139 @@ __global__ void __launch_bounds__(256) bp_pi_ori_z_kernel(const __grid_constant_
       view_trig_mode<INTERP>(A.betas, v, cb, sb);
     }
     const float s = -xc * cb - yc * sb;
-    const float gamma = asinf(s / A.dso);
-    w.temp1 = sqrtf(A.dso * A.dso - s * s);
+    const float gamma = asinf(div_by(s, A.dso, A.inv_dso));
+    const float temp1 = sqrtf(A.dso * A.dso - s * s);
     w.gt2 = gamma * t2;
-    w.den = w.temp1 + xc * sb - yc * cb;
-    w.c = col_setup<INTERP, ADDR>(s / A.ds + A.ws, A.ns);
+    w.den = temp1 + xc * sb - yc * cb;
+    w.temp1 = temp1 * A.zdir;
+    w.gz = w.gt2 * A.zdir;
+    w.rden = __frcp_rn(w.den);
+    w.zv = A.z0 + A.dzv * (float)v;
+    w.c = col_setup<INTERP, ADDR>(div_by(s, A.ds, A.inv_ds) + A.ws, A.ns);
+    w.cols = __all_sync(0xffffffffu, w.c.ok0 && w.c.ok1 && w.c.c1 == w.c.c0 + 1);
     w.view = A.proj + (long long)v * A.view_stride;
+    w.p0 = w.view + w.c.c0;
     return w;
   };
-  auto tval = [&](const ViewTerms& w, float zcj, int v) {
-    const float zoff = zcj - (A.z0 + A.dzv * (float)v);
-    float t = w.temp1 * (zoff - w.gt2) / w.den + w.gt2;
-    return t * A.zdir;
+  // slices j and j + 1 of view w: t of both (the reference's expression, times the direction's sign)
+  auto tval2 = [&](const ViewTerms& w, int j) {
+    const float2 z = make_float2(zc[j], zc[j + 1]);
+    const float2 x = __fmul2_rn(f2(w.temp1), __fadd2_rn(__fadd2_rn(z, f2(-w.zv)), f2(-w.gt2)));
+    return __fadd2_rn(div_by2(x, w.den, w.rden), f2(w.gz));
   };
-  // backward walks, views descending; slice j joins at its a_middle
-  for (int v = vtop; v >= 0 && walking; --v) {
-    const ViewTerms w = terms(v);
+  // row coordinates: TEX8 the reference's expression, whose rounding decides 8-bit weights; EXACT one FMA
+  auto rows_of = [&](float2 t) {
+    if (INTERP == LCT_INTERP_EXACT) return __ffma2_rn(t, f2(A.row_scale), f2(A.wt));
+    return __fadd2_rn(div_by2(__fmul2_rn(t, f2(rows2)), pitch, A.inv_pitch), f2(A.wt));
+  };
+  // adds both samples where |t| <= tin in every lane of the warp: their rows then lie on the detector
+  auto add_inside = [&](const ViewTerms& w, int j, float2 it) {
+    if (INTERP == LCT_INTERP_TEX8) it = __fadd2_rn(__fadd2_rn(it, f2(0.5f)), f2(-0.5f));
+    const float2 m = __fadd2_rd(it, f2(kFloorMagic));
+    const float2 b = f2sub(it, __fadd2_rn(m, f2(-kFloorMagic)));
+    auto sample = [&](float row, float bb) {
+      const float* p = w.p0 + (long long)(__float_as_int(row) - kFloorBits) * A.ns;
+      const float* q = p + A.ns;
+      const float v00 = __ldg(p), v01 = __ldg(p + 1), v10 = __ldg(q), v11 = __ldg(q + 1);
+      if (INTERP == LCT_INTERP_TEX8) return blend<INTERP>(w.c.a, bb, v00, v01, v10, v11);
+      const float top = fmaf(w.c.a, v01 - v00, v00), bot = fmaf(w.c.a, v11 - v10, v10);
+      return fmaf(bb, bot - top, top);
+    };
+    sum[j] += sample(m.x, b.x);
+    sum[j + 1] += sample(m.y, b.y);
+  };
+  auto add_masked = [&](const ViewTerms& w, int j, float2 it, bool add0, bool add1) {
+    if (add0) sum[j] += sample_rows<INTERP, ADDR>(w.view, A.ns, A.nt, w.c, it.x);
+    if (add1) sum[j + 1] += sample_rows<INTERP, ADDR>(w.view, A.ns, A.nt, w.c, it.y);
+  };
+  const float stop = pitch / 4;
+  // the row coordinate is wt + 2 (nt - 1) t / pitch: |t| a few roundings below pitch / 4 keeps both
+  // rows of a sample in [0, nt - 1] when wt is the central row (A.rows_centred)
+  const float tin = A.rows_centred ? stop * (1.0f - 8e-6f) : -1.0f;
+  constexpr unsigned kAll = (1u << kPiNZ) - 1u;
+  int alo = INT_MAX, ahi = INT_MIN;  // the slices' a_middle lie in [alo, ahi]
 #pragma unroll
-    for (int j = 0; j < kPiNZ; ++j) {
-      if (!((walking >> j) & 1u) || v > amid[j]) continue;
-      const float t = tval(w, zc[j], v);
-      if (t > pitch / 4 || t < -pitch / 4) {
-        walking &= ~(1u << j);
-        amin[j] = v;
+  for (int j = 0; j < kPiNZ; ++j)
+    if (j < nzc) {
+      alo = min(alo, amid[j]);
+      ahi = max(ahi, amid[j]);
+    }
+  // backward walks, views descending; slice j joins at its a_middle
+  for (int v = vtop; v >= 0; --v) {
+    const bool steady = v <= alo && __all_sync(0xffffffffu, walking == kAll);
+    unsigned need = walking, any = kAll;
+    if (!steady) {
+      if (v > alo) {
+#pragma unroll
+        for (int j = 0; j < kPiNZ; ++j)
+          if (v > amid[j]) need &= ~(1u << j);
+      }
+      any = __reduce_or_sync(0xffffffffu, need);
+      if (!any) {
+        if (!__any_sync(0xffffffffu, walking != 0)) break;
         continue;
       }
-      const float it = t * 2 * (A.nt - 1) / pitch + A.wt;
-      sum[j] += sample_rows<INTERP, ADDR>(w.view, A.ns, A.nt, w.c, it);
+    }
+    const ViewTerms w = terms(v);
+#pragma unroll
+    for (int j = 0; j < kPiNZ; j += 2) {
+      if (!((any >> j) & 3u)) continue;
+      const float2 t = tval2(w, j);
+      const bool far0 = t.x > stop || t.x < -stop, far1 = t.y > stop || t.y < -stop;
+      const float2 it = rows_of(t);
+      if (w.cols && __all_sync(0xffffffffu, fabsf(t.x) <= tin && fabsf(t.y) <= tin && ((need >> j) & 3u) == 3u)) {
+        add_inside(w, j, it);
+        continue;
+      }
+      bool add0 = (need >> j) & 1u, add1 = (need >> (j + 1)) & 1u;
+      if (add0 && far0) {
+        walking &= ~(1u << j);
+        amin[j] = v;
+        add0 = false;
+      }
+      if (add1 && far1) {
+        walking &= ~(1u << (j + 1));
+        amin[j + 1] = v;
+        add1 = false;
+      }
+      add_masked(w, j, it, add0, add1);
     }
   }
   // forward: views a_middle + 1 .. a_min + half (the reference has no bound against n_angle,
   // :225; views past the end would sample outside the array, which reads as 0 -- left out)
-  int vlo = INT_MAX, vhi = -1;
+  int vlo = INT_MAX, vhi = -1, vall = INT_MAX;  // every slice of every lane takes (ahi, vall]
 #pragma unroll
   for (int j = 0; j < kPiNZ; ++j)
     if (j < nzc) {
       vlo = min(vlo, amid[j] + 1);
-      vhi = max(vhi, min(amin[j] + A.half, A.n_angle - 1));
+      if (present) vhi = max(vhi, min(amin[j] + A.half, A.n_angle - 1));
+      vall = min(vall, amin[j] + A.half);
     }
+  vhi = __reduce_max_sync(0xffffffffu, vhi);
+  vall = __reduce_min_sync(0xffffffffu, nzc == kPiNZ && present ? vall : -1);
   for (int v = vlo; v <= vhi; ++v) {
+    unsigned need = kAll, any = kAll;
+    if (v <= ahi || v > vall) {
+      need = 0;
+#pragma unroll
+      for (int j = 0; j < kPiNZ; ++j)
+        if (j < nzc && v >= amid[j] + 1 && v <= amin[j] + A.half) need |= 1u << j;
+      if (!present) need = 0;
+      any = __reduce_or_sync(0xffffffffu, need);
+      if (!any) continue;
+    }
     const ViewTerms w = terms(v);
 #pragma unroll
-    for (int j = 0; j < kPiNZ; ++j) {
-      if (j >= nzc || v < amid[j] + 1 || v > amin[j] + A.half) continue;
-      const float t = tval(w, zc[j], v);
-      const float it = t * 2 * (A.nt - 1) / pitch + A.wt;
-      sum[j] += sample_rows<INTERP, ADDR>(w.view, A.ns, A.nt, w.c, it);
+    for (int j = 0; j < kPiNZ; j += 2) {
+      if (!((any >> j) & 3u)) continue;
+      const float2 t = tval2(w, j), it = rows_of(t);
+      if (w.cols && __all_sync(0xffffffffu, fabsf(t.x) <= tin && fabsf(t.y) <= tin && ((need >> j) & 3u) == 3u))
+        add_inside(w, j, it);
+      else
+        add_masked(w, j, it, (need >> j) & 1u, (need >> (j + 1)) & 1u);
     }
   }
+  if (!present) return;
 #pragma unroll
   for (int j = 0; j < kPiNZ; ++j)
     if (j < nzc)
@@ -510,6 +623,11 @@ static void fill_common(BpArgsDev& d, const lct_geom& g, const lct_img& ig) {
   d.half = g.n_proj_turn / 2;  // CUDA/Backprojector.cu:148
   d.view_stride = (long long)g.nt * g.ns;
   d.pitch = g.pitch;
+  d.inv_pitch = 1.0f / g.pitch;
+  d.row_scale = (float)(2.0 * (g.nt - 1) / (double)g.pitch);
+  d.rows_centred = g.pitch > 0.f && g.wt == 0.5f * (float)(g.nt - 1) && g.nt < 4096;
+  d.inv_dso = 1.0f / g.dso;
+  d.inv_ds = 1.0f / g.ds;
 }
 
 template <int NZ, int INTERP, int ADDR>
@@ -667,8 +785,8 @@ LCT_API int lct_backproject_pi_ori(const lct_geom* g, const lct_img* ig, const f
   a.betas = d_betas;
   a.img = d_img;
   a.nz = ig->nz;
-  dim3 grid((ig->nx + kBpTX - 1) / kBpTX, (ig->ny + kBpTY - 1) / kBpTY, (ig->nz + kPiNZ - 1) / kPiNZ);
-  dim3 block(kBpTX, kBpTY);
+  dim3 grid((ig->nx + kPiTX - 1) / kPiTX, (ig->ny + kPiTY - 1) / kPiTY, (ig->nz + kPiNZ - 1) / kPiNZ);
+  dim3 block(kPiTX, kPiTY);
   cudaStream_t s = (cudaStream_t)stream;
   bool tex = interp == LCT_INTERP_TEX8, clamp = addr == LCT_ADDR_CLAMP;
   // the view trig table in shared memory (8 bytes per view) up to kPiTrigMaxViews views; longer

@@ -28,6 +28,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "fp32_pair.cuh"
 #include "lct_internal.h"
 #include "tc_ptx.cuh"
 #include "tex_emul.cuh"
@@ -146,38 +147,23 @@ __device__ __forceinline__ const float4* quad_view_ptr(const BpQuadArgs& A, int 
   return A.quads + v * A.qstride;
 }
 
-// EXACT floor without conversions: for |x| < 2^22, x + 1.5 * 2^23 rounded toward -inf is
-// 1.5 * 2^23 + floor(x) exactly, so its bit pattern is kMagicBits + floor(x) and subtracting the
-// constant back (exact: both operands lie within a factor of two) gives floor(x).  Outside that
-// range the bit pattern still orders like x, so a clamp on it clamps floor(x).
-constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
-constexpr int kMagicBits = 0x4B400000;
-
-// view base biased so that a column bit pattern (clamped to kMagicBits + [-2, ns]) times 16 and a
+// view base biased so that a column bit pattern (clamped to kFloorBits + [-2, ns]) times 16 and a
 // row bit pattern times the row pitch add up to the quad's address, one wide multiply-add per
-// sample; rows are clamped to kMagicBits + [0, nt + 2]
-// (EXACT, whose row coordinate carries + 2) or kMagicBits + [-2, nt] (TEX8)
+// sample; rows are clamped to kFloorBits + [0, nt + 2]
+// (EXACT, whose row coordinate carries + 2) or kFloorBits + [-2, nt] (TEX8)
 template <int INTERP>
 __device__ __forceinline__ unsigned long long quad_view_bias(const float4* view, unsigned qrow_bytes) {
-  constexpr int kRow0 = INTERP == LCT_INTERP_TEX8 ? kMagicBits - 2 : kMagicBits;
-  return reinterpret_cast<unsigned long long>(view) - (unsigned long long)(kMagicBits - 2) * 16ull -
+  constexpr int kRow0 = INTERP == LCT_INTERP_TEX8 ? kFloorBits - 2 : kFloorBits;
+  return reinterpret_cast<unsigned long long>(view) - (unsigned long long)(kFloorBits - 2) * 16ull -
          (unsigned long long)kRow0 * qrow_bytes;
-}
-
-// Blackwell's packed FP32 pairs (FFMA2, FADD2, FMUL2): one instruction for two lanes, each lane
-// rounded exactly as the scalar operation; x - y is written fma(y, -1, x), one rounding like the
-// subtraction.
-__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 f2sub(float2 x, float2 y) {
-  return __ffma2_rn(y, make_float2(-1.0f, -1.0f), x);
 }
 
 // column p: weight a (the fraction) and 16 * (clamped column bit pattern) added to the biased view base
 __device__ __forceinline__ unsigned long long quad_col(unsigned long long vbias, float p,
                                                              int ns, float& a) {
-  const float t = __fadd_rd(p, kMagic);
-  a = p - (t - kMagic);
-  const int cb = min(max(__float_as_int(t), kMagicBits - 2), kMagicBits + ns);
+  const float t = __fadd_rd(p, kFloorMagic);
+  a = p - (t - kFloorMagic);
+  const int cb = min(max(__float_as_int(t), kFloorBits - 2), kFloorBits + ns);
   return vbias + (unsigned long long)(unsigned)cb * 16ull;
 }
 
@@ -234,17 +220,6 @@ __device__ __forceinline__ float asin_half(float x) {
                                  0.04546250030398369f), t, 0.07495353370904922f), t,
                        0.16666752099990845f);
   return fmaf(__fmul_rn(x, t), p, x);
-}
-
-// x / d rounded to nearest for a launch-constant d with r = RN(1 / d): the quotient estimate's
-// remainder is exact in an FMA and one more FMA rounds correctly (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34(1), 1990), except
-// that a divisor whose fraction bits are all ones may leave a power of two one ulp off; 3
-// operations where a division by a variable is a subroutine.  tests/test_div_by.py compares every
-// fraction of x with the division.
-__device__ __forceinline__ float div_by(float x, float d, float r) {
-  const float q = __fmul_rn(x, r);
-  return fmaf(fmaf(-q, d, x), r, q);
 }
 
 // One tile: voxel columns [bx*kQTX, +kQTX) x [by*kQTY, +kQTY), slab/slice chunk bz.  Called with
@@ -431,11 +406,11 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
           y = __ffma2_rn(J, K, U);
         else
           y = __fadd2_rn(__fadd2_rn(__fadd2_rn(qh, f2(wt)), f2(0.5f)), f2(-0.5f));
-        const float2 t = __fadd2_rd(y, f2(kMagic));
-        const float2 b = f2sub(y, __fadd2_rn(t, f2(-kMagic)));
+        const float2 t = __fadd2_rd(y, f2(kFloorMagic));
+        const float2 b = f2sub(y, __fadd2_rn(t, f2(-kFloorMagic)));
         int r1 = __float_as_int(t.x), r2 = __float_as_int(t.y);
         if constexpr (!kIn) {
-          constexpr int kRow0 = INTERP == LCT_INTERP_TEX8 ? kMagicBits - 2 : kMagicBits;
+          constexpr int kRow0 = INTERP == LCT_INTERP_TEX8 ? kFloorBits - 2 : kFloorBits;
           r1 = min(max(r1, kRow0), kRow0 + A.nt + 2);
           r2 = min(max(r2, kRow0), kRow0 + A.nt + 2);
         }
@@ -464,8 +439,8 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
           // T00 + a dx + b dy + w11 dxy with b = round-half-up of the fraction and w11 =
           // round-half-up(a b), both on the 1/256 grid: B = 256 b and W = 256 w11 are the whole
           // parts of exact sums (the quads' row differences carry the 1/256)
-          const float2 B = __fadd2_rn(__fadd2_rd(__ffma2_rn(b, f2(256.0f), f2(0.5f)), f2(kMagic)), f2(-kMagic));
-          const float2 W = __fadd2_rn(__fadd2_rd(__ffma2_rn(make_float2(a1, a2), B, f2(0.5f)), f2(kMagic)), f2(-kMagic));
+          const float2 B = __fadd2_rn(__fadd2_rd(__ffma2_rn(b, f2(256.0f), f2(0.5f)), f2(kFloorMagic)), f2(-kFloorMagic));
+          const float2 W = __fadd2_rn(__fadd2_rd(__ffma2_rn(make_float2(a1, a2), B, f2(0.5f)), f2(kFloorMagic)), f2(-kFloorMagic));
           const float s1 = fmaf(W.x, v0.w, fmaf(B.x, v0.y, fmaf(a1, v0.z, v0.x)));
           const float s2 = fmaf(W.y, v1.w, fmaf(B.y, v1.y, fmaf(a2, v1.z, v1.x)));
           sum = fmaf(w1, s1, fmaf(w2, s2, acc[j]));
@@ -688,11 +663,11 @@ __device__ __forceinline__ void bp_tma_tile(const BpQuadArgs& A, const CUtensorM
       const unsigned long long q1 = quad_col(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
       const unsigned long long q2 = quad_col(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
       // the thread's quad columns (0 .. ns + 2) and its first / last slice's quad rows
-      const int qc1 = (int)((q1 - qv.x) >> 4) - (kMagicBits - 2);
-      const int qc2 = (int)((q2 - qv.y) >> 4) - (kMagicBits - 2);
+      const int qc1 = (int)((q1 - qv.x) >> 4) - (kFloorBits - 2);
+      const int qc2 = (int)((q2 - qv.y) >> 4) - (kFloorBits - 2);
       auto qrow = [&](float u) {
-        const int rb = __float_as_int(__fadd_rd(u, kMagic));
-        return min(max(rb, kMagicBits), kMagicBits + A.nt + 2) - kMagicBits;
+        const int rb = __float_as_int(__fadd_rd(u, kFloorMagic));
+        return min(max(rb, kFloorBits), kFloorBits + A.nt + 2) - kFloorBits;
       };
       const int4 bo = s_box[k];
       bool in_box = false;
@@ -710,15 +685,15 @@ __device__ __forceinline__ void bp_tma_tile(const BpQuadArgs& A, const CUtensorM
       // shared-memory bases biased like the global ones: + row bit pattern * row bytes
       const uint32_t sbase = stage0 + st * kTmaStageBytes;
       const uint32_t sbv = sbase + 16u * (uint32_t)(qc1 - bo.y) -
-                           (uint32_t)(kMagicBits + bo.x) * kTmaRowBytes;
+                           (uint32_t)(kFloorBits + bo.x) * kTmaRowBytes;
       const uint32_t sbc = sbase + kTmaBoxBytes + 16u * (uint32_t)(qc2 - bo.w) -
-                           (uint32_t)(kMagicBits + bo.z) * kTmaRowBytes;
+                           (uint32_t)(kFloorBits + bo.z) * kTmaRowBytes;
       auto sample = [&](bool smem, bool clamp, unsigned long long gq, uint32_t sq0, float a,
                         float u) -> float {
-        const float t = __fadd_rd(u, kMagic);
-        const float b = u - (t - kMagic);
+        const float t = __fadd_rd(u, kFloorMagic);
+        const float b = u - (t - kFloorMagic);
         int rb = __float_as_int(t);
-        if (clamp) rb = min(max(rb, kMagicBits), kMagicBits + A.nt + 2);
+        if (clamp) rb = min(max(rb, kFloorBits), kFloorBits + A.nt + 2);
         const float4 v = smem ? lds128(sq0 + (uint32_t)rb * kTmaRowBytes)
                               : __ldg(reinterpret_cast<const float4*>(
                                     gq + (unsigned long long)(unsigned)rb * A.qrow_bytes));
