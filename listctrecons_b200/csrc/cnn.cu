@@ -5,20 +5,27 @@
 // 3x3 convolutions (5->32, 6 x 32->32, 32->1), ReLU between them -> a residual r added to the
 // centre slice.  BF16 weights and activations, FP32 accumulation.
 //
-// HBM layout: every activation / delta is channels-last bf16 [B][H][W+2][32] (64 bytes per
-// pixel; one zero pad column on each side, pixel x at column x+1; channels beyond a layer's
-// width are zero).  Weights are packed per layer as bf16 [N][9 taps x 32 channels].
+// HBM layout: every activation / delta is bf16 [B][H + 2][4][wp][8]: per padded row four planes of
+// eight channels, 16 bytes per pixel and plane; pixel x of row y at column x + 1 of row y + 1, wp = W + 2
+// rounded up to 8.  Rows 0 and H + 1 and the columns outside the image stay zero.  The network input has one plane (5 channels, 3 zero).  A
+// staged tile is one TMA box, and in shared memory eight pixels of a plane are one unswizzled core
+// matrix: an operand may start at any pixel, so ONE box serves all nine taps.  (TMA sees 8-byte
+// elements, two per pixel, in blocks of 8 pixels where a box is wider than 128.)
+// Weights are packed per layer as bf16 [32][9 taps x 32 channels].
 //
-// Convolution = implicit GEMM on tcgen05 in a persistent, warp-specialised kernel: a tile is
-// 8 px x 16 rows (M 128) x N output channels (N = 32, or 16 for the 1-channel last layer) over
-// K = 9 taps x 32 channels.  Per tile, three 4-D TMA boxes {32 ch, 8 px, 18 rows, 1 slice} with
-// 64-byte swizzle (one per column offset; rows outside the image come back as TMA's zero fill)
-// serve all nine taps, each row offset being a whole swizzle atom; the packed weights
-// (9 x N x 64 bytes) are loaded once per CTA; two M128 x N x K16 MMAs per tap accumulate in one
-// of two TMEM buffers.  Fused epilogues: bias + ReLU -> bf16 (forward), ReLU mask of the
-// previous activation -> bf16 delta (backward data), FP32 residual (training), and the
-// acceptance gate writing the corrected volume (inference).
-// Weight gradients: the same tcgen05 machinery with K = pixels (both operands MN-major).
+// Convolution on tcgen05, persistent and warp-specialised: a tile is 8 output rows x up to 128 pixels.
+// Pixels are the M operand, and the three vertical taps of one column offset the N operand: input row r
+// (of ten), column offset dx and 16 channels are ONE M128 x N96 x K16 MMA that adds tap (dy, dx) to the
+// accumulators of output rows r - 2, r - 1 and r, 32 columns apart in tensor memory, so a pixel's
+// channels are read from shared memory 3 x 10 / 8 times instead of 9 (N64 and N32 at the tile's edges).
+// Two buffers of 8 x 32 columns fill tensor memory; the packed weights sit in shared memory for the
+// CTA's lifetime.  Per output the taps add in the order (dx, dy, channel half).
+// Bound: shared-memory operand reads (7 KB per MMA), then HBM.  512 x 512, 32 slices: 190 us per
+// hidden layer; one tap per MMA (M128 x N32, three boxes per tile) 308 us.
+// Fused epilogues: bias + ReLU -> bf16 (forward), ReLU mask of the previous activation -> bf16 delta
+// (backward data), FP32 residual (training), and the acceptance gate writing the corrected volume
+// (inference).
+// Weight gradients: tcgen05 with K = pixels (both operands MN-major from the same layout).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -35,10 +42,13 @@ namespace lct {
 constexpr int kCnnLayers = 8, kCnnC = 32, kCnnTaps = 9, kCnnK = kCnnTaps * kCnnC;  // K = 288
 constexpr int kCnnParams = 57249;     // sum over layers of cin*cout*9 + cout
 constexpr int kWSlot = kCnnC * kCnnK;  // packed weights of one layer, elements
-// output tile 8 px x 16 rows = the M 128 of one MMA; M row m = row * 8 + px
-constexpr int kConvTW = 8, kConvTH = 16, kConvM = kConvTW * kConvTH;
-constexpr int kConvStages = 6;    // A boxes in flight (3 per tile)
-constexpr int kConvThreads = 192; // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 epilogue
+constexpr int kConvRows = 8;      // output rows of a tile
+constexpr int kConvIn = kConvRows + 2;
+constexpr int kConvMaxN = 128;    // pixels of a tile, a multiple of 8 (its box starts on a block)
+constexpr int kConvThreads = 320; // warp 0 copies, warp 1 MMA + TMEM, warps 2-9 epilogue
+constexpr int kConvMaxStages = 8;
+constexpr uint32_t kConvZero = 128 * 16 + 32;  // a plane of zeros for the network input's absent channels
+constexpr uint32_t kSmemMax = 226 * 1024;      // dynamic shared memory of the CNN kernels
 
 LCT_HD constexpr int cnn_cin(int l) { return l == 0 ? 5 : 32; }
 LCT_HD constexpr int cnn_cout(int l) { return l == kCnnLayers - 1 ? 1 : 32; }
@@ -47,265 +57,276 @@ LCT_HD constexpr int cnn_off(int l) { return l == 0 ? 0 : 1472 + (l - 1) * 9248;
 enum ConvEpi : int { kEpiRelu = 0, kEpiMask = 1, kEpiResid = 2, kEpiGate = 3 };
 
 struct ConvArgs {
-  int H, W, wp, tiles_x, tiles_y;
+  int H, W, wp, n_px, tiles_x, tiles_y, stages;
+  int rows;                        // output rows of a tile
+  uint32_t stage_bytes;
   long long n_tiles;
-  const float* bias;               // [N] (forward epilogues)
-  __nv_bfloat16* out_act;          // Relu / Mask: [B][H][wp][32]
-  const __nv_bfloat16* mask_act;   // Mask: activation whose sign gates the delta
+  const __nv_bfloat16* w;          // packed weights
+  const float* bias;               // [32] (forward epilogues; [1] for the last layer)
   float* out_f;                    // Resid: r [B][H][W]; Gate: corrected slices [B][H][W]
   const float* xc;                 // Gate: plain slices [B][H][W]
+  __nv_bfloat16* out_act;          // Relu / Mask: [B][H + 2][4][wp][8]
+  const __nv_bfloat16* mask_act;   // Mask: activation whose sign gates the delta
   float calib, inv_scale, bound;   // Gate
   unsigned long long* n_reject;    // Gate
   int* status;
-};
-
-template <int N>
-struct ConvCfg {
-  // one A box: 32 channels x 8 px x 18 rows (the tile's rows and one halo row on each side)
-  static constexpr uint32_t BoxA = kConvTW * (kConvTH + 2) * kCnnC * 2;  // 9216 B
-  static constexpr uint32_t RowA = kConvTW * kCnnC * 2;                  // 512 B = one atom
-  static constexpr uint32_t TapB = N * kCnnC * 2;        // 2 KB (N=32) or 1 KB (N=16)
-  static constexpr uint32_t BBytes = kCnnTaps * TapB;
-  static constexpr uint32_t Smem = 1024 + kConvStages * BoxA + BBytes + 256;
-  static constexpr uint32_t TmemCols = 64;  // two 32-column accumulators
-  static constexpr uint32_t Idesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                                    ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kConvM >> 4) << 24);
 };
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
-__device__ __forceinline__ void conv_tile(const ConvArgs& a, long long t, int& x0, int& y0,
-                                          int& b) {
+// tile t: slice b, first output row y0, first pixel x0
+__device__ __forceinline__ void conv_tile(const ConvArgs& a, long long t, int& x0, int& y0, int& b) {
   const long long per = (long long)a.tiles_x * a.tiles_y;
   b = (int)(t / per);
   const int r = (int)(t % per);
-  y0 = (r / a.tiles_x) * kConvTH;
-  x0 = (r % a.tiles_x) * kConvTW;
+  y0 = (r / a.tiles_x) * a.rows;
+  x0 = (r % a.tiles_x) * a.n_px;
 }
 
 __device__ __forceinline__ bool conv_aborted(int* flag) {
   return *reinterpret_cast<volatile int*>(flag) != 0;
 }
 
-// Persistent implicit-GEMM 3x3 convolution: CTA c takes tiles c, c + grid, ...  Per tile, three
-// A boxes (one per column offset dx) feed nine taps: tap (dy, dx) reads box dx from row dy,
-// i.e. at +dy * 512 bytes -- a whole 64-byte-swizzle atom, so every operand start stays on the
-// swizzle pattern.  Two TMEM accumulators let the epilogue of one tile overlap the MMAs of the
-// next.  Every wait is bounded; on a timeout the CTA drains its copies and MMAs, raises the
-// device status word and leaves its remaining tiles unwritten.
-template <int N, int EPI>
-__global__ void __launch_bounds__(kConvThreads, 3)
-    conv_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
-                   const ConvArgs a) {
-  using Cfg = ConvCfg<N>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* sa = smem;
-  uint8_t* sb = smem + kConvStages * Cfg::BoxA;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sb + Cfg::BBytes);
-  // full[S] empty[S] wbar acc_full[2] acc_empty[2] mma_done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kConvStages + 6);
+// bytes of a plane of a staged row: a convolution's (the pixels and a block of 8), a gradient's
+// activation (the pixels and one on each side)
+LCT_HD constexpr uint32_t conv_plane(int n_px) { return (uint32_t)(n_px + 8) * 16; }
+LCT_HD constexpr uint32_t dw_plane(int n_px) { return (uint32_t)(n_px + 2) * 16; }
+
+// PLANES: planes of the input (1: the network input, whose channels 8..15 read a zeroed plane of
+// shared memory and whose second half of 16 channels does not exist; 4: an activation).
+// Every wait is bounded; on a timeout the CTA drains its copies and MMAs, raises the device status
+// word and leaves its remaining tiles unwritten.
+template <int EPI, int PLANES>
+__global__ void __launch_bounds__(kConvThreads, 1)
+    conv_tc_kernel(const __grid_constant__ CUtensorMap mbox, const ConvArgs a) {
+  constexpr bool kLast = EPI == kEpiResid || EPI == kEpiGate;
+  constexpr int kHalves = PLANES == 1 ? 1 : 2;  // K16 steps per tap
+  constexpr int kCo = kLast ? 16 : 32;          // accumulator columns of an output row
+  constexpr uint32_t kBuf = kConvRows * kCo;    // columns of a buffer
+  constexpr uint32_t kTmem = 2 * kBuf;
+  constexpr uint32_t kWPlane = 3 * kCo * 16, kWBlock = 2 * kWPlane;  // weights of (dx, half), [2][3 kCo][8]
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ __align__(8) uint64_t bars[2 * kConvMaxStages + 5];
+  __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
-  __shared__ float s_bias[32];  // the layer's biases, read by every tile's epilogue
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t full0 = smem_u32(&bars[0]);
-  const uint32_t empty0 = smem_u32(&bars[kConvStages]);
-  const uint32_t wbar = smem_u32(&bars[2 * kConvStages]);
-  const uint32_t accf0 = smem_u32(&bars[2 * kConvStages + 1]);
-  const uint32_t acce0 = smem_u32(&bars[2 * kConvStages + 3]);
-  const uint32_t mdone = smem_u32(&bars[2 * kConvStages + 5]);
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int N = a.n_px, S = a.stages;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kConvMaxStages]);
+  const uint32_t accf0 = smem_u32(&bars[2 * kConvMaxStages]), acce0 = accf0 + 16, mdone = accf0 + 32;
+  // stages, (PLANES 1) the zero plane, weights; an operand's rows past the tile's pixels read on into
+  // what follows, which only reaches accumulator rows that are not stored
+  const uint32_t cs = conv_plane(N), rs = PLANES * cs;
+  const uint32_t stage0 = smem_u32(smem), zero0 = stage0 + (uint32_t)S * a.stage_bytes;
+  const uint32_t w0 = zero0 + (PLANES == 1 ? kConvZero : 0u);
 
-  if (threadIdx.x < 32)
-    s_bias[threadIdx.x] = (EPI != kEpiMask && threadIdx.x < N) ? a.bias[threadIdx.x] : 0.f;
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int s = 0; s < kConvStages; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
-    mbar_init(wbar, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(accf0 + 8 * i, 1);
-      mbar_init(acce0 + 8 * i, 4);  // one arrival per epilogue warp
+      mbar_init(acce0 + 8 * i, 8);  // one arrival per epilogue warp
     }
     mbar_init(mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (PLANES == 1)
+    for (uint32_t i = threadIdx.x * 16; i < kConvZero; i += kConvThreads * 16)
+      *reinterpret_cast<uint4*>(smem + (zero0 - stage0) + i) = make_uint4(0u, 0u, 0u, 0u);
+  // weights: block (dx, half), plane of 8 channels, row (2 - dy) kCo + co
+  for (int i = threadIdx.x; i < 3 * kHalves * 2 * 3 * kCo; i += kConvThreads) {
+    const int row = i % (3 * kCo), c = i / (3 * kCo) % 2, blk = i / (6 * kCo);
+    const int dy = 2 - row / kCo, co = row % kCo, dx = blk / kHalves, h = blk % kHalves;
+    *reinterpret_cast<uint4*>(smem + (w0 - stage0) + blk * kWBlock + c * kWPlane + row * 16) =
+        __ldg(reinterpret_cast<const uint4*>(a.w + co * kCnnK + (dy * 3 + dx) * kCnnC + 16 * h + 8 * c));
+  }
+  fence_async_smem();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "r"(Cfg::TmemCols)
+                     smem_u32(&tmem_slot)),
+                 "r"(kTmem)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_slot, 0);  // uniform to the compiler
+  if (warp >= 2) {  // accumulators start at zero, and the epilogue leaves them so
+    for (uint32_t c = warp < 6 ? 0 : kBuf; c < (warp < 6 ? kBuf : kTmem); c += 16)
+      tmem_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c);
+    tmem_wait_st();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 
   if (warp == 0) {
+    // producer: one box per tile (rows and columns outside the padded image read as zero)
     if (lane == 0) {
-      // producer: the layer's packed weights once, then three A boxes per tile
-      mbar_expect_tx(wbar, Cfg::BBytes);
-      for (int k = 0; k < kCnnTaps; ++k)
-        tma_load_2d(smem_u32(sb + k * Cfg::TapB), &mw, k * kCnnC, 0, wbar);
-      long long kg = 0;
-      bool stop = false;
-      for (long long t = blockIdx.x; t < a.n_tiles && !stop; t += gridDim.x) {
+      long long k = 0;
+      for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
         int x0, y0, b;
         conv_tile(a, t, x0, y0, b);
-        for (int l = 0; l < 3; ++l, ++kg) {
-          const int s = (int)(kg % kConvStages);
-          if (kg >= kConvStages &&
-              !mbar_wait(empty0 + 8 * s, (uint32_t)(((kg / kConvStages) - 1) & 1))) {
-            atomicExch(&s_abort, 1);
-            stop = true;
-            break;
-          }
-          if (conv_aborted(&s_abort)) {
-            stop = true;
-            break;
-          }
-          mbar_expect_tx(full0 + 8 * s, Cfg::BoxA);
-          // pixel x of the tile, column offset dx = l - 1, sits at padded column x + l
-          tma_load_4d(smem_u32(sa + s * Cfg::BoxA), &mx, 0, x0 + l, y0 - 1, b, full0 + 8 * s);
-        }
-      }
-      if (conv_aborted(&s_abort)) {  // let copies in flight land before the CTA exits
-        mbar_wait(wbar, 0);
-        for (long long k = (kg > kConvStages ? kg - kConvStages : 0); k < kg; ++k)
-          mbar_wait(full0 + 8 * (int)(k % kConvStages), (uint32_t)((k / kConvStages) & 1));
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // MMA issuer
-      bool ok = mbar_wait(wbar, 0);
-      if (!ok) atomicExch(&s_abort, 1);
-      long long kg = 0;
-      int it = 0;
-      for (long long t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x, ++it) {
-        const int buf = it & 1;
-        if (it >= 2 && !mbar_wait(acce0 + 8 * buf, (uint32_t)(((it >> 1) - 1) & 1))) {
+        const int s = (int)(k % S);
+        if (k >= S && !mbar_wait(empty0 + 8 * s, (uint32_t)(((k / S) - 1) & 1))) {
           atomicExch(&s_abort, 1);
           break;
         }
         if (conv_aborted(&s_abort)) break;
-        tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(buf * 32);
-        for (int l = 0; l < 3 && ok; ++l, ++kg) {
-          const int s = (int)(kg % kConvStages);
-          if (!mbar_wait(full0 + 8 * s, (uint32_t)((kg / kConvStages) & 1))) {
-            atomicExch(&s_abort, 1);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t base = smem_u32(sa + s * Cfg::BoxA);
+        mbar_expect_tx(full0 + 8 * s, kConvIn * rs);
+        tma_load_5d(stage0 + s * a.stage_bytes, &mbox, 0, x0 / 8, 0, y0, b, full0 + 8 * s);
+      }
+      if (conv_aborted(&s_abort))  // let copies in flight land before the CTA exits
+        for (long long q = (k > S ? k - S : 0); q < k; ++q)
+          mbar_wait(full0 + 8 * (int)(q % S), (uint32_t)((q / S) & 1));
+    }
+  } else if (warp == 1) {
+    // the whole warp runs the loop, so that descriptors and addresses stay warp-uniform values; one
+    // elected lane issues
+    long long k = 0;
+    bool ok = true;
+    for (long long t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x, ++k) {
+      const int buf = (int)(k & 1), s = (int)(k % S);
+      ok = __all_sync(0xFFFFFFFFu, (k < 2 || mbar_wait(acce0 + 8 * buf, (uint32_t)(((k >> 1) - 1) & 1))) &&
+                                       mbar_wait(full0 + 8 * s, (uint32_t)((k / S) & 1)));
+      if (!ok && lane == 0) atomicExch(&s_abort, 1);
+      if (!ok || __any_sync(0xFFFFFFFFu, conv_aborted(&s_abort))) break;
+      tc_fence_after();
+      const uint32_t d = tmem + (uint32_t)buf * kBuf, st = stage0 + s * a.stage_bytes;
+      if (elect_one()) {
 #pragma unroll
-          for (int dy = 0; dy < 3; ++dy) {
-            const uint64_t da = desc_sw64(base + dy * Cfg::RowA);
-            const uint64_t db = desc_sw64(smem_u32(sb + (dy * 3 + l) * Cfg::TapB));
-            umma_bf16(d, da, db, Cfg::Idesc, (l | dy) ? 1u : 0u);
-            umma_bf16(d, da + 2, db + 2, Cfg::Idesc, 1u);  // +32 bytes: channels 16..31
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+          for (int r = 0; r < kConvIn; ++r) {
+            // output rows j0 .. j1 take tap r - j of input row r
+            const int j0 = r < 2 ? 0 : r - 2, j1 = r < kConvRows ? r : kConvRows - 1, n = (j1 - j0 + 1) * kCo;
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
+#pragma unroll
+            for (int h = 0; h < kHalves; ++h) {
+              const uint32_t at = st + r * rs + 2 * h * cs + 16 * dx;
+              const uint32_t wt = w0 + (dx * kHalves + h) * kWBlock + (2 - (r - j0)) * kCo * 16;
+              umma_bf16(d + j0 * kCo, desc_plain(at, PLANES == 1 ? zero0 - at : cs, 128),
+                        desc_plain(wt, kWPlane, 128), idesc, 1u);
+            }
           }
-          umma_commit(empty0 + 8 * s);
-        }
-        if (!ok) break;
+        umma_commit(empty0 + 8 * s);
         umma_commit(accf0 + 8 * buf);
       }
-      umma_commit(mdone);  // every MMA issued above has finished once this arrives
-      if (!mbar_wait(mdone, 0)) atomicExch(&s_abort, 1);
+      __syncwarp();
     }
+    if (elect_one()) umma_commit(mdone);  // every MMA issued above has finished once this arrives
+    __syncwarp();
+    if (!mbar_wait(mdone, 0)) atomicExch(&s_abort, 1);
   } else {
-    // epilogue: warp w reads TMEM lanes 32 * (w % 4) ... + 31
-    const int qd = warp & 3;
-    const int m = qd * 32 + lane;
-    const int yy = m / kConvTW, px = m % kConvTW;
-    const float* bias = s_bias;
-    int it = 0;
-    for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
-      const int buf = it & 1;
-      // warp-uniform decision: the TMEM load below is .sync.aligned
-      const bool got = __all_sync(0xFFFFFFFFu, mbar_wait(accf0 + 8 * buf, (uint32_t)((it >> 1) & 1)));
-      if (!got) {
+    // epilogue: the two warps of quadrant q hold pixels 32 q .. + 31, a lane one pixel, four of the
+    // output rows each
+    constexpr int kRows = kConvRows / 2;
+    const int px = (warp & 3) * 32 + lane, j0 = warp < 6 ? 0 : kRows;
+    const uint32_t tl = (uint32_t)((warp & 3) * 32) << 16;
+    float bias[EPI == kEpiRelu ? 32 : 1];
+    if constexpr (EPI == kEpiRelu) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) bias[i] = __ldg(a.bias + i);
+    } else {
+      bias[0] = kLast ? __ldg(a.bias) : 0.f;
+    }
+    const long long rowq = (long long)a.wp * 4;  // 16-byte units of a padded row
+    long long k = 0;
+    for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
+      const int buf = (int)(k & 1);
+      int x0, y0, b;
+      conv_tile(a, t, x0, y0, b);
+      y0 += j0;
+      const int x = x0 + px, rows = min(kRows, a.H - y0);
+      const bool in = px < N && x < a.W;
+      // plane 0 of the pixel in this warp's first row, and the pixel in an unpadded volume
+      const long long at = ((long long)b * (a.H + 2) + y0 + 1) * rowq + x + 1;
+      const long long o0 = ((long long)b * a.H + y0) * a.W + x;
+      // what the epilogue reads of other arrays is loaded before the wait
+      uint4 m[EPI == kEpiMask ? 4 * kRows : 1];
+      float xc[EPI == kEpiGate ? kRows : 1];
+      if constexpr (EPI == kEpiMask) {
+#pragma unroll
+        for (int j = 0; j < kRows; ++j)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            m[4 * j + c] = in && j < rows ? __ldg(reinterpret_cast<const uint4*>(a.mask_act) + at + j * rowq +
+                                                  (long long)c * a.wp)
+                                          : make_uint4(0u, 0u, 0u, 0u);
+      }
+      if constexpr (EPI == kEpiGate) {
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) xc[j] = in && j < rows ? __ldg(a.xc + o0 + (long long)j * a.W) : 0.f;
+      }
+      // warp-uniform decision: the TMEM accesses below are .sync.aligned
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(accf0 + 8 * buf, (uint32_t)((k >> 1) & 1)))) {
         if (lane == 0) atomicExch(&s_abort, 1);
         break;
       }
       if (__any_sync(0xFFFFFFFFu, conv_aborted(&s_abort))) break;
       tc_fence_after();
-      int x0, y0, b;
-      conv_tile(a, t, x0, y0, b);
-      const int x = x0 + px, y = y0 + yy;
-      const bool in = x < a.W && y < a.H;
-      const uint32_t ta = tmem + (uint32_t)(buf * 32) + ((uint32_t)(qd * 32) << 16);
-      if constexpr (N == 32) {
-        uint32_t r[32];
-        tmem_ld32(ta, r);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acce0 + 8 * buf);
-        if (in) {
-          const long long pix = ((long long)b * a.H + y) * a.wp + x + 1;
-          uint4* dst = reinterpret_cast<uint4*>(a.out_act + pix * kCnnC);
-          if constexpr (EPI == kEpiRelu) {
+      const uint32_t ta = tmem + (uint32_t)buf * kBuf + (uint32_t)(j0 * kCo) + tl;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              float v[8];
+      for (int j = 0; j < kRows; ++j) {
+        const bool mine = in && j < rows;
+        if constexpr (!kLast) {
+          uint32_t r[32];
+          tmem_ld32(ta + j * 32, r);
+          tmem_zero16(ta + j * 32);  // the next tile accumulates from zero
+          tmem_zero16(ta + j * 32 + 16);
+          uint4* dst = reinterpret_cast<uint4*>(a.out_act) + at + j * rowq;
 #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                v[j] = fmaxf(__uint_as_float(r[8 * g + j]) + bias[8 * g + j], 0.f);
-              dst[g] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
-                                  pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-            }
-          } else {
-            const uint4* msk = reinterpret_cast<const uint4*>(a.mask_act + pix * kCnnC);
+          for (int c = 0; c < 4; ++c) {
+            float v[8];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const uint4 mv = msk[g];
-              const uint32_t mwd[4] = {mv.x, mv.y, mv.z, mv.w};
-              float v[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const int16_t bits = (int16_t)((mwd[j >> 1] >> (16 * (j & 1))) & 0xFFFFu);
-                v[j] = bits > 0 ? __uint_as_float(r[8 * g + j]) : 0.f;
+            for (int e = 0; e < 8; ++e) {
+              const float u = __uint_as_float(r[8 * c + e]);
+              if constexpr (EPI == kEpiRelu) {
+                v[e] = fmaxf(u + bias[8 * c + e], 0.f);
+              } else {
+                const uint4 q = m[4 * j + c];
+                const uint32_t w = e < 2 ? q.x : (e < 4 ? q.y : (e < 6 ? q.z : q.w));
+                v[e] = (int16_t)(e & 1 ? w >> 16 : w & 0xFFFFu) > 0 ? u : 0.f;
               }
-              dst[g] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
-                                  pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
             }
+            if (mine)
+              dst[(long long)c * a.wp] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                                    pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
           }
-        }
-      } else {
-        uint32_t r[16];
-        tmem_ld16(ta, r);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acce0 + 8 * buf);
-        const long long o = ((long long)b * a.H + y) * a.W + x;
-        const float rr = __uint_as_float(r[0]) + bias[0];
-        if constexpr (EPI == kEpiResid) {
-          if (in) a.out_f[o] = rr;
         } else {
-          bool rej = false;
-          if (in) {
-            const float plain = a.calib * a.xc[o];
-            const float dlt = rr * a.inv_scale;
-            const bool keep = fabsf(dlt) <= a.bound;  // NaN fails the test: plain is kept
-            a.out_f[o] = keep ? plain + dlt : plain;
-            rej = !keep;
+          uint32_t r[16];
+          tmem_ld16(ta + j * 16, r);
+          tmem_zero16(ta + j * 16);
+          const long long o = o0 + (long long)j * a.W;
+          const float rr = __uint_as_float(r[0]) + bias[0];
+          if constexpr (EPI == kEpiResid) {
+            if (mine) a.out_f[o] = rr;
+          } else {
+            bool rej = false;
+            if (mine) {
+              const float plain = a.calib * xc[j];
+              const float dlt = rr * a.inv_scale;
+              const bool keep = fabsf(dlt) <= a.bound;  // NaN fails the test: plain is kept
+              a.out_f[o] = keep ? plain + dlt : plain;
+              rej = !keep;
+            }
+            const unsigned msk = __ballot_sync(0xFFFFFFFFu, rej);
+            if (lane == 0 && msk && a.n_reject)
+              atomicAdd(a.n_reject, (unsigned long long)__popc(msk));
           }
-          const unsigned msk = __ballot_sync(0xFFFFFFFFu, rej);
-          if (lane == 0 && msk && a.n_reject)
-            atomicAdd(a.n_reject, (unsigned long long)__popc(msk));
         }
       }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acce0 + 8 * buf);
     }
   }
 
@@ -313,42 +334,35 @@ __global__ void __launch_bounds__(kConvThreads, 3)
   __syncthreads();
   if (threadIdx.x == 0 && conv_aborted(&s_abort) && a.status) atomicExch(a.status, kDevWaitTimeout);
   if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(Cfg::TmemCols)
-                 : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmem) : "memory");
 }
 
-// Network input: channel k of slice b = k_in * plane(b, k), k < 5; pads and channels >= 5 zero.
-// plane(b, k) = b*5 + k for stacked training inputs [B][5][H][W], or the volume slice
+// Network input: channel k of slice b = k_in * plane(b, k), k < 5 (channels 5..7 zero; the pads stay
+// zero).  plane(b, k) = b*5 + k for stacked training inputs [B][5][H][W], or the volume slice
 // clamp(z0 + b + k - 2, 0, nz - 1) for inference over a volume [nz][H][W].
-__global__ void cnn_prep_kernel(const float* __restrict__ src, int vol_mode, int z0, int nz,
-                                int B, int H, int W, int wp, float k_in,
-                                __nv_bfloat16* __restrict__ a0) {
+__global__ void __launch_bounds__(256) cnn_prep_kernel(const float* __restrict__ src, int vol_mode, int z0,
+                                                       int nz, int B, int H, int W, int wp, float k_in,
+                                                       __nv_bfloat16* __restrict__ a0) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)B * H * wp) return;
-  const int col = (int)(i % wp);
-  const long long q = i / wp;
-  const int y = (int)(q % H), b = (int)(q / H), x = col - 1;
-  float v[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  if (x >= 0 && x < W) {
+  if (i >= (long long)B * H * W) return;
+  const int x = (int)(i % W);
+  const long long q = i / W;
+  const int y = (int)(q % H), b = (int)(q / H);
+  float v[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      long long plane;
-      if (vol_mode) {
-        int z = z0 + b + k - 2;
-        z = z < 0 ? 0 : (z > nz - 1 ? nz - 1 : z);
-        plane = z;
-      } else {
-        plane = (long long)b * 5 + k;
-      }
-      v[k] = __fmul_rn(k_in, src[(plane * H + y) * W + x]);
+  for (int k = 0; k < 5; ++k) {
+    long long plane;
+    if (vol_mode) {
+      int z = z0 + b + k - 2;
+      z = z < 0 ? 0 : (z > nz - 1 ? nz - 1 : z);
+      plane = z;
+    } else {
+      plane = (long long)b * 5 + k;
     }
+    v[k] = __fmul_rn(k_in, __ldg(src + (plane * H + y) * W + x));
   }
-  uint4* dst = reinterpret_cast<uint4*>(a0 + i * kCnnC);
-  dst[0] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], 0.f), 0u);
-  dst[1] = make_uint4(0u, 0u, 0u, 0u);
-  dst[2] = make_uint4(0u, 0u, 0u, 0u);
-  dst[3] = make_uint4(0u, 0u, 0u, 0u);
+  uint4* dst = reinterpret_cast<uint4*>(a0 + (((long long)b * (H + 2) + y + 1) * wp + x + 1) * 8);
+  *dst = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], 0.f), 0u);
 }
 
 // MSE loss of (k_in x_c + r) against s t and its gradient 2 d / n -> channel 0 of the last
@@ -370,7 +384,9 @@ __global__ void __launch_bounds__(256) cnn_loss_kernel(const float* __restrict__
     const float yv = __fadd_rn(__fmul_rn(k_in, xc), r[p]);
     const float d = __fsub_rn(yv, __fmul_rn(s, tgt[p]));
     d2 = d * d;
-    dz[((b * H + y) * wp + x + 1) * kCnnC] = __float2bfloat16_rn(__fmul_rn(d, two_over_n));
+    // plane 0, channel 0; the other channels of this delta stay zero
+    *reinterpret_cast<uint4*>(dz + ((b * (H + 2) + y + 1) * 4 * wp + x + 1) * 8) =
+        make_uint4(pack_bf16x2(__fmul_rn(d, two_over_n), 0.f), 0u, 0u, 0u);
   }
   for (int o = 16; o; o >>= 1) d2 += __shfl_xor_sync(0xFFFFFFFFu, d2, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = d2;
@@ -382,105 +398,150 @@ __global__ void __launch_bounds__(256) cnn_loss_kernel(const float* __restrict__
   }
 }
 
-// Weight gradients of one layer on tcgen05, no transposes: with K = pixels, both channels-last
-// operands are MN-major (32 channels = one 64-byte swizzle row per pixel, 8 pixels = one atom).
-//   D_dx[dy * 32 + ci][co] += sum_p act[p + (dy - 1, dx - 1)][ci] * dz[p][co]
-// Per 8 px x 16 rows tile: one activation box {32 ch, 8 px, 19 rows} per dx whose rows r and
-// r + 1 .. are the dy blocks (M = 128: the three dy blocks at +512 B and one discarded block),
-// and one delta box {32 ch, 8 px, 16 rows} (N = 32); K = 128 pixels = 8 MMAs of K16 per dx.
-// A CTA accumulates over all its tiles in three TMEM accumulators and adds them to the gradient
-// once.  Pads and rows outside the image are zero in the deltas, so they add nothing.
-constexpr int kDwStages = 3, kDwThreads = 128, kDwRows = kConvTH + 3;
-struct DwCfg {
-  static constexpr uint32_t BoxA = kConvTW * kDwRows * kCnnC * 2;  // 9728 B
-  static constexpr uint32_t BoxD = kConvTW * kConvTH * kCnnC * 2;  // 8192 B
-  static constexpr uint32_t Stage = 3 * BoxA + BoxD;               // 37376 B, 512-aligned
-  static constexpr uint32_t Smem = 1024 + kDwStages * Stage + 128;
-  static constexpr uint32_t TmemCols = 128;                         // 3 x 32 used
-  static constexpr uint32_t Idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                                    ((uint32_t)(32 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-};
+// Weight and bias gradients of one layer, no transposes: with K = pixels, both operands are MN-major
+// core matrices of the layout (8 pixels x 8 channels, 128 contiguous bytes).  For a group of three delta
+// rows j and the five activation rows o around them,
+//   D_dx[32 j + co][32 o + ci] += sum_p dz[row j, p][co] * act[row o, p + dx - 1][ci]
+// is one M128 x N160 x K16 MMA per dx and 16 pixels: M the planes of consecutive delta rows (the fourth
+// row is discarded), N those of the activation rows, shifted by the start of the operand.  The blocks
+// with o - j = dy in 0..2 are the gradient's; nine of fifteen useful, but loading an M128 operand costs
+// about 64 clocks and a column 0.4, so few wide MMAs beat nine exact ones.  The network input has one
+// plane: 32 o becomes 8 o and N 48.
+// A tile is 6 rows x up to 64 pixels: one box of eight activation rows and one of six delta rows
+// (whatever lies outside the image reads as zero).  A CTA accumulates over all its tiles in three TMEM
+// accumulators, sums the blocks over j in shared memory and adds them to the gradient once.  Four
+// further warps sum the staged deltas per channel: the bias gradient.
+// Bound: the MMAs' operand loads.  16 x 256^2: 42-49 us per layer; with one tap's activations as M128 and
+// N32, and a separate pass for the biases, 57-87 + 24 us.
+constexpr int kDwThreads = 192, kDwSums = kDwThreads / 32 - 2, kDwGroups = 2, kDwRows = 3 * kDwGroups, kDwMaxP = 64, kDwMaxStages = 4;
 
-__global__ void __launch_bounds__(kDwThreads)
-    cnn_dw_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mz,
-                     const ConvArgs a, int cin, int cout, float* __restrict__ gw) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kDwStages * DwCfg::Stage);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kDwStages + 1);
+template <int PLANES>  // planes of the activation: 1 (network input) or 4
+__global__ void __launch_bounds__(kDwThreads, 1)
+    cnn_dw_tc_kernel(const __grid_constant__ CUtensorMap mact, const __grid_constant__ CUtensorMap mdz,
+                     const ConvArgs a, int cin, int cout, float* __restrict__ gw, float* __restrict__ gb) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ __align__(8) uint64_t bars[2 * kDwMaxStages + 1];
+  __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t full0 = smem_u32(&bars[0]);
-  const uint32_t empty0 = smem_u32(&bars[kDwStages]);
-  const uint32_t mdone = smem_u32(&bars[2 * kDwStages]);
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int P = a.n_px, S = a.stages;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kDwMaxStages]);
+  const uint32_t mdone = smem_u32(&bars[2 * kDwMaxStages]);
+  const uint32_t stage0 = smem_u32(smem);
+  const uint32_t cs = dw_plane(P), rs = PLANES * cs;  // activation plane, row
+  const uint32_t zs = (uint32_t)P * 16, zoff = ((kDwRows + 2) * rs + 127) / 128 * 128;  // delta plane, offset
+  constexpr int kCi = PLANES * 8, kN = PLANES == 1 ? 48 : 160;  // columns of an activation row, of D_dx
+  constexpr uint32_t kCols = PLANES == 1 ? 256 : 512;
+  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                              ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int s = 0; s < kDwStages; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1 + kDwSums);  // the MMAs and the summing warps
     }
     mbar_init(mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "r"(DwCfg::TmemCols)
+                     smem_u32(&tmem_slot)),
+                 "r"(kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_slot, 0);
 
-  if (warp == 0 && lane == 0) {
-    long long it = 0;
-    for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
-      const int s = (int)(it % kDwStages);
-      if (it >= kDwStages &&
-          !mbar_wait(empty0 + 8 * s, (uint32_t)(((it / kDwStages) - 1) & 1))) {
-        atomicExch(&s_abort, 1);
-        break;
+  if (warp == 0) {
+    if (lane == 0) {
+      long long k = 0;
+      for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
+        const int s = (int)(k % S);
+        if (k >= S && !mbar_wait(empty0 + 8 * s, (uint32_t)(((k / S) - 1) & 1))) {
+          atomicExch(&s_abort, 1);
+          break;
+        }
+        if (conv_aborted(&s_abort)) break;
+        int x0, y0, b;
+        conv_tile(a, t, x0, y0, b);
+        const uint32_t fb = full0 + 8 * s, st = stage0 + s * a.stage_bytes;
+        mbar_expect_tx(fb, (kDwRows + 2) * rs + kDwRows * 4 * zs);
+        tma_load_4d(st, &mact, 2 * x0, 0, y0, b, fb);
+        tma_load_4d(st + zoff, &mdz, 2 * x0, 0, y0, b, fb);
       }
-      if (conv_aborted(&s_abort)) break;
-      int x0, y0, b;
-      conv_tile(a, t, x0, y0, b);
-      uint8_t* st = smem + s * DwCfg::Stage;
-      const uint32_t fb = full0 + 8 * s;
-      mbar_expect_tx(fb, DwCfg::Stage);
-      for (int dx = 0; dx < 3; ++dx)  // pixel x, column offset dx - 1: padded column x + dx
-        tma_load_4d(smem_u32(st + dx * DwCfg::BoxA), &ma, 0, x0 + dx, y0 - 1, b, fb);
-      tma_load_4d(smem_u32(st + 3 * DwCfg::BoxA), &mz, 0, x0 + 1, y0, b, fb);
+      if (conv_aborted(&s_abort))  // let copies in flight land before the CTA exits
+        for (long long q = (k > S ? k - S : 0); q < k; ++q)
+          mbar_wait(full0 + 8 * (int)(q % S), (uint32_t)((q / S) & 1));
     }
-    if (conv_aborted(&s_abort))  // let copies in flight land before the CTA exits
-      for (long long k = (it > kDwStages ? it - kDwStages : 0); k < it; ++k)
-        mbar_wait(full0 + 8 * (int)(k % kDwStages), (uint32_t)((k / kDwStages) & 1));
-  } else if (warp == 1 && lane == 0) {
-    long long it = 0;
-    bool first = true;
-    for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
-      const int s = (int)(it % kDwStages);
-      if (!mbar_wait(full0 + 8 * s, (uint32_t)((it / kDwStages) & 1))) {
-        atomicExch(&s_abort, 1);
+  } else if (warp == 1) {
+    long long k = 0;
+    uint32_t more = 0;  // 0 for the first MMA of each accumulator
+    for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
+      const int s = (int)(k % S);
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(full0 + 8 * s, (uint32_t)((k / S) & 1)))) {
+        if (lane == 0) atomicExch(&s_abort, 1);
         break;
       }
       tc_fence_after();
-      const uint32_t st = smem_u32(smem + s * DwCfg::Stage);
+      int x0, y0, b;
+      conv_tile(a, t, x0, y0, b);
+      const int groups = (min(P, a.W - x0) + 15) / 16;
+      const uint32_t st = stage0 + s * a.stage_bytes;
+      if (elect_one()) {
 #pragma unroll
-      for (int dx = 0; dx < 3; ++dx) {
+        for (int q = 0; q < kDwGroups; ++q) {
+          uint64_t za = desc_plain(st + zoff + 12 * q * zs, 128, zs), ab = desc_plain(st + 3 * q * rs, 128, cs);
+          for (int g = 0; g < groups; ++g, za += 16, ab += 16) {
 #pragma unroll
-        for (int k = 0; k < kConvTH / 2; ++k) {  // K16 = two 8-pixel atoms = 1024 B
-          const uint64_t da = desc_mn_sw64(st + dx * DwCfg::BoxA + k * 1024, 512, 512);
-          const uint64_t dz = desc_mn_sw64(st + 3 * DwCfg::BoxA + k * 1024, 512, 512);
-          umma_bf16(tmem + dx * 32, da, dz, DwCfg::Idesc, (first && k == 0) ? 0u : 1u);
+            for (int dx = 0; dx < 3; ++dx) umma_bf16(tmem + dx * kN, za, ab + (uint64_t)dx, kIdesc, more);
+            more = 1;
+          }
+        }
+        umma_commit(empty0 + 8 * s);
+      }
+      __syncwarp();
+    }
+    if (elect_one()) umma_commit(mdone);
+  } else if (warp >= 2) {
+    // bias gradient: lane = (plane, pixel mod 8), every fourth delta row
+    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    long long k = 0;
+    for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
+      const int s = (int)(k % S);
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(full0 + 8 * s, (uint32_t)((k / S) & 1)))) {
+        if (lane == 0) atomicExch(&s_abort, 1);
+        break;
+      }
+      int x0, y0, b;
+      conv_tile(a, t, x0, y0, b);
+      const int px = min(P, a.W - x0), zrows = min(kDwRows, a.H - y0);
+      for (int r = warp - 2; r < zrows; r += kDwSums) {
+        const uint8_t* p = smem + (size_t)s * a.stage_bytes + zoff + (uint32_t)(4 * r + (lane & 3)) * zs;
+#pragma unroll 4
+        for (int i = lane >> 2; i < px; i += 8) {
+          const uint4 q = *reinterpret_cast<const uint4*>(p + i * 16);
+          const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            sum[2 * e] += __uint_as_float(w[e] << 16);
+            sum[2 * e + 1] += __uint_as_float(w[e] & 0xFFFF0000u);
+          }
         }
       }
-      first = false;
-      umma_commit(empty0 + 8 * s);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty0 + 8 * s);
     }
-    umma_commit(mdone);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 4);
+      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 8);
+      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 16);
+      const int co = 8 * lane + e;
+      if (lane < 4 && co < cout && !conv_aborted(&s_abort)) atomicAdd(&gb[co], sum[e]);
+    }
   }
   __syncwarp();
   const bool done = __all_sync(0xFFFFFFFFu, mbar_wait(mdone, 0));
@@ -488,44 +549,37 @@ __global__ void __launch_bounds__(kDwThreads)
   tc_fence_after();
   if (!done || conv_aborted(&s_abort)) {
     if (threadIdx.x == 0 && a.status) atomicExch(a.status, kDevWaitTimeout);
-  } else if (blockIdx.x < a.n_tiles) {
-    // warp w holds rows 32 w ..: dy = w (w = 3 is the discarded block), ci = lane
-    const int dy = warp, ci = lane;
+  } else {
+    // warp j < 3 holds delta row j, lane = co: block (o, dx) is tap dy = o - j; the stages are free now
+    float* part = reinterpret_cast<float*>(smem);  // [dy][dx][ci][co]
+    for (int j = 0; j < 3; ++j) {
+      if (warp == j) {
 #pragma unroll
-    for (int dx = 0; dx < 3; ++dx) {
-      uint32_t r[32];
-      tmem_ld32(tmem + dx * 32 + ((uint32_t)(warp * 32) << 16), r);
-      if (dy < 3 && ci < cin) {
+        for (int tap = 0; tap < 9; ++tap) {
+          uint32_t r[PLANES == 1 ? 16 : 32];
+          const uint32_t at = tmem + (uint32_t)((tap % 3) * kN + (j + tap / 3) * kCi) + ((uint32_t)(j * 32) << 16);
+          if constexpr (PLANES == 1)
+            tmem_ld16(at, r);
+          else
+            tmem_ld32(at, r);
+          float* p = part + tap * kCi * 32 + lane;
 #pragma unroll
-        for (int co = 0; co < 32; ++co)
-          if (co < cout) atomicAdd(&gw[((co * cin + ci) * 3 + dy) * 3 + dx], __uint_as_float(r[co]));
+          for (int ci = 0; ci < kCi; ++ci) p[ci * 32] = (j ? p[ci * 32] : 0.f) + __uint_as_float(r[ci]);
+        }
       }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < cout * cin * 9; i += kDwThreads) {
+      const int tap = i % 9, ci = i / 9 % cin, co = i / (9 * cin);
+      atomicAdd(&gw[i], part[(tap * kCi + ci) * 32 + co]);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(DwCfg::TmemCols)
+                 "r"(kCols)
                  : "memory");
-}
-
-// Bias gradients: sum of the deltas over the slices' padded pixels (pads are zero).
-__global__ void __launch_bounds__(256) cnn_db_kernel(const __nv_bfloat16* __restrict__ dz,
-                                                     long long n_pix, int cout,
-                                                     float* __restrict__ gb) {
-  __shared__ float red[8][kCnnC];
-  const int c = threadIdx.x & 31, g = threadIdx.x >> 5;
-  float acc = 0.f;
-  for (long long p = (long long)blockIdx.x * 8 + g; p < n_pix; p += (long long)gridDim.x * 8)
-    acc += __bfloat162float(dz[p * kCnnC + c]);
-  red[g][c] = acc;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float v = 0.f;
-    for (int k = 0; k < 8; ++k) v += red[k][threadIdx.x];
-    if (threadIdx.x < cout) atomicAdd(&gb[threadIdx.x], v);
-  }
 }
 
 __global__ void cnn_adam_kernel(float* __restrict__ p, const float* __restrict__ g,
@@ -564,22 +618,26 @@ using namespace lct;
 
 struct lct_cnn {
   int device = 0, cap = 0, H = 0, W = 0, wp = 0, sms = 148;
+  int n_px = 16, dw_px = 16;       // tile widths of the convolutions and of the weight gradients
   bool train = false;
-  int n_act = 0;
-  long long act_elems = 0;
+  int n_act = 0;                   // activations: outputs of layers 0..6 (training), or 2
+  long long act_elems = 0;         // of one activation / delta; the network input has a quarter
   float* d_p = nullptr;  // params, grads, Adam m, Adam v: 4 x kCnnParams
   float* d_g = nullptr;
   float* d_m = nullptr;
   float* d_v = nullptr;
   __nv_bfloat16* d_wf = nullptr;  // 8 forward slots
   __nv_bfloat16* d_wb = nullptr;  // 8 backward slots (slot 0 unused)
+  // boxes of the convolutions' inputs and of the weight gradients; activations: [0] the network input,
+  // [1 + i] buffer i
+  CUtensorMap m_in[kCnnLayers], m_dwa[kCnnLayers];
+  CUtensorMap m_zin[3], m_dwz[3];  // the same for the deltas
+  __nv_bfloat16* d_in = nullptr;  // network input
   __nv_bfloat16* d_act = nullptr; // n_act activation buffers
   __nv_bfloat16* d_dz = nullptr;  // training: 3 delta buffers
   float* d_r = nullptr;           // training: residual [cap][H][W]
   double* d_loss = nullptr;
   unsigned long long* d_rej = nullptr;
-  CUtensorMap m_act[kCnnLayers], m_dz[3], m_wf[kCnnLayers], m_wb[kCnnLayers];
-  CUtensorMap m_dwa[kCnnLayers], m_dwz[3];  // weight-gradient boxes
   float calib = 1.f, in_scale = 1.f;
   int adam_t = 0;
   long long last_n = 0;
@@ -589,96 +647,86 @@ namespace lct {
 
 static __nv_bfloat16* act_buf(lct_cnn* c, int i) { return c->d_act + (size_t)i * c->act_elems; }
 static __nv_bfloat16* dz_buf(lct_cnn* c, int i) { return c->d_dz + (size_t)i * c->act_elems; }
-// input buffer of layer l (training keeps every activation; inference ping-pongs two)
-static int act_in(const lct_cnn* c, int l) { return c->train ? l : (l & 1); }
+// buffer of layer l's output (training keeps every activation; inference ping-pongs two), and map index
+// of layer l's input
+static int out_buf(const lct_cnn* c, int l) { return c->train ? l : (l & 1); }
+static int in_map(const lct_cnn* c, int l) { return l == 0 ? 0 : 1 + out_buf(c, l - 1); }
 
-// channels-last bf16 [cap][H][wp][32], box {32 ch, 8 px, rows, 1 slice}, 64-byte swizzle
-static int act_map(CUtensorMap* m, const void* base, int cap, int H, int wp, int rows) {
+// Boxes of the convolutions: bf16 [cap][H + 2][planes][wp / 8][8 pixels] as 8-byte elements, box
+// {8 pixels, px / 8 + 1 blocks, planes, rows, 1}.
+static int conv_map(CUtensorMap* m, __nv_bfloat16* base, const lct_cnn* c, int planes) {
   auto fn = tensor_map_encoder();
   if (!fn) return LCT_ERR_UNSUPPORTED;
-  cuuint64_t dims[4] = {(cuuint64_t)kCnnC, (cuuint64_t)wp, (cuuint64_t)H, (cuuint64_t)cap};
-  cuuint64_t strides[3] = {(cuuint64_t)kCnnC * 2, (cuuint64_t)wp * kCnnC * 2,
-                           (cuuint64_t)H * wp * kCnnC * 2};
-  cuuint32_t box[4] = {(cuuint32_t)kCnnC, (cuuint32_t)kConvTW, (cuuint32_t)rows, 1};
+  const size_t plane = (size_t)16 * c->wp, row = plane * planes, slice = row * (c->H + 2);
+  cuuint64_t dims[5] = {16, (cuuint64_t)c->wp / 8, (cuuint64_t)planes, (cuuint64_t)(c->H + 2), (cuuint64_t)c->cap};
+  cuuint64_t strides[4] = {128, plane, row, slice};
+  cuuint32_t box[5] = {16, (cuuint32_t)(c->n_px / 8 + 1), (cuuint32_t)planes, (cuuint32_t)kConvIn, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, base, dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? LCT_OK : LCT_ERR_UNSUPPORTED;
+}
+
+// Boxes of the gradients: bf16 [cap][H + 2][planes][wp][8] as 8-byte elements, box {px, planes, rows, 1}.  inner: only the
+// image's pixels, from row 0 and column 0 of the image (stores outside are dropped); else with the pads.
+static int act_map(CUtensorMap* m, __nv_bfloat16* base, const lct_cnn* c, int planes, int px, int rows,
+                   bool inner) {
+  auto fn = tensor_map_encoder();
+  if (!fn) return LCT_ERR_UNSUPPORTED;
+  const size_t col = 16, plane = col * c->wp, row = plane * planes, slice = row * (c->H + 2);
+  cuuint64_t dims[4] = {(cuuint64_t)(inner ? c->W : c->wp) * 2, (cuuint64_t)planes,
+                        (cuuint64_t)(inner ? c->H : c->H + 2), (cuuint64_t)c->cap};
+  cuuint64_t strides[3] = {plane, row, slice};
+  cuuint32_t box[4] = {(cuuint32_t)(px * 2), (cuuint32_t)planes, (cuuint32_t)rows, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  uint8_t* p = reinterpret_cast<uint8_t*>(base) + (inner ? row + col : 0);
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, p, dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? LCT_OK : LCT_ERR_UNSUPPORTED;
 }
 
-static int weight_map(CUtensorMap* m, const void* base, int rows) {
-  auto fn = tensor_map_encoder();
-  if (!fn) return LCT_ERR_UNSUPPORTED;
-  cuuint64_t dims[2] = {(cuuint64_t)kCnnK, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)kCnnK * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kCnnC, (cuuint32_t)rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? LCT_OK : LCT_ERR_UNSUPPORTED;
-}
-
-// per device: dynamic shared memory set, and resident CTAs per SM of each variant
-static bool conv_attr_done[64];
-static int conv_occ[64][2];
-static int dw_occ[64];
-
-template <typename K>
-static int tc_attr(K kernel, int smem_bytes, int threads, int* occ) {
-  int st = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            smem_bytes));
-  // all of the unified L1 as shared memory, so that several CTAs fit on an SM
-  if (!st)
-    st = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                          cudaSharedmemCarveoutMaxShared));
-  // resident CTAs per SM from the kernel's own resources (shared memory, registers, threads);
-  // the runtime's occupancy query answers 1 for this kernel although three fit.  CTAs never
-  // wait on one another, so a grid larger than what is resident only queues.
-  cudaFuncAttributes fa;
-  int dev = 0;
-  cudaDeviceProp pr;
-  if (!st) st = cuda_status(cudaFuncGetAttributes(&fa, kernel));
-  if (!st) st = cuda_status(cudaGetDevice(&dev));
-  if (!st) st = cuda_status(cudaGetDeviceProperties(&pr, dev));
-  if (st) return st;
-  const size_t smem = smem_bytes + fa.sharedSizeBytes + pr.reservedSharedMemPerBlock;
-  const int by_smem = (int)(pr.sharedMemPerMultiprocessor / smem);
-  const int regs_warp = ((fa.numRegs * 32 + 255) / 256) * 256;
-  const int by_regs = pr.regsPerMultiprocessor / (regs_warp * (threads / 32));
-  const int by_threads = pr.maxThreadsPerMultiProcessor / threads;
-  int o = by_smem < by_regs ? by_smem : by_regs;
-  o = o < by_threads ? o : by_threads;
-  *occ = o;
-  return o < 1 ? LCT_ERR_UNSUPPORTED : LCT_OK;
+// Tile width for an image of W pixels: as few tiles of at most `most` pixels as it takes, alike in width,
+// a multiple of `step`
+static int tile_px(int W, int most, int step) {
+  const int tiles = (W + most - 1) / most;
+  return ((W + tiles - 1) / tiles + step - 1) / step * step;
 }
 
 static int conv_prepare(int dev) {
-  if (dev < 0 || dev >= 64) return LCT_ERR_UNSUPPORTED;
   static std::mutex mu;  // host threads may create workspaces on one device together
+  static bool done[64] = {false};
+  if (dev < 0 || dev >= 64) return LCT_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lock(mu);
-  if (conv_attr_done[dev]) return LCT_OK;
-  int st, o[4];
-  if ((st = tc_attr(conv_tc_kernel<32, kEpiRelu>, ConvCfg<32>::Smem, kConvThreads, &o[0]))) return st;
-  if ((st = tc_attr(conv_tc_kernel<32, kEpiMask>, ConvCfg<32>::Smem, kConvThreads, &o[1]))) return st;
-  if ((st = tc_attr(conv_tc_kernel<16, kEpiResid>, ConvCfg<16>::Smem, kConvThreads, &o[2]))) return st;
-  if ((st = tc_attr(conv_tc_kernel<16, kEpiGate>, ConvCfg<16>::Smem, kConvThreads, &o[3]))) return st;
-  if ((st = tc_attr(cnn_dw_tc_kernel, DwCfg::Smem, kDwThreads, &dw_occ[dev]))) return st;
-  conv_occ[dev][0] = o[0] < o[1] ? o[0] : o[1];
-  conv_occ[dev][1] = o[2] < o[3] ? o[2] : o[3];
-  conv_attr_done[dev] = true;
+  if (done[dev]) return LCT_OK;
+  auto attr = [](auto kernel) {
+    return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+  };
+  int st;
+  if ((st = attr(conv_tc_kernel<kEpiRelu, 1>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiRelu, 4>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiMask, 4>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiResid, 4>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiGate, 4>))) return st;
+  if ((st = attr(cnn_dw_tc_kernel<1>))) return st;
+  if ((st = attr(cnn_dw_tc_kernel<4>))) return st;
+  done[dev] = true;
   return LCT_OK;
 }
 
-template <int N, int EPI>
-static int launch_conv(const CUtensorMap& mx, const CUtensorMap& mw, ConvArgs a, int B, int dev,
-                       int sms, cudaStream_t s) {
+template <int EPI, int PLANES>
+static int launch_conv(const CUtensorMap& in, ConvArgs a, int B, int sms, cudaStream_t s) {
   a.n_tiles = (long long)B * a.tiles_x * a.tiles_y;
   if (a.n_tiles <= 0) return LCT_OK;
-  const long long resident = (long long)sms * conv_occ[dev][N == 32 ? 0 : 1];
-  const unsigned grid = (unsigned)(a.n_tiles < resident ? a.n_tiles : resident);
-  conv_tc_kernel<N, EPI><<<grid, kConvThreads, ConvCfg<N>::Smem, s>>>(mx, mw, a);
+  a.stage_bytes = (kConvIn * PLANES * conv_plane(a.n_px) + 127) / 128 * 128;
+  const bool last = EPI == kEpiResid || EPI == kEpiGate;
+  const uint32_t fixed = (PLANES == 1 ? kConvZero : 0u) + 3u * (PLANES == 1 ? 1u : 2u) * 2u * 3u * (last ? 16u : 32u) * 16u;
+  const uint32_t tail = 128 * 16;  // an operand of the last plane may read this far past it
+  a.stages = std::min<int>(kConvMaxStages, (int)((kSmemMax - fixed - tail) / a.stage_bytes));
+  const size_t smem = (size_t)a.stages * a.stage_bytes + fixed + tail;
+  const unsigned grid = (unsigned)std::min<long long>(a.n_tiles, sms);  // tensor memory: one CTA per SM
+  conv_tc_kernel<EPI, PLANES><<<grid, kConvThreads, smem, s>>>(in, a);
   return launch_status();
 }
 
@@ -687,8 +735,10 @@ static ConvArgs conv_args(const lct_cnn* c) {
   a.H = c->H;
   a.W = c->W;
   a.wp = c->wp;
-  a.tiles_x = (c->W + kConvTW - 1) / kConvTW;
-  a.tiles_y = (c->H + kConvTH - 1) / kConvTH;
+  a.n_px = c->n_px;
+  a.rows = kConvRows;
+  a.tiles_x = (c->W + a.n_px - 1) / a.n_px;
+  a.tiles_y = (c->H + kConvRows - 1) / kConvRows;
   a.status = device_status_ptr();
   return a;
 }
@@ -700,23 +750,24 @@ static int run_pack(lct_cnn* c, cudaStream_t s) {
 
 static int run_prep(lct_cnn* c, const float* src, int vol_mode, int z0, int nz, int B,
                     cudaStream_t s) {
-  const long long n = (long long)B * c->H * c->wp;
+  const long long n = (long long)B * c->H * c->W;
   const float k_in = c->calib * c->in_scale;
   cnn_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, vol_mode, z0, nz, B, c->H,
-                                                             c->W, c->wp, k_in, act_buf(c, 0));
+                                                             c->W, c->wp, k_in, c->d_in);
   return launch_status();
 }
 
-// hidden layers 0..6 of the forward pass on B slices already in act_buf(0)
+// hidden layers 0..6 of the forward pass on B slices already in d_in
 static int run_hidden(lct_cnn* c, int B, cudaStream_t s) {
   ConvArgs a = conv_args(c);
   int st;
   for (int l = 0; l < kCnnLayers - 1; ++l) {
     a.bias = c->d_p + cnn_off(l) + cnn_cin(l) * cnn_cout(l) * 9;
-    a.out_act = act_buf(c, c->train ? l + 1 : ((l + 1) & 1));
-    if ((st = launch_conv<32, kEpiRelu>(c->m_act[act_in(c, l)], c->m_wf[l], a, B, c->device,
-                                        c->sms, s)))
-      return st;
+    a.w = c->d_wf + (size_t)l * kWSlot;
+    a.out_act = act_buf(c, out_buf(c, l));
+    const CUtensorMap& in = c->m_in[in_map(c, l)];
+    st = l == 0 ? launch_conv<kEpiRelu, 1>(in, a, B, c->sms, s) : launch_conv<kEpiRelu, 4>(in, a, B, c->sms, s);
+    if (st) return st;
   }
   return LCT_OK;
 }
@@ -725,6 +776,7 @@ static int last_bias_and_args(lct_cnn* c, ConvArgs& a) {
   a = conv_args(c);
   const int l = kCnnLayers - 1;
   a.bias = c->d_p + cnn_off(l) + cnn_cin(l) * cnn_cout(l) * 9;
+  a.w = c->d_wf + (size_t)l * kWSlot;
   return LCT_OK;
 }
 
@@ -735,8 +787,8 @@ static int cnn_forward_impl(lct_cnn* c, const float* d_in5, int B, cudaStream_t 
   ConvArgs a;
   last_bias_and_args(c, a);
   a.out_f = c->d_r;
-  return launch_conv<16, kEpiResid>(c->m_act[act_in(c, kCnnLayers - 1)], c->m_wf[kCnnLayers - 1],
-                                    a, B, c->device, c->sms, s);
+  const CUtensorMap& in = c->m_in[in_map(c, kCnnLayers - 1)];
+  return launch_conv<kEpiResid, 4>(in, a, B, c->sms, s);
 }
 
 static int cnn_backward_impl(lct_cnn* c, const float* d_in5, const float* d_target, int B,
@@ -752,26 +804,33 @@ static int cnn_backward_impl(lct_cnn* c, const float* d_in5, const float* d_targ
   c->last_n = n;
   ConvArgs a = conv_args(c);
   ConvArgs da = conv_args(c);
+  da.n_px = c->dw_px;
+  da.rows = kDwRows;
+  da.tiles_x = (c->W + da.n_px - 1) / da.n_px;
+  da.tiles_y = (c->H + kDwRows - 1) / kDwRows;
   da.n_tiles = (long long)B * da.tiles_x * da.tiles_y;
-  const long long dw_res = (long long)c->sms * dw_occ[c->device];
-  const unsigned dw_grid = (unsigned)(da.n_tiles < dw_res ? da.n_tiles : dw_res);
-  const long long n_pix = (long long)B * c->H * c->wp;
-  const unsigned db_grid = (unsigned)std::min<long long>((n_pix + 7) / 8, (long long)c->sms * 8);
+  const unsigned dw_grid = (unsigned)std::min<long long>(da.n_tiles, c->sms);
   int cur = 2;
   for (int l = kCnnLayers - 1; l >= 0; --l) {
     float* gw = c->d_g + cnn_off(l);
     float* gb = gw + cnn_cin(l) * cnn_cout(l) * 9;
-    cnn_dw_tc_kernel<<<dw_grid, kDwThreads, DwCfg::Smem, s>>>(c->m_dwa[l], c->m_dwz[cur], da,
-                                                                cnn_cin(l), cnn_cout(l), gw);
-    if ((st = launch_status())) return st;
-    cnn_db_kernel<<<db_grid, 256, 0, s>>>(dz_buf(c, cur), n_pix, cnn_cout(l), gb);
+    const int planes = l == 0 ? 1 : 4;
+    da.stage_bytes = ((kDwRows + 2) * planes * dw_plane(da.n_px) + 127) / 128 * 128 +
+                     kDwRows * 4 * (uint32_t)da.n_px * 16;
+    // the last group's discarded delta row, and the network input's sixth activation row, read past it
+    const uint32_t tail = 4 * (uint32_t)da.n_px * 16 + 2 * dw_plane(da.n_px);
+    da.stages = std::min<int>(kDwMaxStages, (int)((kSmemMax - tail) / da.stage_bytes));
+    const size_t dw_smem = std::max((size_t)da.stages * da.stage_bytes + tail, sizeof(float) * 9 * kCnnC * kCnnC);
+    auto dw = l == 0 ? cnn_dw_tc_kernel<1> : cnn_dw_tc_kernel<4>;
+    dw<<<dw_grid, kDwThreads, dw_smem, s>>>(c->m_dwa[in_map(c, l)], c->m_dwz[cur], da, cnn_cin(l), cnn_cout(l),
+                                            gw, gb);
     if ((st = launch_status())) return st;
     if (l == 0) break;
     const int nxt = cur == 2 ? 0 : (cur ^ 1);
+    a.w = c->d_wb + (size_t)l * kWSlot;
     a.out_act = dz_buf(c, nxt);
-    a.mask_act = act_buf(c, l);
-    if ((st = launch_conv<32, kEpiMask>(c->m_dz[cur], c->m_wb[l], a, B, c->device, c->sms, s)))
-      return st;
+    a.mask_act = act_buf(c, out_buf(c, l - 1));
+    if ((st = launch_conv<kEpiMask, 4>(c->m_zin[cur], a, B, c->sms, s))) return st;
     cur = nxt;
   }
   return LCT_OK;
@@ -814,6 +873,7 @@ static void free_cnn(lct_cnn* c) {
   if (!c) return;
   cudaFree(c->d_p);
   cudaFree(c->d_wf);
+  cudaFree(c->d_in);
   cudaFree(c->d_act);
   cudaFree(c->d_dz);
   cudaFree(c->d_r);
@@ -835,7 +895,7 @@ LCT_API int lct_cnn_create(int max_slices, int ny, int nx, int flags, uint64_t s
   if (!out || max_slices <= 0 || ny <= 0 || nx <= 0) return LCT_ERR_ARG;
   *out = nullptr;
   if ((flags & ~LCT_CNN_TRAIN) != 0) return LCT_ERR_ARG;
-  const long long wp = (long long)nx + 2;
+  const long long wp = ((long long)nx + 2 + 7) / 8 * 8;
   if (wp > (1LL << 30) || ny > (1 << 30)) return LCT_ERR_ARG;
   lct_cnn* c = new (std::nothrow) lct_cnn;
   if (!c) return LCT_ERR_ALLOC;
@@ -844,8 +904,10 @@ LCT_API int lct_cnn_create(int max_slices, int ny, int nx, int flags, uint64_t s
   c->W = nx;
   c->wp = (int)wp;
   c->train = (flags & LCT_CNN_TRAIN) != 0;
-  c->n_act = c->train ? kCnnLayers : 2;
-  c->act_elems = (long long)max_slices * ny * wp * kCnnC;
+  c->n_px = tile_px(nx, kConvMaxN, 8);
+  c->dw_px = tile_px(nx, kDwMaxP, 16);
+  c->n_act = c->train ? kCnnLayers - 1 : 2;
+  c->act_elems = (long long)max_slices * (ny + 2) * wp * kCnnC;
   int st = cuda_status(cudaGetDevice(&c->device));
   if (!st) st = cuda_status(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device));
   if (!st) st = conv_prepare(c->device);
@@ -859,6 +921,8 @@ LCT_API int lct_cnn_create(int max_slices, int ny, int nx, int flags, uint64_t s
   if (!st) st = cuda_status(cudaMalloc(&c->d_wf, sizeof(__nv_bfloat16) * 2 * kCnnLayers * kWSlot));
   if (!st) c->d_wb = c->d_wf + kCnnLayers * kWSlot;
   const size_t act_bytes = sizeof(__nv_bfloat16) * (size_t)c->act_elems;
+  if (!st) st = cuda_status(cudaMalloc(&c->d_in, act_bytes / 4));
+  if (!st) st = cuda_status(cudaMemset(c->d_in, 0, act_bytes / 4));
   if (!st) st = cuda_status(cudaMalloc(&c->d_act, act_bytes * c->n_act));
   if (!st) st = cuda_status(cudaMemset(c->d_act, 0, act_bytes * c->n_act));
   if (!st && c->train) {
@@ -868,17 +932,15 @@ LCT_API int lct_cnn_create(int max_slices, int ny, int nx, int flags, uint64_t s
   }
   if (!st) st = cuda_status(cudaMalloc(&c->d_loss, sizeof(double)));
   if (!st) st = cuda_status(cudaMalloc(&c->d_rej, sizeof(unsigned long long)));
-  for (int i = 0; i < c->n_act && !st; ++i)
-    st = act_map(&c->m_act[i], act_buf(c, i), c->cap, c->H, c->wp, kConvTH + 2);
-  for (int i = 0; i < 3 && !st && c->train; ++i)
-    st = act_map(&c->m_dz[i], dz_buf(c, i), c->cap, c->H, c->wp, kConvTH + 2);
-  for (int i = 0; i < c->n_act && !st && c->train; ++i)  // weight gradients: 19-row boxes
-    st = act_map(&c->m_dwa[i], act_buf(c, i), c->cap, c->H, c->wp, kDwRows);
-  for (int i = 0; i < 3 && !st && c->train; ++i)
-    st = act_map(&c->m_dwz[i], dz_buf(c, i), c->cap, c->H, c->wp, kConvTH);
-  for (int l = 0; l < kCnnLayers && !st; ++l) {
-    st = weight_map(&c->m_wf[l], c->d_wf + (size_t)l * kWSlot, l == kCnnLayers - 1 ? 16 : 32);
-    if (!st) st = weight_map(&c->m_wb[l], c->d_wb + (size_t)l * kWSlot, 32);
+  for (int i = 0; i <= c->n_act && !st; ++i) {  // i = 0: the network input
+    __nv_bfloat16* p = i == 0 ? c->d_in : act_buf(c, i - 1);
+    const int planes = i == 0 ? 1 : 4;
+    st = conv_map(&c->m_in[i], p, c, planes);
+    if (!st && c->train) st = act_map(&c->m_dwa[i], p, c, planes, c->dw_px + 2, kDwRows + 2, false);
+  }
+  for (int i = 0; i < 3 && !st && c->train; ++i) {
+    st = conv_map(&c->m_zin[i], dz_buf(c, i), c, 4);
+    if (!st) st = act_map(&c->m_dwz[i], dz_buf(c, i), c, 4, c->dw_px, kDwRows, true);
   }
   if (!st) {
     std::vector<float> p;
@@ -1013,8 +1075,8 @@ int cnn_infer_range(lct_cnn* c, const float* d_vol, float* d_out, int nz, int z0
     a.inv_scale = 1.f / c->in_scale;
     a.bound = bound;
     a.n_reject = c->d_rej;
-    st = launch_conv<16, kEpiGate>(c->m_act[act_in(c, kCnnLayers - 1)], c->m_wf[kCnnLayers - 1],
-                                   a, B, c->device, c->sms, s);
+    const CUtensorMap& in = c->m_in[in_map(c, kCnnLayers - 1)];
+    st = launch_conv<kEpiGate, 4>(in, a, B, c->sms, s);
   }
   return st;
 }
