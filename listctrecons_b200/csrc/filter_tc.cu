@@ -7,14 +7,17 @@
 // (the dropped Rlo*Tlo term and the split residue are ~2^-16 relative per product).
 //
 // GEMM D[M x N] = A[M x K] B[K x N] with A = rows (K-major, as stored) and B given K-major as
-// B^T[n][k] = h[n - k + ns] (itself Toeplitz, materialised once per taps, zero padded to
-// Npad = Kpad = ns rounded up to 256).  One CTA computes a 128 x 256 tile of D:
-//   * 4 warps; warp 0 / lane 0 issues TMA loads (tiled, 128-byte swizzle, no multicast) of the
-//     four 64-deep K slices (A hi/lo 128 x 64, B hi/lo 256 x 64) into a 2-stage ring;
-//   * warp 1 / lane 0 issues tcgen05.mma.kind::f16 (M128 N256 K16, BF16 in, FP32 accumulate
-//     in TMEM, 3 products per K16 step) and frees each stage with tcgen05.commit;
-//   * all 4 warps drain the 128 x 256 FP32 accumulator from TMEM (tcgen05.ld 32x32b) and store
-//     the columns n < ns.
+// B^T[n][k] = h[n - k + ns] (itself Toeplitz, materialised once per taps).  Rows of planes are padded
+// to 8 samples (16 bytes); TMA's zero fill pads K to whole slices.  Persistent CTAs take 128 x 256 tiles
+// of D, columns fastest (a row block's planes then come from L2 for its second and third tile):
+//   * warp 0 issues TMA loads (tiled, 64-byte swizzle, no multicast) of 32-deep K slices -- P planes of
+//     A (128 x 32) and of B (256 x 32) -- into a ring of 3 (P = 3) or 4 (P = 2) stages;
+//   * warp 1 issues tcgen05.mma.kind::f16 (M128, N up to 256, K16, BF16 in, FP32 accumulate in TMEM; 3 or
+//     6 products per K16 step) into one of two accumulators and frees each stage with tcgen05.commit;
+//   * warps 2-5 drain the other accumulator (tcgen05.ld 32x32b) and store the columns n < ns.
+// Bound: tensor pipe.  Loading an M128 operand costs about 64 clocks and a column of N 0.4, so N is
+// as wide as TMEM takes twice.  117,312 rows of 736, P = 3: 0.53 ms (L2 feeds 8.8 TB/s of planes); 128 x 128 tiles, one per CTA with
+// load, math and store in turn, 0.69 ms.
 // Every mbarrier wait is bounded; a wait that runs out raises the device status word, the CTA
 // stops issuing work, waits (bounded) for the copies it started, frees its TMEM and returns.
 #include <cuda.h>
@@ -28,24 +31,19 @@
 
 namespace lct {
 
-constexpr int kTcM = 128, kTcK = 64, kTcStages = 2, kTcThreads = 128, kTcPad = 256;
+constexpr int kTcM = 128, kTcN = 256, kTcK = 32, kTcThreads = 192, kTcMaxStages = 4;
 
 // P = bf16 planes per operand: P = 2 -> 3 products (BF16x3), P = 3 -> 6 products (BF16x6).
-// Both keep a 96 KB stage: 128 x 256 tiles for P = 2, 128 x 128 for P = 3.
 template <int P>
 struct TcCfg {
-  static constexpr int N = P == 2 ? 256 : 128;
   static constexpr uint32_t TileA = kTcM * kTcK * 2;
-  static constexpr uint32_t TileB = N * kTcK * 2;
+  static constexpr uint32_t TileB = kTcN * kTcK * 2;
   static constexpr uint32_t Stage = P * TileA + P * TileB;
-  static constexpr uint32_t Smem = kTcStages * Stage + 128 + 1024;  // + barriers + alignment
-  static constexpr uint32_t TmemCols = N;
-  // kind::f16 instruction descriptor: FP32 D, BF16 A and B, both K-major, M x N
-  static constexpr uint32_t Idesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                                    ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
+  static constexpr int Stages = P == 2 ? 4 : 3;
+  static constexpr uint32_t Smem = Stages * Stage + 1024;  // + alignment
 };
 
-__host__ __device__ inline int tc_pad(int ns) { return (ns + kTcPad - 1) / kTcPad * kTcPad; }
+__host__ __device__ inline int tc_pad(int ns) { return (ns + 7) / 8 * 8; }
 
 // ---------------------------------------------------------------------------------------
 // operand preparation
@@ -60,7 +58,8 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16 (&p)[P]) {
   }
 }
 
-// rows fp32 [M][ns] -> P planes [M][kpad] (zero columns k >= ns); plane stride m * kpad
+// rows fp32 [M][ns] -> P planes [M][kpad] (zero columns k >= ns); plane stride m * kpad.  A thread
+// block takes one row
 template <int P>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ rows, long long m,
                                                          int ns, int kpad,
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(256) toeplitz_kernel(const float* __restrict__
 }
 
 // ---------------------------------------------------------------------------------------
-// the GEMM: grid (kpad / N, ceil(M / 128)), 128 threads, TcCfg<P>::Smem dynamic shared memory.
+// the GEMM: grid min(tiles, SMs), 192 threads, TcCfg<P>::Smem dynamic shared memory.
 // Products per K16 step: P = 2: (0,0) (0,1) (1,0);  P = 3: those and (0,2) (1,1) (2,0).
 // ---------------------------------------------------------------------------------------
 template <int P>
@@ -135,136 +134,172 @@ struct TcMaps {
 template <int P>
 __global__ void __launch_bounds__(kTcThreads, 1)
     filter_tc_kernel(const __grid_constant__ TcMaps<P> maps, float* __restrict__ out, long long m,
-                     int ns, int ktiles, int* status) {
+                     int ns, int n_tiles_n, long long n_tiles, int* status) {
   using Cfg = TcCfg<P>;
+  constexpr int S = Cfg::Stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kTcStages * Cfg::Stage);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kTcStages + 1);
+  __shared__ __align__(8) uint64_t bars[2 * kTcMaxStages + 5];
+  __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * Cfg::N;
-  const long long m0 = (long long)blockIdx.y * kTcM;
-  const uint32_t full0 = smem_u32(&bars[0]);
-  const uint32_t empty0 = smem_u32(&bars[kTcStages]);
-  const uint32_t accum = smem_u32(&bars[2 * kTcStages]);
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t stage0 = smem_u32(smem);
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kTcMaxStages]);
+  const uint32_t accf0 = smem_u32(&bars[2 * kTcMaxStages]), acce0 = accf0 + 16, mdone = accf0 + 32;
+  const int ktiles = (ns + kTcK - 1) / kTcK;
 
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int s = 0; s < kTcStages; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
     }
-    mbar_init(accum, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(accf0 + 8 * i, 1);
+      mbar_init(acce0 + 8 * i, 4);  // one arrival per epilogue warp
+    }
+    mbar_init(mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
+  if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "r"(Cfg::TmemCols)
+                     smem_u32(&tmem_slot)),
+                 "r"(2 * kTcN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_slot, 0);
+  auto aborted = [&] { return *reinterpret_cast<volatile int*>(&s_abort) != 0; };
 
-  if (warp == 0 && lane == 0) {
-    // producer: TMA ring, stage = P A-planes then P B-planes
-    int issued = 0;
-    for (int kt = 0; kt < ktiles; ++kt) {
-      const int s = kt % kTcStages;
-      if (kt >= kTcStages && !mbar_wait(empty0 + 8 * s, ((kt / kTcStages) - 1) & 1)) {
-        atomicExch(&s_abort, 1);
-        break;
-      }
-      if (atomicAdd(&s_abort, 0)) break;
-      uint8_t* st = smem + s * Cfg::Stage;
-      const uint32_t fb = full0 + 8 * s;
-      mbar_expect_tx(fb, Cfg::Stage);
-      const int k0 = kt * kTcK;
+  if (warp == 0) {
+    if (lane == 0) {
+      long long kg = 0;  // slices issued
+      bool stop = false;
+      for (long long t = blockIdx.x; t < n_tiles && !stop; t += gridDim.x) {
+        const int n0 = (int)(t % n_tiles_n) * kTcN, m0 = (int)(t / n_tiles_n) * kTcM;
+        for (int kt = 0; kt < ktiles; ++kt, ++kg) {
+          const int s = (int)(kg % S);
+          if (kg >= S && !mbar_wait(empty0 + 8 * s, (uint32_t)(((kg / S) - 1) & 1))) {
+            atomicExch(&s_abort, 1);
+            stop = true;
+            break;
+          }
+          if (aborted()) {
+            stop = true;
+            break;
+          }
+          const uint32_t st = stage0 + s * Cfg::Stage, fb = full0 + 8 * s;
+          mbar_expect_tx(fb, Cfg::Stage);
 #pragma unroll
-      for (int i = 0; i < P; ++i) tma_load_2d(smem_u32(st + i * Cfg::TileA), &maps.a[i], k0, (int)m0, fb);
+          for (int i = 0; i < P; ++i) tma_load_2d(st + i * Cfg::TileA, &maps.a[i], kt * kTcK, m0, fb);
 #pragma unroll
-      for (int i = 0; i < P; ++i)
-        tma_load_2d(smem_u32(st + P * Cfg::TileA + i * Cfg::TileB), &maps.b[i], k0, n0, fb);
-      issued = kt + 1;
-    }
-    // copies still in flight land on their full barriers before the CTA may exit
-    for (int kt = (issued > kTcStages ? issued - kTcStages : 0); kt < issued; ++kt)
-      if (atomicAdd(&s_abort, 0)) mbar_wait(full0 + 8 * (kt % kTcStages), (kt / kTcStages) & 1);
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer
-    for (int kt = 0; kt < ktiles; ++kt) {
-      const int s = kt % kTcStages;
-      if (!mbar_wait(full0 + 8 * s, (kt / kTcStages) & 1)) {
-        atomicExch(&s_abort, 1);
-        break;
-      }
-      tc_fence_after();
-      uint8_t* st = smem + s * Cfg::Stage;
-      uint64_t a[P], b[P];
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        a[i] = desc_sw128(smem_u32(st + i * Cfg::TileA));
-        b[i] = desc_sw128(smem_u32(st + P * Cfg::TileA + i * Cfg::TileB));
-      }
-#pragma unroll
-      for (int j = 0; j < kTcK / 16; ++j) {
-        const uint64_t dk = (uint64_t)((j * 32) >> 4);  // 16 bf16 = 32 bytes along K
-        umma_bf16(tmem, a[0] + dk, b[0] + dk, Cfg::Idesc, (kt | j) ? 1u : 0u);
-        umma_bf16(tmem, a[0] + dk, b[1] + dk, Cfg::Idesc, 1u);
-        umma_bf16(tmem, a[1] + dk, b[0] + dk, Cfg::Idesc, 1u);
-        if (P == 3) {
-          umma_bf16(tmem, a[0] + dk, b[P - 1] + dk, Cfg::Idesc, 1u);
-          umma_bf16(tmem, a[1] + dk, b[1] + dk, Cfg::Idesc, 1u);
-          umma_bf16(tmem, a[P - 1] + dk, b[0] + dk, Cfg::Idesc, 1u);
+          for (int i = 0; i < P; ++i)
+            tma_load_2d(st + P * Cfg::TileA + i * Cfg::TileB, &maps.b[i], kt * kTcK, n0, fb);
         }
       }
-      umma_commit(empty0 + 8 * s);
+      if (aborted())  // copies still in flight land on their full barriers before the CTA may exit
+        for (long long q = (kg > S ? kg - S : 0); q < kg; ++q)
+          mbar_wait(full0 + 8 * (int)(q % S), (uint32_t)((q / S) & 1));
     }
-    umma_commit(accum);
-  }
-  __syncwarp();
-
-  // epilogue: warp w owns TMEM lanes (rows) 32w .. 32w + 31
-  const bool done = mbar_wait(accum, 0);
-  tc_fence_after();
-  if (!done || atomicAdd(&s_abort, 0)) {
-    if (threadIdx.x == 0 && status) atomicExch(status, kDevWaitTimeout);
+  } else if (warp == 1) {
+    // the whole warp runs the loop, so that descriptors stay warp-uniform; one elected lane issues
+    long long kg = 0, it = 0;
+    bool ok = true;
+    for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++it) {
+      const int buf = (int)(it & 1), n0 = (int)(t % n_tiles_n) * kTcN;
+      const int n = min(kTcN, (ns - n0 + 15) / 16 * 16);
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+                             ((uint32_t)(kTcM >> 4) << 24);
+      const uint32_t d = tmem + (uint32_t)(buf * kTcN);
+      ok = __all_sync(0xFFFFFFFFu, it < 2 || mbar_wait(acce0 + 8 * buf, (uint32_t)(((it >> 1) - 1) & 1)));
+      for (int kt = 0; kt < ktiles && ok; ++kt, ++kg) {
+        const int s = (int)(kg % S);
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(full0 + 8 * s, (uint32_t)((kg / S) & 1)) && !aborted());
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t st = stage0 + s * Cfg::Stage;
+        if (elect_one()) {
+          uint64_t a[P], b[P];
+#pragma unroll
+          for (int i = 0; i < P; ++i) {
+            a[i] = desc_sw64(st + i * Cfg::TileA);
+            b[i] = desc_sw64(st + P * Cfg::TileA + i * Cfg::TileB);
+          }
+#pragma unroll
+          for (int j = 0; j < kTcK / 16; ++j) {
+            const uint64_t dk = (uint64_t)((j * 32) >> 4);  // 16 bf16 = 32 bytes along K
+            umma_bf16(d, a[0] + dk, b[0] + dk, idesc, (kt | j) ? 1u : 0u);
+            umma_bf16(d, a[0] + dk, b[1] + dk, idesc, 1u);
+            umma_bf16(d, a[1] + dk, b[0] + dk, idesc, 1u);
+            if (P == 3) {
+              umma_bf16(d, a[0] + dk, b[P - 1] + dk, idesc, 1u);
+              umma_bf16(d, a[1] + dk, b[1] + dk, idesc, 1u);
+              umma_bf16(d, a[P - 1] + dk, b[0] + dk, idesc, 1u);
+            }
+          }
+          umma_commit(empty0 + 8 * s);
+          if (kt == ktiles - 1) umma_commit(accf0 + 8 * buf);
+        }
+        __syncwarp();
+      }
+      if (!ok && lane == 0) atomicExch(&s_abort, 1);
+    }
+    if (elect_one()) umma_commit(mdone);  // every MMA issued above has finished once this arrives
+    __syncwarp();
+    if (!mbar_wait(mdone, 0)) atomicExch(&s_abort, 1);
   } else {
-    const long long row = m0 + warp * 32 + lane;
-    float* orow = out + row * ns;
+    // epilogue: the warp of quadrant q holds rows 32 q .. + 31 of the tile
+    const int q = warp & 3;
     // 16-byte stores only where every row start is 16-byte aligned
     const bool vec = ((ns & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    long long it = 0;
+    for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
+      const int buf = (int)(it & 1), n0 = (int)(t % n_tiles_n) * kTcN;
+      const long long row = (t / n_tiles_n) * kTcM + q * 32 + lane;
+      // warp-uniform decision: the TMEM loads below are .sync.aligned
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(accf0 + 8 * buf, (uint32_t)((it >> 1) & 1)))) {
+        if (lane == 0) atomicExch(&s_abort, 1);
+        break;
+      }
+      if (__any_sync(0xFFFFFFFFu, aborted())) break;
+      tc_fence_after();
+      float* orow = out + row * ns;
+      const int cols = min(kTcN, ns - n0);
 #pragma unroll 1
-    for (int c = 0; c < Cfg::N / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32), r);
-      const int col0 = n0 + c * 32;
-      if (row < m) {
-        if (vec && col0 + 32 <= ns) {
+      for (int c = 0; c < cols; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(tmem + (uint32_t)(buf * kTcN + c) + ((uint32_t)(q * 32) << 16), r);
+        const int col0 = n0 + c;
+        if (row < m) {
+          if (vec && col0 + 32 <= ns) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(orow + col0 + i) =
-                make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]),
-                            __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
-        } else {
+            for (int i = 0; i < 32; i += 4)
+              *reinterpret_cast<float4*>(orow + col0 + i) =
+                  make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]),
+                              __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+          } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (col0 + i < ns) orow[col0 + i] = __uint_as_float(r[i]);
+            for (int i = 0; i < 32; ++i)
+              if (col0 + i < ns) orow[col0 + i] = __uint_as_float(r[i]);
+          }
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acce0 + 8 * buf);
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0)
+  if (threadIdx.x == 0 && aborted() && status) atomicExch(status, kDevWaitTimeout);
+  if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(Cfg::TmemCols)
+                 "r"(2 * kTcN)
                  : "memory");
 }
 
@@ -285,7 +320,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// 2-D bf16 tensor [rows][cols] (cols contiguous), box {64, box_rows}, 128-byte swizzle
+// 2-D bf16 tensor [rows][cols] (cols contiguous), box {kTcK, box_rows}, 64-byte swizzle
 static int make_map(CUtensorMap* map, const void* base, long long rows, int cols, int box_rows) {
   auto fn = tensor_map_encoder();
   if (!fn) return LCT_ERR_UNSUPPORTED;
@@ -294,7 +329,7 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, int cols
   cuuint32_t box[2] = {(cuuint32_t)kTcK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? LCT_OK : LCT_ERR_ARG;
 }
@@ -318,17 +353,16 @@ int tc_build_toeplitz(int ns, const float* d_h, void* scratch, int mode, cudaStr
   return launch_status();
 }
 
-static bool tc_attr_done[2][64];
-
 template <int P>
 static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cudaStream_t s) {
   using Cfg = TcCfg<P>;
   const int kp = tc_pad(ns);
-  const long long mt = (nrows + kTcM - 1) / kTcM;
+  const int nt = (ns + kTcN - 1) / kTcN;
+  const long long mt = (nrows + kTcM - 1) / kTcM, tiles = mt * nt;
   if (mt > 65535) return LCT_ERR_ARG;
   __nv_bfloat16* b = static_cast<__nv_bfloat16*>(scratch);
-  __nv_bfloat16* a = b + (size_t)P * kp * kp;
-  if (ns % 4 == 0 && kp % 4 == 0 && reinterpret_cast<uintptr_t>(d_rows) % 16 == 0 &&
+  __nv_bfloat16* a = b + (size_t)P * kp * kp;  // 16-byte aligned: kp is a multiple of 8
+  if (ns % 4 == 0 && reinterpret_cast<uintptr_t>(d_rows) % 16 == 0 &&
       reinterpret_cast<uintptr_t>(a) % 8 == 0)
     split_rows4_kernel<P><<<(unsigned)((nrows + kSplitRows - 1) / kSplitRows), 256, 0, s>>>(
         reinterpret_cast<const float4*>(d_rows), nrows, ns / 4, kp / 4, reinterpret_cast<uint2*>(a));
@@ -339,24 +373,27 @@ static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cu
   TcMaps<P> maps;
   for (int i = 0; i < P; ++i) {
     if ((st = make_map(&maps.a[i], a + (size_t)i * nrows * kp, nrows, kp, kTcM))) return st;
-    if ((st = make_map(&maps.b[i], b + (size_t)i * kp * kp, kp, kp, Cfg::N))) return st;
+    if ((st = make_map(&maps.b[i], b + (size_t)i * kp * kp, kp, kp, kTcN))) return st;
   }
-  int dev = 0;
+  int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   {
     static std::mutex mu;  // host threads may share a device
+    static int sms_of[64] = {0};  // 0: attribute not set yet on that device
     std::lock_guard<std::mutex> lock(mu);
-    if (dev >= 64 || !tc_attr_done[P - 2][dev]) {
+    if (dev >= 64 || !sms_of[dev]) {
       if ((st = cuda_status(cudaFuncSetAttribute(filter_tc_kernel<P>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  Cfg::Smem))))
         return st;
-      if (dev < 64) tc_attr_done[P - 2][dev] = true;
+      if ((st = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))) return st;
+      if (dev < 64) sms_of[dev] = sms;
+    } else {
+      sms = sms_of[dev];
     }
   }
-  dim3 grid(kp / Cfg::N, (unsigned)mt);
-  filter_tc_kernel<P><<<grid, kTcThreads, Cfg::Smem, s>>>(maps, d_rows, nrows, ns, kp / kTcK,
-                                                          device_status_ptr());
+  filter_tc_kernel<P><<<(unsigned)std::min<long long>(tiles, sms), kTcThreads, Cfg::Smem, s>>>(
+      maps, d_rows, nrows, ns, nt, tiles, device_status_ptr());
   return launch_status();
 }
 

@@ -87,14 +87,14 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// K-major operand, 128-byte swizzle: 8-row x 128-byte atoms, 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
+// K-major operand, 64-byte swizzle: 8-row x 64-byte atoms, 512 bytes apart
+__device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {
   uint64_t d = 0;
   d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;            // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;  // stride byte offset: next 8-row atom
-  d |= (uint64_t)1 << 46;            // descriptor version
-  d |= (uint64_t)2 << 61;            // 128-byte swizzle
+  d |= (uint64_t)1 << 16;           // leading byte offset (unused for swizzled K-major)
+  d |= (uint64_t)(512 >> 4) << 32;  // stride byte offset: next 8-row atom
+  d |= (uint64_t)1 << 46;           // descriptor version
+  d |= (uint64_t)4 << 61;           // 64-byte swizzle
   return d;
 }
 // Unswizzled operand: core matrices of 8 rows x 16 bytes, 128 contiguous bytes each, so a tile may
