@@ -62,16 +62,17 @@ __device__ double noisy_integral(double p, double i0, uint64_t seed, uint64_t id
     n = floor(lam + sqrt(lam * (-2.0 * log(u1))) * cospi(2.0 * u2) + 0.5);
   }
   if (n < 1.0) n = 1.0;
-  return -log(n / i0);
+  return -log(n * (1.0 / i0));
 }
 
 // Bound: the FP64 pipe.  With M = the ellipsoid's frame scaled to a unit sphere, the ray S + l D
 // meets it where |M (S - c) + l M D| = 1, a quadratic with coefficients A = |M D|^2, B and C.  D is
 // (Dx, Dy) of the column and tz of the row, so A is a quadratic and B a line in tz whose
 // coefficients need the column only: a thread makes kSimRows rows of one column and pays, per
-// ellipsoid, 13 operations for the column and 5 per row (A, B, B^2 - A C), where the products with
-// the rotation and six divisions per ray took about 100.  The chord sqrt(disc) / A is one rsqrt.
-// 600 views x 64 x 736, 40 ellipsoids, I0 = 1e5: 1.3 ms, one ray per thread with everything
+// ellipsoid, about 20 operations for the column and 2 per row (the discriminant B^2 - A C, a quadratic
+// in the row), where the products with the rotation and six divisions per ray took about 100.  The
+// chord sqrt(disc) / A, where there is one, is one rsqrt.
+// 600 views x 64 x 736, 40 ellipsoids, I0 = 1e5: 1.1 ms, one ray per thread with everything
 // evaluated per ray 8.4 ms.
 constexpr int kSimRows = 16;     // rows per thread and pass
 constexpr int kSimThreads = 128; // columns per CTA
@@ -83,7 +84,7 @@ struct SimEllipsoid {            // one ellipsoid seen from one view
 };
 
 // grid (ceil(ns / 128), row chunks, views); CTA: 128 columns x rows_per_cta rows of one view
-__global__ void __launch_bounds__(kSimThreads) sim_project_kernel(
+__global__ void __launch_bounds__(kSimThreads, 5) sim_project_kernel(
     const double* __restrict__ ell, int ne, int ns, int nt, int rows_per_cta, float ds, float dt,
     float ws, float wt, float dso, const double* __restrict__ angles,
     const double* __restrict__ zpos, long long v0, double i0, uint64_t seed,
@@ -133,21 +134,28 @@ __global__ void __launch_bounds__(kSimThreads) sim_project_kernel(
     for (int r = 0; r < kSimRows; ++r) p[r] = 0.0;
     for (int m = 0; m < ne; ++m) {
       const SimEllipsoid& e = s_e[m];
-      // A and B at row it0 + r: A0 + r (A1 + r A2), B0 + r B1
+      // A and B at row it0 + r: A0 + r (A1 + r A2), B0 + r B1; the discriminant B^2 - A c is a
+      // quadratic in r too, and A is needed where it is positive only
       const double ul = fma(dx, e.xz2, dy * e.yz2), tl = fma(t0, e.zz, ul);
       const double A0 = fma(t0, tl, fma(dxx, e.xx, fma(dxy, e.xy2, dyy * e.yy)));
       const double A1 = step * fma(t0, e.zz, tl), A2 = step * step * e.zz;
       const double B0 = fma(t0, e.bz, fma(dx, e.bx, dy * e.by)), B1 = step * e.bz;
       const double c = e.c, mu2 = e.mu2;
+      const double d0 = fma(B0, B0, -(A0 * c)), d1 = fma(2.0 * B0, B1, -(A1 * c)), d2 = fma(B1, B1, -(A2 * c));
+      unsigned hit = 0;
 #pragma unroll
-      for (int r = 0; r < kSimRows; ++r) {
-        const double A = fma((double)r, fma((double)r, A2, A1), A0);
-        const double B = fma((double)r, B1, B0);
-        const double disc = fma(B, B, -(A * c));
-        if (disc > 0.0) p[r] = fma(mu2 * disc, rsqrt(disc * A * A), p[r]);  // sqrt(disc) / A
-      }
+      for (int r = 0; r < kSimRows; ++r)
+        if (fma((double)r, fma((double)r, d2, d1), d0) > 0.0) hit |= 1u << r;
+      if (!hit) continue;
+#pragma unroll
+      for (int r = 0; r < kSimRows; ++r)
+        if ((hit >> r) & 1u) {
+          const double disc = fma((double)r, fma((double)r, d2, d1), d0);
+          const double A = fma((double)r, fma((double)r, A2, A1), A0);
+          p[r] = fma(mu2 * disc, rsqrt(disc * A * A), p[r]);  // sqrt(disc) / A
+        }
     }
-#pragma unroll 1
+#pragma unroll 2
     for (int r = 0; r < kSimRows; ++r) {
       const int it = it0 + r;
       if (it >= row1) break;
