@@ -7,16 +7,16 @@
 // (the dropped Rlo*Tlo term and the split residue are ~2^-16 relative per product).
 //
 // GEMM D[M x N] = A[M x K] B[K x N] with A = rows (K-major, as stored) and B given K-major as
-// B^T[n][k] = h[n - k + ns] (itself Toeplitz, materialised once per taps).  Rows of planes are padded
-// to 8 samples (16 bytes); TMA's zero fill pads K to whole slices.  Persistent CTAs take 128 x 256 tiles
-// of D, columns fastest (a row block's planes then come from L2 for its second and third tile):
+// B^T[n][k] = h[n - k + ns] (itself Toeplitz, materialised once per taps), both zero padded to whole K
+// slices.  Persistent CTAs take tiles of D, 128 rows x up to 256 columns (tc_width), columns fastest (a
+// row block's planes then come from L2 for its second and third tile):
 //   * warp 0 issues TMA loads (tiled, 64-byte swizzle, no multicast) of 32-deep K slices -- P planes of
-//     A (128 x 32) and of B (256 x 32) -- into a ring of 3 (P = 3) or 4 (P = 2) stages;
+//     A (128 x 32) and of B (width x 32) -- into a ring of 3 to 6 stages;
 //   * warp 1 issues tcgen05.mma.kind::f16 (M128, N up to 256, K16, BF16 in, FP32 accumulate in TMEM; 3 or
 //     6 products per K16 step) into one of two accumulators and frees each stage with tcgen05.commit;
 //   * warps 2-5 drain the other accumulator (tcgen05.ld 32x32b) and store the columns n < ns.
-// Bound: tensor pipe.  Loading an M128 operand costs about 64 clocks and a column of N 0.4, so N is
-// as wide as TMEM takes twice.  117,312 rows of 736, P = 3: 0.53 ms (L2 feeds 8.8 TB/s of planes); 128 x 128 tiles, one per CTA with
+// Bound: tensor pipe and TMA.  Loading an M128 operand costs about 64 clocks and a column of N 0.4, so
+// N is as wide as TMEM takes twice.  117,312 rows of 736, P = 3: 0.53 ms; 128 x 128 tiles, one per CTA with
 // load, math and store in turn, 0.69 ms.
 // Every mbarrier wait is bounded; a wait that runs out raises the device status word, the CTA
 // stops issuing work, waits (bounded) for the copies it started, frees its TMEM and returns.
@@ -31,19 +31,17 @@
 
 namespace lct {
 
-constexpr int kTcM = 128, kTcN = 256, kTcK = 32, kTcThreads = 192, kTcMaxStages = 4;
+constexpr int kTcM = 128, kTcN = 256, kTcK = 32, kTcThreads = 192, kTcMaxStages = 6;
+constexpr uint32_t kTcSmem = 225 * 1024;  // dynamic shared memory: stages and alignment
 
 // P = bf16 planes per operand: P = 2 -> 3 products (BF16x3), P = 3 -> 6 products (BF16x6).
-template <int P>
-struct TcCfg {
-  static constexpr uint32_t TileA = kTcM * kTcK * 2;
-  static constexpr uint32_t TileB = kTcN * kTcK * 2;
-  static constexpr uint32_t Stage = P * TileA + P * TileB;
-  static constexpr int Stages = P == 2 ? 4 : 3;
-  static constexpr uint32_t Smem = Stages * Stage + 1024;  // + alignment
-};
+// a stage: P planes of A (128 x 32) and of B (width x 32)
+constexpr uint32_t kTcTileA = kTcM * kTcK * 2;
+__host__ __device__ constexpr uint32_t tc_tile_b(int width) { return (uint32_t)width * kTcK * 2; }
 
-__host__ __device__ inline int tc_pad(int ns) { return (ns + 7) / 8 * 8; }
+// planes are padded to whole 64-byte K slices, so that every row of a TMA box is aligned (404 columns
+// padded to 408, 816-byte rows: 3,500 clocks a stage instead of 2,200)
+__host__ __device__ inline int tc_pad(int ns) { return (ns + kTcK - 1) / kTcK * kTcK; }
 
 // ---------------------------------------------------------------------------------------
 // operand preparation
@@ -122,7 +120,7 @@ __global__ void __launch_bounds__(256) toeplitz_kernel(const float* __restrict__
 }
 
 // ---------------------------------------------------------------------------------------
-// the GEMM: grid min(tiles, SMs), 192 threads, TcCfg<P>::Smem dynamic shared memory.
+// the GEMM: grid min(tiles, SMs), 192 threads; tiles of 128 rows x `width` columns, S stages.
 // Products per K16 step: P = 2: (0,0) (0,1) (1,0);  P = 3: those and (0,2) (1,1) (2,0).
 // ---------------------------------------------------------------------------------------
 template <int P>
@@ -134,9 +132,8 @@ struct TcMaps {
 template <int P>
 __global__ void __launch_bounds__(kTcThreads, 1)
     filter_tc_kernel(const __grid_constant__ TcMaps<P> maps, float* __restrict__ out, long long m,
-                     int ns, int n_tiles_n, long long n_tiles, int* status) {
-  using Cfg = TcCfg<P>;
-  constexpr int S = Cfg::Stages;
+                     int ns, int width, int S, int n_tiles_n, long long n_tiles, int* status) {
+  const uint32_t tile_b = tc_tile_b(width), stage = P * (kTcTileA + tile_b);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -181,7 +178,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       long long kg = 0;  // slices issued
       bool stop = false;
       for (long long t = blockIdx.x; t < n_tiles && !stop; t += gridDim.x) {
-        const int n0 = (int)(t % n_tiles_n) * kTcN, m0 = (int)(t / n_tiles_n) * kTcM;
+        const int n0 = (int)(t % n_tiles_n) * width, m0 = (int)(t / n_tiles_n) * kTcM;
         for (int kt = 0; kt < ktiles; ++kt, ++kg) {
           const int s = (int)(kg % S);
           if (kg >= S && !mbar_wait(empty0 + 8 * s, (uint32_t)(((kg / S) - 1) & 1))) {
@@ -193,13 +190,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             stop = true;
             break;
           }
-          const uint32_t st = stage0 + s * Cfg::Stage, fb = full0 + 8 * s;
-          mbar_expect_tx(fb, Cfg::Stage);
+          const uint32_t st = stage0 + s * stage, fb = full0 + 8 * s;
+          mbar_expect_tx(fb, stage);
 #pragma unroll
-          for (int i = 0; i < P; ++i) tma_load_2d(st + i * Cfg::TileA, &maps.a[i], kt * kTcK, m0, fb);
+          for (int i = 0; i < P; ++i) tma_load_2d(st + i * kTcTileA, &maps.a[i], kt * kTcK, m0, fb);
 #pragma unroll
           for (int i = 0; i < P; ++i)
-            tma_load_2d(st + P * Cfg::TileA + i * Cfg::TileB, &maps.b[i], kt * kTcK, n0, fb);
+            tma_load_2d(st + P * kTcTileA + i * tile_b, &maps.b[i], kt * kTcK, n0, fb);
         }
       }
       if (aborted())  // copies still in flight land on their full barriers before the CTA may exit
@@ -211,8 +208,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     long long kg = 0, it = 0;
     bool ok = true;
     for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++it) {
-      const int buf = (int)(it & 1), n0 = (int)(t % n_tiles_n) * kTcN;
-      const int n = min(kTcN, (ns - n0 + 15) / 16 * 16);
+      const int buf = (int)(it & 1), n0 = (int)(t % n_tiles_n) * width;
+      const int n = min(width, (ns - n0 + 15) / 16 * 16);
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
                              ((uint32_t)(kTcM >> 4) << 24);
       const uint32_t d = tmem + (uint32_t)(buf * kTcN);
@@ -222,13 +219,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         ok = __all_sync(0xFFFFFFFFu, mbar_wait(full0 + 8 * s, (uint32_t)((kg / S) & 1)) && !aborted());
         if (!ok) break;
         tc_fence_after();
-        const uint32_t st = stage0 + s * Cfg::Stage;
+        const uint32_t st = stage0 + s * stage;
         if (elect_one()) {
           uint64_t a[P], b[P];
 #pragma unroll
           for (int i = 0; i < P; ++i) {
-            a[i] = desc_sw64(st + i * Cfg::TileA);
-            b[i] = desc_sw64(st + P * Cfg::TileA + i * Cfg::TileB);
+            a[i] = desc_sw64(st + i * kTcTileA);
+            b[i] = desc_sw64(st + P * kTcTileA + i * tile_b);
           }
 #pragma unroll
           for (int j = 0; j < kTcK / 16; ++j) {
@@ -255,11 +252,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   } else {
     // epilogue: the warp of quadrant q holds rows 32 q .. + 31 of the tile
     const int q = warp & 3;
-    // 16-byte stores only where every row start is 16-byte aligned
+    // 32-byte stores (whole sectors) where every row starts on 32 bytes, 16-byte ones on 16 bytes
+    const bool vec8 = ((ns & 7) == 0) && ((reinterpret_cast<uintptr_t>(out) & 31) == 0);
     const bool vec = ((ns & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
     long long it = 0;
     for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
-      const int buf = (int)(it & 1), n0 = (int)(t % n_tiles_n) * kTcN;
+      const int buf = (int)(it & 1), n0 = (int)(t % n_tiles_n) * width;
       const long long row = (t / n_tiles_n) * kTcM + q * 32 + lane;
       // warp-uniform decision: the TMEM loads below are .sync.aligned
       if (!__all_sync(0xFFFFFFFFu, mbar_wait(accf0 + 8 * buf, (uint32_t)((it >> 1) & 1)))) {
@@ -269,14 +267,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       if (__any_sync(0xFFFFFFFFu, aborted())) break;
       tc_fence_after();
       float* orow = out + row * ns;
-      const int cols = min(kTcN, ns - n0);
+      const int cols = min(width, ns - n0);
 #pragma unroll 1
       for (int c = 0; c < cols; c += 32) {
         uint32_t r[32];
         tmem_ld32(tmem + (uint32_t)(buf * kTcN + c) + ((uint32_t)(q * 32) << 16), r);
         const int col0 = n0 + c;
         if (row < m) {
-          if (vec && col0 + 32 <= ns) {
+          if (vec8 && c + 32 <= cols) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8)
+              stg256(orow + col0 + i, r[i], r[i + 1], r[i + 2], r[i + 3], r[i + 4], r[i + 5], r[i + 6], r[i + 7]);
+          } else if (vec && c + 32 <= cols) {
 #pragma unroll
             for (int i = 0; i < 32; i += 4)
               *reinterpret_cast<float4*>(orow + col0 + i) =
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (col0 + i < ns) orow[col0 + i] = __uint_as_float(r[i]);
+              if (c + i < cols) orow[col0 + i] = __uint_as_float(r[i]);
           }
         }
       }
@@ -353,12 +355,32 @@ int tc_build_toeplitz(int ns, const float* d_h, void* scratch, int mode, cudaStr
   return launch_status();
 }
 
+// Tile width: few wide tiles cost fewer operand loads, many narrow ones fill the last round of SMs and
+// leave less epilogue exposed at the end.  Per MMA about 64 + 0.37 width clocks, or what TMA takes to
+// deliver the stage (29 bytes per clock and SM in rows of 64 bytes, few SMs loading or all).  736 columns,
+// clocks per MMA: 256 wide 211, 192 wide 185, 128 wide 144.
+static int tc_width(int ns, long long mt, int P, int sms) {
+  const int prods = P == 3 ? 6 : 3;
+  const double steps = (double)((ns + kTcK - 1) / kTcK) * 2 * prods;
+  int best = kTcN;
+  double best_cost = 1e300;
+  for (int nt = (ns + kTcN - 1) / kTcN; nt <= (ns + 63) / 64; ++nt) {
+    const int w = ((ns + nt - 1) / nt + 15) / 16 * 16;
+    const long long tiles = mt * ((ns + w - 1) / w);
+    const double mma = std::max(64.0 + 0.37 * w, P * (kTcTileA + (double)tc_tile_b(w)) / (2 * prods) / 29.0);
+    const double cost = (double)((tiles + sms - 1) / sms) * steps * mma + 20.0 * w;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = w;
+    }
+  }
+  return best;
+}
+
 template <int P>
 static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cudaStream_t s) {
-  using Cfg = TcCfg<P>;
   const int kp = tc_pad(ns);
-  const int nt = (ns + kTcN - 1) / kTcN;
-  const long long mt = (nrows + kTcM - 1) / kTcM, tiles = mt * nt;
+  const long long mt = (nrows + kTcM - 1) / kTcM;
   if (mt > 65535) return LCT_ERR_ARG;
   __nv_bfloat16* b = static_cast<__nv_bfloat16*>(scratch);
   __nv_bfloat16* a = b + (size_t)P * kp * kp;  // 16-byte aligned: kp is a multiple of 8
@@ -370,11 +392,6 @@ static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cu
     split_rows_kernel<P><<<(unsigned)nrows, 256, 0, s>>>(d_rows, nrows, ns, kp, a);
   int st = launch_status();
   if (st) return st;
-  TcMaps<P> maps;
-  for (int i = 0; i < P; ++i) {
-    if ((st = make_map(&maps.a[i], a + (size_t)i * nrows * kp, nrows, kp, kTcM))) return st;
-    if ((st = make_map(&maps.b[i], b + (size_t)i * kp * kp, kp, kp, kTcN))) return st;
-  }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   {
@@ -384,7 +401,7 @@ static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cu
     if (dev >= 64 || !sms_of[dev]) {
       if ((st = cuda_status(cudaFuncSetAttribute(filter_tc_kernel<P>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 Cfg::Smem))))
+                                                 kTcSmem))))
         return st;
       if ((st = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))) return st;
       if (dev < 64) sms_of[dev] = sms;
@@ -392,8 +409,17 @@ static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cu
       sms = sms_of[dev];
     }
   }
-  filter_tc_kernel<P><<<(unsigned)std::min<long long>(tiles, sms), kTcThreads, Cfg::Smem, s>>>(
-      maps, d_rows, nrows, ns, nt, tiles, device_status_ptr());
+  const int w = tc_width(ns, mt, P, sms);
+  TcMaps<P> maps;
+  for (int i = 0; i < P; ++i) {
+    if ((st = make_map(&maps.a[i], a + (size_t)i * nrows * kp, nrows, kp, kTcM))) return st;
+    if ((st = make_map(&maps.b[i], b + (size_t)i * kp * kp, kp, kp, w))) return st;
+  }
+  const uint32_t stage = P * (kTcTileA + tc_tile_b(w));
+  const int S = (int)std::min<uint32_t>(kTcMaxStages, (kTcSmem - 1024) / stage);
+  const int nt = (ns + w - 1) / w;
+  filter_tc_kernel<P><<<(unsigned)std::min<long long>(mt * nt, sms), kTcThreads, S * stage + 1024, s>>>(
+      maps, d_rows, nrows, ns, w, S, nt, mt * nt, device_status_ptr());
   return launch_status();
 }
 

@@ -74,6 +74,13 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, uint32_
 }
 // waits for the calling thread's own copies
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// one 32-byte store (32-byte aligned)
+__device__ __forceinline__ void stg256(float* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
+                                       uint32_t f, uint32_t g, uint32_t h) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a), "r"(b), "r"(c),
+               "r"(d), "r"(e), "r"(f), "r"(g), "r"(h)
+               : "memory");
+}
 __device__ __forceinline__ float4 lds128(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
