@@ -230,10 +230,11 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
   __shared__ int2 s_jr[kQVB];        // slices [jlo, jhi) of the chunk whose window holds ia
   __shared__ float2 s_zb[kQVB];      // EXACT: source z of both views without the fan-angle term
   __shared__ ulonglong2 s_qv[kQVB];  // biased bases of both views (quad_view_bias)
-  __shared__ ulonglong2 s_pfb[kQVB]; // prefetch box origins of both views
-  __shared__ int4 s_pfs[kQVB];       // prefetch box rows and column spans
+  __shared__ unsigned long long s_pfb[2][kQVB];  // prefetch box origins of the views and conjugates
+  __shared__ int2 s_pfs[2][kQVB];                // prefetch box rows and column spans
 
   const int tid = threadIdx.y * kQTX + threadIdx.x;
+  const unsigned pf_off = (unsigned)((tid >> 4) & 7) * A.qrow_bytes;  // this thread's row of a prefetch box
   const int ix = bx * kQTX + threadIdx.x;
   const int iy = by * kQTY + threadIdx.y;
   const int slab = bz / A.zchunks;
@@ -299,10 +300,10 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
                                   quad_view_bias<INTERP>(v2, A.qrow_bytes));
       int4 b1, b2;
       prefetch_boxes(A, c1, s1, c2, s2, ia, xr0, xr1, yr0, yr1, zc0, zcl, b1, b2);
-      s_pfb[tid] = make_ulonglong2(
-          reinterpret_cast<unsigned long long>(v1) + (unsigned long long)b1.x * A.qrow_bytes + 16ull * b1.z,
-          reinterpret_cast<unsigned long long>(v2) + (unsigned long long)b2.x * A.qrow_bytes + 16ull * b2.z);
-      s_pfs[tid] = make_int4(b1.y - b1.x + 1, b1.w - b1.z, b2.y - b2.x + 1, b2.w - b2.z);
+      s_pfb[0][tid] = reinterpret_cast<unsigned long long>(v1) + (unsigned long long)b1.x * A.qrow_bytes + 16ull * b1.z;
+      s_pfb[1][tid] = reinterpret_cast<unsigned long long>(v2) + (unsigned long long)b2.x * A.qrow_bytes + 16ull * b2.z;
+      s_pfs[0][tid] = make_int2(b1.y - b1.x + 1, b1.w - b1.z);
+      s_pfs[1][tid] = make_int2(b2.y - b2.x + 1, b2.w - b2.z);
       int jlo = nzc, jhi = 0;
       for (int j = 0; j < nzc; ++j)
         if (ia >= A.a_min[z0 + j] && ia < A.a_mid[z0 + j]) {
@@ -321,14 +322,11 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         // its value unused: a load brings in the sector it touches, and a prefetch instruction
         // does no better per sector and costs more (512^2 x 256 from 736 x 64 views: 64.5 ms so,
         // 70.8 ms with one prefetch.global.L1 per 128-byte line, slower with one per sector).
-        const int pf_conj = tid >> 7, pf_col = 2 * (tid & 15);
-        const int4 sz = s_pfs[k + 1];
-        const int rows = pf_conj ? sz.z : sz.x, cspan = pf_conj ? sz.w : sz.y;
-        if (pf_col <= cspan + 1) {
-          const ulonglong2 bs = s_pfb[k + 1];
-          unsigned long long a = (pf_conj ? bs.y : bs.x) + 16ull * (unsigned)min(pf_col, cspan) +
-                                 (unsigned long long)((tid >> 4) & 7) * A.qrow_bytes;
-          for (int r = (tid >> 4) & 7; r < rows; r += 8, a += 8ull * A.qrow_bytes) {
+        const int2 sz = s_pfs[tid >> 7][k + 1];
+        const int pf_col = 2 * (tid & 15);
+        if (pf_col <= sz.y + 1) {
+          unsigned long long a = s_pfb[tid >> 7][k + 1] + 16u * (unsigned)min(pf_col, sz.y) + pf_off;
+          for (int r = (tid >> 4) & 7; r < sz.x; r += 8, a += 8u * A.qrow_bytes) {
             unsigned unused;
             asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(unused) : "l"(a));
           }
@@ -356,7 +354,7 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
           theta = asinf(sx);
         const float tho = __fmul_rn(theta, A.inv_orbit);
         const float t = fmaf(-phat, phat, A.dso2);
-        const float sq = __fmul_rn(t, rsqrtf(t));
+        const float sq = __fmul_rn(t, rsqrt_fast(t));
         const float l1 = fmaf(xc, sb, fmaf(-yc, cb, sq));
         const float l2 = fmaf(xc, sb2, fmaf(-yc, cb2, sq));
         // source z from the staged per-view term: zr = (ia + tho) dzv + z0
@@ -364,7 +362,7 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         const float zr1 = fmaf(tho, A.dzv, zb.x), zr2 = fmaf(-tho, A.dzv, zb.y);
         // k = kq / l, kd = k dz (no per-slice z register); weights halved around one reciprocal --
         // the factor 2 is restored, exactly, at the output
-        const float r1 = __fdividef(1.0f, l1), r2 = __fdividef(1.0f, l2);
+        const float r1 = rcp_fast(l1), r2 = rcp_fast(l2);
         K = make_float2(__fmul_rn(A.kqdz, r1), __fmul_rn(A.kqdz, r2));
         M = make_float2(__fmul_rn(__fsub_rn(zc0, zr1), __fmul_rn(A.kq, r1)),
                         __fmul_rn(__fsub_rn(zc0, zr2), __fmul_rn(A.kq, r2)));
@@ -380,7 +378,7 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         const float l2 = fmaf(xc, sb2, fmaf(-yc, cb2, sq));
         const float zr1 = fmaf(__fadd_rn((float)ia, tho), A.dzv, A.z0);
         const float zr2 = fmaf(__fsub_rn((float)(ia + A.half), tho), A.dzv, A.z0);
-        K = make_float2(__fdividef(A.kq, l1), __fdividef(A.kq, l2));
+        K = make_float2(__fmul_rn(A.kq, rcp_fast(l1)), __fmul_rn(A.kq, rcp_fast(l2)));
         M = make_float2(__fmul_rn(-zr1, K.x), __fmul_rn(-zr2, K.y));
         // the reference's texture coordinate carries + 0.5
         q1 = quad_col(qv.x, __fsub_rn(__fadd_rn(__fadd_rn(delta_p, A.ws), 0.5f), 0.5f), A.ns, a1);
@@ -422,14 +420,14 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         if constexpr (INTERP == LCT_INTERP_EXACT) {
           // the pair weights sum to one in every case -- (-qh2, qh1) / (qh1 - qh2), (0, 1),
           // (1, 0), (1/2, 1/2) -- so w1 s1 + w2 s2 = s2 + w1 (s1 - s2)
-          float w1 = -qh.y * __fdividef(1.0f, qh.x - qh.y);
+          float w1 = -qh.y * rcp_fast(qh.x - qh.y);
           if constexpr (!kIn) w1 = out1 ? (out2 ? 0.5f : 0.0f) : (out2 ? 1.0f : w1);
           const float2 p0 = __ffma2_rn(A1, make_float2(v0.z, v0.w), make_float2(v0.x, v0.y));
           const float2 p1 = __ffma2_rn(A2, make_float2(v1.z, v1.w), make_float2(v1.x, v1.y));
           const float s1 = fmaf(b.x, p0.y, p0.x), s2 = fmaf(b.y, p1.y, p1.x);
           sum = fmaf(w1, s1 - s2, acc[j] + s2);
         } else {
-          const float r = __fdividef(2.0f, qh.x - qh.y);
+          const float r = 2.0f * rcp_fast(qh.x - qh.y);
           float w1 = -qh.y * r, w2 = qh.x * r;
           if constexpr (!kIn) {
             w1 = out1 ? (out2 ? 1.0f : 0.0f) : (out2 ? 2.0f : w1);

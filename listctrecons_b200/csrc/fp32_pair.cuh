@@ -21,6 +21,20 @@ __device__ __forceinline__ float2 f2sub(float2 x, float2 y) {
 constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kFloorBits = 0x4B400000;
 
+// The hardware's approximate reciprocal and reciprocal square root without the scaling that the
+// general forms wrap around them for subnormal and huge arguments (distances and row differences are
+// neither); the same values otherwise.
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_fast(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // x / d rounded to nearest for a launch-constant d with r = RN(1 / d): the quotient estimate's
 // remainder is exact in an FMA and one more FMA rounds correctly (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34(1), 1990), except
