@@ -411,9 +411,11 @@ __global__ void __launch_bounds__(256) cnn_loss_kernel(const float* __restrict__
 // (whatever lies outside the image reads as zero).  A CTA accumulates over all its tiles in three TMEM
 // accumulators, sums the blocks over j in shared memory and adds them to the gradient once.  Four
 // further warps sum the staged deltas per channel: the bias gradient.
-// Bound: the MMAs' operand loads.  16 x 256^2: 42-49 us per layer; with one tap's activations as M128 and
-// N32, and a separate pass for the biases, 57-87 + 24 us.
+// Bound: the MMAs' operand loads (about 137 clocks each, 1.7 us per tile and SM, 32 of 40 us).  16 x 256^2:
+// 39-41 us per layer; with one tap's activations as M128 and N32, and a separate pass for the biases,
+// 57-87 + 24 us.
 constexpr int kDwThreads = 192, kDwSums = kDwThreads / 32 - 2, kDwGroups = 2, kDwRows = 3 * kDwGroups, kDwMaxP = 64, kDwMaxStages = 4;
+constexpr int kDwPitch = 33, kDwPart = 9 * kCnnC * kDwPitch;  // a warp's gradient blocks: [ci][tap][co], padded rows
 
 template <int PLANES>  // planes of the activation: 1 (network input) or 4
 __global__ void __launch_bounds__(kDwThreads, 1)
@@ -423,6 +425,7 @@ __global__ void __launch_bounds__(kDwThreads, 1)
   __shared__ __align__(8) uint64_t bars[2 * kDwMaxStages + 1];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
+  __shared__ float s_bias[kDwSums][32];
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int P = a.n_px, S = a.stages;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kDwMaxStages]);
@@ -506,7 +509,9 @@ __global__ void __launch_bounds__(kDwThreads, 1)
     }
     if (elect_one()) umma_commit(mdone);
   } else if (warp >= 2) {
-    // bias gradient: lane = (plane, pixel mod 8), every fourth delta row
+    // bias gradient: lane = (plane, pixel mod 8), every fourth delta row; the eight lanes of a plane read
+    // 128 consecutive bytes (lane = (pixel mod 8, plane): planes a multiple of 128 bytes apart, 4-way
+    // bank conflicts in the memory that feeds the MMAs; 2-3 us of a 16 x 256^2 layer)
     float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     long long k = 0;
     for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
@@ -519,9 +524,9 @@ __global__ void __launch_bounds__(kDwThreads, 1)
       conv_tile(a, t, x0, y0, b);
       const int px = min(P, a.W - x0), zrows = min(kDwRows, a.H - y0);
       for (int r = warp - 2; r < zrows; r += kDwSums) {
-        const uint8_t* p = smem + (size_t)s * a.stage_bytes + zoff + (uint32_t)(4 * r + (lane & 3)) * zs;
+        const uint8_t* p = smem + (size_t)s * a.stage_bytes + zoff + (uint32_t)(4 * r + (lane >> 3)) * zs;
 #pragma unroll 4
-        for (int i = lane >> 2; i < px; i += 8) {
+        for (int i = lane & 7; i < px; i += 8) {
           const uint4 q = *reinterpret_cast<const uint4*>(p + i * 16);
           const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -536,11 +541,10 @@ __global__ void __launch_bounds__(kDwThreads, 1)
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
+      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 1);
+      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 2);
       sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 4);
-      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 8);
-      sum[e] += __shfl_xor_sync(0xFFFFFFFFu, sum[e], 16);
-      const int co = 8 * lane + e;
-      if (lane < 4 && co < cout && !conv_aborted(&s_abort)) atomicAdd(&gb[co], sum[e]);
+      if ((lane & 7) == 0) s_bias[warp - 2][lane + e] = sum[e];  // channel 8 (lane / 8) + e
     }
   }
   __syncwarp();
@@ -550,29 +554,41 @@ __global__ void __launch_bounds__(kDwThreads, 1)
   if (!done || conv_aborted(&s_abort)) {
     if (threadIdx.x == 0 && a.status) atomicExch(a.status, kDevWaitTimeout);
   } else {
-    // warp j < 3 holds delta row j, lane = co: block (o, dx) is tap dy = o - j; the stages are free now
-    float* part = reinterpret_cast<float*>(smem);  // [dy][dx][ci][co]
-    for (int j = 0; j < 3; ++j) {
-      if (warp == j) {
+    // warp j < 3 holds delta row j, lane = co: block (o, dx) is tap dy = o - j.  The stages are free now:
+    // each of the three warps lays its blocks out there, and every thread sums them over j on its way to
+    // the gradient.  [ci][tap] in the gradient's own order and rows of 33, so neither side meets a bank
+    // conflict ([tap][ci][co], summed over j by the three warps in turn: 32-way conflicts, 48 -> 44.5 us)
+    float* part = reinterpret_cast<float*>(smem);  // [j][ci][tap][co]
+    if (warp < 3) {
 #pragma unroll
-        for (int tap = 0; tap < 9; ++tap) {
-          uint32_t r[PLANES == 1 ? 16 : 32];
-          const uint32_t at = tmem + (uint32_t)((tap % 3) * kN + (j + tap / 3) * kCi) + ((uint32_t)(j * 32) << 16);
-          if constexpr (PLANES == 1)
-            tmem_ld16(at, r);
-          else
-            tmem_ld32(at, r);
-          float* p = part + tap * kCi * 32 + lane;
+      for (int tap = 0; tap < 9; ++tap) {
+        uint32_t r[PLANES == 1 ? 16 : 32];
+        const uint32_t at =
+            tmem + (uint32_t)((tap % 3) * kN + (warp + tap / 3) * kCi) + ((uint32_t)(warp * 32) << 16);
+        if constexpr (PLANES == 1)
+          tmem_ld16(at, r);
+        else
+          tmem_ld32(at, r);
+        float* p = part + warp * kDwPart + tap * kDwPitch + lane;
 #pragma unroll
-          for (int ci = 0; ci < kCi; ++ci) p[ci * 32] = (j ? p[ci * 32] : 0.f) + __uint_as_float(r[ci]);
-        }
+        for (int ci = 0; ci < kCi; ++ci) p[ci * 9 * kDwPitch] = __uint_as_float(r[ci]);
       }
-      __syncthreads();
     }
-    for (int i = threadIdx.x; i < cout * cin * 9; i += kDwThreads) {
-      const int tap = i % 9, ci = i / 9 % cin, co = i / (9 * cin);
-      atomicAdd(&gw[i], part[(tap * kCi + ci) * 32 + co]);
+    __syncthreads();
+    // one warp adds the biases: all CTAs meet on one 128-byte line, and an atomic of each summing warp and
+    // channel took its L2 slice about 5 us
+    if (threadIdx.x < cout) {
+      float b = 0.f;
+#pragma unroll
+      for (int w = 0; w < kDwSums; ++w) b += s_bias[w][threadIdx.x];
+      atomicAdd(&gb[threadIdx.x], b);
     }
+    const int per = 9 * cin;
+    for (int co = warp; co < cout; co += kDwThreads / 32)
+      for (int i = lane; i < per; i += 32) {
+        const float* p = part + i * kDwPitch + co;
+        atomicAdd(&gw[co * per + i], (p[0] + p[kDwPart]) + p[2 * kDwPart]);
+      }
   }
   tc_fence_before();
   __syncthreads();
@@ -820,7 +836,7 @@ static int cnn_backward_impl(lct_cnn* c, const float* d_in5, const float* d_targ
     // the last group's discarded delta row, and the network input's sixth activation row, read past it
     const uint32_t tail = 4 * (uint32_t)da.n_px * 16 + 2 * dw_plane(da.n_px);
     da.stages = std::min<int>(kDwMaxStages, (int)((kSmemMax - tail) / da.stage_bytes));
-    const size_t dw_smem = std::max((size_t)da.stages * da.stage_bytes + tail, sizeof(float) * 9 * kCnnC * kCnnC);
+    const size_t dw_smem = std::max((size_t)da.stages * da.stage_bytes + tail, sizeof(float) * 3 * kDwPart);
     auto dw = l == 0 ? cnn_dw_tc_kernel<1> : cnn_dw_tc_kernel<4>;
     dw<<<dw_grid, kDwThreads, dw_smem, s>>>(c->m_dwa[in_map(c, l)], c->m_dwz[cur], da, cnn_cin(l), cnn_cout(l),
                                             gw, gb);
