@@ -419,14 +419,14 @@ __global__ void __launch_bounds__(kPiTX* kPiTY, 4) bp_pi_ori_z_kernel(const __gr
   const float pitch = A.pitch;
   const float t2 = (float)((double)pitch / (2 * kRefPi));  // :209, double through PI
   const float rows2 = (float)(2 * (A.nt - 1));  // t * 2 * (nt - 1): the doubling is exact
-  float zc[kPiNZ], sum[kPiNZ];
+  float zi[kPiNZ], sum[kPiNZ];  // slice j's number from the central one
   int amid[kPiNZ], amin[kPiNZ];
   unsigned walking = 0;  // bit j: slice j's backward walk has not stopped
   int vtop = -1;
 #pragma unroll
   for (int j = 0; j < kPiNZ; ++j) {
-    zc[j] = ((float)(z0 + j) - A.wz) * A.dz;
-    int a = (int)roundf((zc[j] - A.z0) / A.dzv);
+    zi[j] = (float)(z0 + j) - A.wz;
+    int a = (int)roundf((zi[j] * A.dz - A.z0) / A.dzv);
     a = a < 0 ? 0 : a;
     a = a > A.n_angle - 1 ? A.n_angle - 1 : a;
     amid[j] = a;
@@ -472,8 +472,10 @@ __global__ void __launch_bounds__(kPiTX* kPiTY, 4) bp_pi_ori_z_kernel(const __gr
   };
   // slices j and j + 1 of view w: t of both (the reference's expression, times the direction's sign)
   auto tval2 = [&](const ViewTerms& w, int j) {
-    const float2 z = make_float2(zc[j], zc[j + 1]);
-    const float2 x = __fmul2_rn(f2(w.temp1), __fadd2_rn(__fadd2_rn(z, f2(-w.zv)), f2(-w.gt2)));
+    // the slice's z less the source's with one rounding: rounding the slice's z first moves t by an ulp of
+    // z, and some voxels in 100,000 then stop their walk a view apart
+    const float2 z = __ffma2_rn(make_float2(zi[j], zi[j + 1]), f2(A.dz), f2(-w.zv));
+    const float2 x = __fmul2_rn(f2(w.temp1), __fadd2_rn(z, f2(-w.gt2)));
     return __fadd2_rn(div_by2(x, w.den, w.rden), f2(w.gz));
   };
   // row coordinates: TEX8 the reference's expression, whose rounding decides 8-bit weights; EXACT one FMA
