@@ -740,6 +740,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
       L.interp = interp;
       L.addr = addr;
       L.nz_thread = bp_nz_default(*g, *ig);
+      L.z_base = 8;
       st = launch_bp_par_quads(*g, *ig, L, q, s);
     }
     int st2 = scratch_free(q, s);

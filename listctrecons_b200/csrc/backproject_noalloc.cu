@@ -80,5 +80,6 @@ LCT_API int lct_backproject_par_noalloc(const lct_geom* g, const lct_img* ig,
   L.interp = interp;
   L.addr = addr;
   L.nz_thread = bp_nz_default(*g, *ig);
+  L.z_base = 8;
   return launch_bp_par_quads(*g, *ig, L, q, s);
 }

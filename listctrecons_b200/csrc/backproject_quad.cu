@@ -14,7 +14,7 @@
 // EXACT keeps FP64 view trigonometry and full FP32 weights; TEX8 keeps the reference's order
 // for the sample column (phat/dso, theta*dso/ds) and the texture unit's 8-bit weight rules, bit
 // for bit, in the same packed path: divisions by launch constants as three FMAs, 8-bit weights as
-// whole numbers from round-down adds (256^2 x 32 from 672 x 16 views: 4.17 ms, 5.13 ms in scalar
+// whole numbers from round-down adds (256^2 x 32 from 672 x 16 views: 4.05 ms, 5.13 ms in scalar
 // code with IEEE divisions, FRND and F2I).
 // Both: floor, fraction and index of a sample from one round-down add (no conversions)
 // and one wide multiply-add for its address; per-view terms staged in shared memory 128 views
@@ -83,6 +83,7 @@ struct BpQuadArgs {
   int view_lo, view_hi, part;  // BpLaunch::view_lo / view_hi / part
   float kqdz;           // kq * dz (EXACT: row step per slice = kqdz / l)
   unsigned qrow_bytes;  // bytes per quad row, 16 * qcols
+  int z_base;           // EXACT: slices whose row coordinates share one base (0: a thread's)
   int rows_inside_ok;   // 2 wt + 2.5 < nt + 3: |qhat| <= wt puts floor(qhat + wt + 2) in [1, nt + 2]
   int slab_view[kBpMaxSlabs];
   int slab_z0[kBpMaxSlabs];
@@ -224,7 +225,7 @@ __device__ __forceinline__ float asin_half(float x) {
 
 // One tile: voxel columns [bx*kQTX, +kQTX) x [by*kQTY, +kQTY), slab/slice chunk bz.  Called with
 // CTA-uniform arguments by every thread of a 256-thread CTA.
-template <int NZ, int INTERP, bool PART, bool RING>
+template <int NZ, int INTERP, bool PART, bool RING, bool BASED>
 __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by, int bz) {
   __shared__ float4 s_cs[kQVB];      // cos, sin of view ia and of its conjugate ia + half
   __shared__ int2 s_jr[kQVB];        // slices [jlo, jhi) of the chunk whose window holds ia
@@ -247,6 +248,11 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
   const float xc = __fmul_rn((float)ix - A.wx, A.dx);
   const float yc = __fmul_rn((float)iy - A.wy, A.dy);
   const float zc0 = __fmul_rn((float)z0 - A.wz, A.dz);
+  // EXACT row coordinates are base + (slice - base's slice) kd: threads of fewer slices than a base
+  // serves keep that base (BASED), so every slice is rounded as in a thread of z_base slices
+  const int zb = BASED && A.z_base > NZ ? z0 / A.z_base * A.z_base : z0;
+  const int jb = z0 - zb;
+  const float zcb = __fmul_rn((float)zb - A.wz, A.dz);
   const float wt2 = A.wt + 2.0f;
   // prefetch: the tile's corner coordinates and last slice
   const float xr0 = __fmul_rn((float)(bx * kQTX) - A.wx, A.dx);
@@ -364,8 +370,8 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         // the factor 2 is restored, exactly, at the output
         const float r1 = rcp_fast(l1), r2 = rcp_fast(l2);
         K = make_float2(__fmul_rn(A.kqdz, r1), __fmul_rn(A.kqdz, r2));
-        M = make_float2(__fmul_rn(__fsub_rn(zc0, zr1), __fmul_rn(A.kq, r1)),
-                        __fmul_rn(__fsub_rn(zc0, zr2), __fmul_rn(A.kq, r2)));
+        M = make_float2(__fmul_rn(__fsub_rn(zcb, zr1), __fmul_rn(A.kq, r1)),
+                        __fmul_rn(__fsub_rn(zcb, zr2), __fmul_rn(A.kq, r2)));
         U = make_float2(__fadd_rn(M.x, wt2), __fadd_rn(M.y, wt2));
         q1 = quad_col(qv.x, fmaf(theta, A.dso_over_ds, A.ws), A.ns, a1);
         q2 = quad_col(qv.y, fmaf(-theta, A.dso_over_ds, A.ws), A.ns, a2);
@@ -387,9 +393,9 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         a2 = q8(a2);
       }
       const float2 A1 = f2(a1), A2 = f2(a2);
-      // J of slice j: EXACT its number (a constant), TEX8 its z
+      // J of slice j: EXACT its number from the base (a constant where a thread has its own), TEX8 its z
       auto slice_j = [&](int j) {
-        return INTERP == LCT_INTERP_EXACT ? (float)j : __fmul_rn(__fsub_rn((float)(z0 + j), A.wz), A.dz);
+        return INTERP == LCT_INTERP_EXACT ? (BASED ? (float)(jb + j) : (float)j) : __fmul_rn(__fsub_rn((float)(z0 + j), A.wz), A.dz);
       };
       // one slice of the pair, the view and its conjugate as one packed FP32 pair; INSIDE: both
       // samples lie within the detector rows (no tests, no selects, no row clamps).  A slice
@@ -452,7 +458,7 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
       // skipped with no change to any result.  The row coordinate (equal to qhat + wt within a
       // few ulps, far below half a row) then lies inside the quad rows when rows_inside_ok.  A
       // NaN fails the test.  (EXACT, 512^2 x 256 from 736 x 64 views: 69.4 ms with scalar code and
-      // no inside path on partial windows, 64.5 ms so.)
+      // no inside path on partial windows, 64.3 ms so.)
       const float jf = slice_j(jlo & ~(kQGroup - 1));
       const float jl = slice_j(((jhi + kQGroup - 1) & ~(kQGroup - 1)) - 1);
       const bool inside = A.rows_inside_ok && fabsf(fmaf(jf, K.x, M.x)) <= wt &&
@@ -504,9 +510,15 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
 // PART: a view range of the slabs with raw sums carried in img (BpLaunch::part); the whole-
 // launch instantiation has none of that code.  RING: the quads are a ring (bounded recons); the
 // linear instantiation has no modulo in its view bases.
-template <int NZ, int INTERP, int MINB, bool PART, bool RING>
+// BASED: the threads' slices may share their base with other threads' (EXACT, z_base > NZ): always so
+// with 1 and 2 slices; with 4 an instantiation of its own, as the one whose slice numbers are constants
+// is 3% faster (four uneven scans: 36.4 against 37.6 ms).
+template <int NZ, int INTERP>
+constexpr bool kQBased = INTERP == LCT_INTERP_EXACT && NZ < 4;
+
+template <int NZ, int INTERP, int MINB, bool PART, bool RING, bool BASED = kQBased<NZ, INTERP>>
 __global__ void __launch_bounds__(kQTX* kQTY, MINB) bp_quad_kernel(const __grid_constant__ BpQuadArgs A) {
-  bp_quad_tile<NZ, INTERP, PART, RING>(A, blockIdx.x, blockIdx.y, blockIdx.z);
+  bp_quad_tile<NZ, INTERP, PART, RING, BASED>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // EXACT with every view's tile footprint staged in shared memory by TMA.  Per view pair the
@@ -933,7 +945,7 @@ __global__ void __launch_bounds__(kQTX* kQTY, MINB)
 // prefix[s] <= i < prefix[s + 1] and is tile i - prefix[s] of that scan's grid.  Each CTA takes
 // items from *counter (zero before the launch) until the list is exhausted; a scan's tiles run
 // exactly the arithmetic of its own launch.
-template <int NZ, int INTERP, int MINB>
+template <int NZ, int INTERP, int MINB, bool BASED = kQBased<NZ, INTERP>>
 __global__ void __launch_bounds__(kQTX* kQTY, MINB)
     bp_quad_worklist_kernel(const BpQuadArgs* __restrict__ args, const int* __restrict__ prefix,
                             int n_scans, int* __restrict__ counter) {
@@ -961,7 +973,7 @@ __global__ void __launch_bounds__(kQTX* kQTY, MINB)
     const int bx = local % sA.gx;
     const int by = (local / sA.gx) % sA.gy;
     const int bz = local / (sA.gx * sA.gy);
-    bp_quad_tile<NZ, INTERP, false, false>(sA, bx, by, bz);
+    bp_quad_tile<NZ, INTERP, false, false, BASED>(sA, bx, by, bz);
   }
 }
 
@@ -1027,6 +1039,7 @@ static int build_bp_quad_args(const lct_geom& g, const lct_img& ig, const BpLaun
   }
   nzt = L.nz_thread;
   if (nzt != 1 && nzt != 2 && nzt != 4 && nzt != 8 && nzt != 16) nzt = 8;
+  a.z_base = L.z_base;
   a.zchunks = (L.nz + nzt - 1) / nzt;
   a.gx = (ig.nx + kQTX - 1) / kQTX;
   a.gy = (ig.ny + kQTY - 1) / kQTY;
@@ -1051,6 +1064,13 @@ int launch_bp_par_quads(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
   int minb = L.minb;
   if (minb < 1 || minb > 4) minb = 4;  // measured best on B200 (4 CTAs x 256 threads per SM)
   const bool part = L.part != kBpWhole || L.view_lo > 0 || L.view_hi < (1 << 30);
+  if (!tex && nzt == 4 && a.z_base > nzt) {
+    if (a.qring > 0 && part) bp_quad_kernel<4, LCT_INTERP_EXACT, 4, true, true, true><<<grid, block, 0, s>>>(a);
+    else if (a.qring > 0) bp_quad_kernel<4, LCT_INTERP_EXACT, 4, false, true, true><<<grid, block, 0, s>>>(a);
+    else if (part) bp_quad_kernel<4, LCT_INTERP_EXACT, 4, true, false, true><<<grid, block, 0, s>>>(a);
+    else bp_quad_kernel<4, LCT_INTERP_EXACT, 4, false, false, true><<<grid, block, 0, s>>>(a);
+    return launch_status();
+  }
 #define LCT_BPQ(NZV, MB)                                                                          \
   do {                                                                                            \
     if (part && tex) bp_quad_kernel<NZV, LCT_INTERP_TEX8, MB, true, false><<<grid, block, 0, s>>>(a); \
@@ -1190,7 +1210,7 @@ int bp_quad_args_build(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
 }
 
 int launch_bp_quad_worklist(const void* d_args, const int* d_prefix, int n_scans, int* d_counter,
-                            int nz_thread, int interp, int minb, cudaStream_t s) {
+                            int nz_thread, bool based, int interp, int minb, cudaStream_t s) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1198,6 +1218,11 @@ int launch_bp_quad_worklist(const void* d_args, const int* d_prefix, int n_scans
   const BpQuadArgs* args = static_cast<const BpQuadArgs*>(d_args);
   dim3 grid(sms * minb), block(kQTX, kQTY);
   const bool tex = interp == LCT_INTERP_TEX8;
+  if (!tex && nz_thread == 4 && based) {
+    grid.x = sms * 4;
+    bp_quad_worklist_kernel<4, LCT_INTERP_EXACT, 4, true><<<grid, block, 0, s>>>(args, d_prefix, n_scans, d_counter);
+    return launch_status();
+  }
 #define LCT_BPW(NZV, MB)                                                                        \
   do {                                                                                          \
     if (tex)                                                                                    \

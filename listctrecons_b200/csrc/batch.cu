@@ -9,6 +9,7 @@
 // across the SMs; each tile runs the arithmetic of its scan's own launch, so a scan's volume is
 // bit-identical to lct_recon_run with the same options.
 #include <map>
+#include <tuple>
 #include <new>
 #include <utility>
 #include <vector>
@@ -19,6 +20,7 @@
 // thread, CTAs per SM) run in one persistent launch.
 struct BpGroup {
   int nz = 8, minb = 4, n = 0;
+  bool based = false;        // threads of fewer slices than share a base (BpLaunch::z_base)
   void* d_args = nullptr;    // per-scan backprojection arguments
   int* d_prefix = nullptr;   // tile prefix sums, n + 1
   int* d_counter = nullptr;  // work-list cursor, zeroed by the graph before each launch
@@ -62,7 +64,7 @@ static int batch_stage(lct_batch* b, int stage, cudaStream_t s) {
   if (stage == 2 && b->worklist) {
     for (auto& gr : b->groups) {
       if ((st = cuda_status(cudaMemsetAsync(gr.d_counter, 0, sizeof(int), s)))) return st;
-      if ((st = launch_bp_quad_worklist(gr.d_args, gr.d_prefix, gr.n, gr.d_counter, gr.nz,
+      if ((st = launch_bp_quad_worklist(gr.d_args, gr.d_prefix, gr.n, gr.d_counter, gr.nz, gr.based,
                                         b->interp, gr.minb, s)))
         return st;
     }
@@ -130,20 +132,18 @@ LCT_API int lct_batch_create(const lct_plan* const* plans, int n, const lct_reco
     // each scan keeps the thread shape its own run would use (the slices-per-thread heuristic,
     // or the requested / autotuned shape); scans sharing a shape share a work list
     const int asz = bp_quad_args_size();
-    std::map<std::pair<int, int>, std::vector<int>> by_shape;
+    std::map<std::tuple<int, int, bool>, std::vector<int>> by_shape;
     for (int i = 0; i < n; ++i) {
       lct_recon* r = b->recs[i];
       BpLaunch L;
       recon_bp_launch(r, 0, r->info.n_blocks_run, r->d_img, L);
-      r->o.bp_nz = L.nz_thread;  // the scan's own launches use the same shape
       r->o.bp_minb = L.minb > 0 ? L.minb : 4;
-      by_shape[{r->o.bp_nz, r->o.bp_minb}].push_back(i);
+      by_shape[{L.nz_thread, r->o.bp_minb, L.z_base > L.nz_thread}].push_back(i);
     }
     for (auto& kv : by_shape) {
       if (st) break;
       BpGroup gr;
-      gr.nz = kv.first.first;
-      gr.minb = kv.first.second;
+      std::tie(gr.nz, gr.minb, gr.based) = kv.first;
       gr.n = (int)kv.second.size();
       std::vector<char> args((size_t)asz * gr.n);
       std::vector<int> prefix(gr.n + 1, 0);

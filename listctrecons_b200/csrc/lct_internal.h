@@ -68,6 +68,7 @@ struct BpLaunch {
   int slab_z0[kBpMaxSlabs];
   int interp, addr;
   int nz_thread;       // slices per thread (quads: 1, 2, 4, 8, 16; else 8, 16, 32; 0 = choose)
+  int z_base = 0;      // quad kernel, EXACT: slices that share one base of the row coordinate (bp_z_base)
   int minb = 0;        // quad kernel: resident CTAs per SM the register budget targets (0 = 4)
   // quad kernel only: a part of the slabs' views, [view_lo, view_hi) in slab-local indices,
   // carried between parts as raw FP32 sums in img (part kBpWhole / First / Middle / Last); the
@@ -96,6 +97,12 @@ LCT_HD inline long long quad_view_elems(int ns, int nt) { return (long long)(nt 
 // interp: TEX8 quads hold their row differences (dy, dxy) times 2^-8.
 int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, int interp,
                      float4* quads, cudaStream_t s, long long vbase = 0, long long ring = 0);
+// Slices whose EXACT row coordinates are steps from one base (the first of them): 8, or 4 where few are
+// active together, however few a thread takes -- a slice's rounding then depends on neither the image's
+// size nor the split.
+inline int bp_z_base(const lct_geom& g, const lct_img& ig) {
+  return 0.5 * (double)g.pitch / (double)ig.dz < 6.0 ? 4 : 8;
+}
 // Slices per thread of the quad kernel by default: 8, which shares a view's terms among most slices;
 // 4 when a view stays active for fewer than 6 slices ((feed / 2) / dz); and fewer where one slab's
 // 16 x 16 tiles would leave most of the chip's 592 CTA slots empty and the views' latency in series
@@ -108,7 +115,7 @@ inline int bp_nz_default(const lct_geom& g, const lct_img& ig) {
   if (tiles * 16 < 200) return 1;
   if (tiles * 8 < 500) return 2;
   if (tiles * 4 < 500) return 4;
-  return 0.5 * (double)g.pitch / (double)ig.dz < 6.0 ? 4 : 8;
+  return bp_z_base(g, ig);
 }
 // Backprojection from quad-layout views (full windows only; L.proj is ignored, L.quads used).
 int launch_bp_par_quads(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
@@ -155,7 +162,7 @@ int bp_quad_args_size();
 int bp_quad_args_build(const lct_geom& g, const lct_img& ig, const BpLaunch& L,
                        const float4* quads, void* out, int* tiles);
 int launch_bp_quad_worklist(const void* d_args, const int* d_prefix, int n_scans, int* d_counter,
-                            int nz_thread, int interp, int minb, cudaStream_t s);
+                            int nz_thread, bool based, int interp, int minb, cudaStream_t s);
 
 // Rebinning, scan mode: each global parallel view g in [g0, g0 + nviews) is interpolated
 // from the fan buffer whose view 0 is global fan view `fan_first`, with the view shift of

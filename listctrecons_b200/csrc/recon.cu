@@ -400,6 +400,7 @@ static int run_blocks(lct_recon* r, const float* d_fan, float* d_img, cudaStream
       L.interp = r->o.interp;
       L.addr = addr;
       L.nz_thread = bp_nz;
+      L.z_base = pick_bp_z_base(g, ig, r->o.bp_nz);
       L.minb = r->o.bp_minb;
       if (r->quads) {
         if ((st = recon_pack(r, r->d_par, g.n_angle, 0, addr, s))) return st;
@@ -475,6 +476,7 @@ void recon_bp_launch(const lct_recon* r, int b0, int b1, float* d_img, BpLaunch&
   L.interp = r->o.interp;
   L.addr = block_addr(r, b0);
   L.nz_thread = pick_bp_nz(g, r->info.ig, r->o.bp_nz);
+  L.z_base = pick_bp_z_base(g, r->info.ig, r->o.bp_nz);
   L.minb = r->o.bp_minb;
   // betas are indexed by the same slab offset: shift the base by g_first
   L.betas = r->d_betas + r->g_first;

@@ -108,6 +108,10 @@ namespace lct {
 inline int pick_bp_nz(const lct_geom& g, const lct_img& ig, int requested) {
   return requested == 4 || requested == 8 || requested == 16 ? requested : bp_nz_default(g, ig);
 }
+// ... and the slices per base of their row coordinates: a requested thread shape has its own
+inline int pick_bp_z_base(const lct_geom& g, const lct_img& ig, int requested) {
+  return requested == 4 || requested == 8 || requested == 16 ? requested : bp_z_base(g, ig);
+}
 // kernels one filter call launches
 inline int filter_launches(int mode) { return mode == LCT_FILTER_FP32 ? 1 : 2; }
 // addressing of block b (LEGACY: clamped first block, border afterwards)
