@@ -267,7 +267,7 @@ void lct_plan_destroy(lct_plan* plan);
             fetch, CUDA/Backprojector.cu:85-86; QUADS otherwise);
    QUADS_TMA (EXACT only) the quads, with each view's tile footprint staged in shared memory by
             TMA before the samples read it (the same values: bit-identical to QUADS);
-   AUTO     QUADS (on B200 the quad kernel's TEX8 path outran the texture fetch: 121 against
+   AUTO     QUADS (on B200 the quad kernel's TEX8 path outruns the texture fetch: 89 against
             137 ms on a 512^2 x 256 volume of 736 x 64 views). */
 #define LCT_BP_SAMPLER_AUTO 0
 #define LCT_BP_SAMPLER_QUADS 1
