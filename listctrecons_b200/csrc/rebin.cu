@@ -289,11 +289,13 @@ __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* _
   lin_axis<LCT_INTERP_EXACT>(pidx + 0.5, i, wx);
   lin_axis<LCT_INTERP_EXACT>(qidx + 0.5, j, wy);
   const double fk = floor(shift);
-  const float c = (float)(shift - fk);
-  const float w[4] = {(1.0f - wx) * (1.0f - wy), wx * (1.0f - wy), (1.0f - wx) * wy, wx * wy};
-  // texels that count: on the detector (or clamped to it), weight not zero
+  float c = (float)(shift - fk);
+  float w[4] = {(1.0f - wx) * (1.0f - wy), wx * (1.0f - wy), (1.0f - wx) * wy, wx * wy};
+  // texels that count: on the detector (or clamped to it), weight not zero.  The others' weights are
+  // zero, so that a column past the source's distance, whose coordinates and weights are NaN, reads the
+  // border's 0 as any other column outside the detector does
   int off[4];
-  bool ok[4];
+  bool ok[4], any = false;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     int ii = i + (k & 1), jj = j + (k >> 1);
@@ -305,7 +307,10 @@ __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* _
       ok[k] = ok[k] && ii >= 0 && ii < a.ns && jj >= 0 && jj < a.nt;
     }
     off[k] = ok[k] ? jj * a.ns + ii : 0;
+    if (!ok[k]) w[k] = 0.0f;
+    any = any || ok[k];
   }
+  if (!any) c = 0.0f;
   const long long plane = (long long)a.nt * a.ns;
   auto sample = [&](long long v) {
     bool in = true;
