@@ -28,6 +28,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "footprint.cuh"
 #include "fp32_pair.cuh"
 #include "lct_internal.h"
 #include "tc_ptx.cuh"
@@ -171,7 +172,8 @@ __device__ __forceinline__ unsigned long long quad_col(unsigned long long vbias,
 // Prefetch boxes of one tile in view ia (b1) and its conjugate (b2): {row_lo, row_hi, col_lo,
 // col_hi} in quad rows/columns, from the tile's four corners at its first and last slice, widened
 // by one row and column (the interior can bulge slightly past the corners) and clamped to the
-// view's quads.  Only the L1 prefetch reads them.
+// view's quads.  The footprint loads read them, so they lie inside the view whatever the corners are:
+// a corner at the source (a volume that reaches past the source's circle) projects to infinity.
 __device__ __forceinline__ void prefetch_boxes(const BpQuadArgs& A, float c1, float s1, float c2,
                                                float s2, int ia, float x0, float x1, float y0,
                                                float y1, float zc0, float zcl, int4& b1, int4& b2) {
@@ -197,19 +199,13 @@ __device__ __forceinline__ void prefetch_boxes(const BpQuadArgs& A, float c1, fl
       b1.x = min(b1.x, r1); b1.y = max(b1.y, r1);
       b2.x = min(b2.x, r2); b2.y = max(b2.y, r2);
     }
-    const int q1 = __float2int_rd(fmaf(theta, A.dso_over_ds, A.ws)) + 2;
-    const int q2 = __float2int_rd(fmaf(-theta, A.dso_over_ds, A.ws)) + 2;
+    const int q1 = __float2int_rd(fmaf(theta, A.dso_over_ds, A.ws));
+    const int q2 = __float2int_rd(fmaf(-theta, A.dso_over_ds, A.ws));
     b1.z = min(b1.z, q1); b1.w = max(b1.w, q1);
     b2.z = min(b2.z, q2); b2.w = max(b2.w, q2);
   }
-  auto fit = [&](int4& b) {
-    b.x = min(max(b.x - 1, 0), A.nt + 2);
-    b.y = min(max(b.y + 1, b.x), A.nt + 2);
-    b.z = min(max(b.z - 1, 0), A.ns + 2);
-    b.w = min(max(b.w + 1, b.z), A.ns + 2);
-  };
-  fit(b1);
-  fit(b2);
+  b1 = box_in_view(b1, A.ns, A.nt);
+  b2 = box_in_view(b2, A.ns, A.nt);
 }
 
 // asin on |x| <= 0.5 as x + x^3 P(x^2), P of degree 4 fitted by least squares (weighted for the
