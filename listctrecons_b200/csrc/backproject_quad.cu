@@ -448,18 +448,18 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
         if (add) acc[j] = sum;
       };
       constexpr int kQGroup = kQGroupOf<NZ>;
-      // qhat is monotone in j (a monotone rounding of a linear function), so the first and last
-      // slices of the groups that run bound every |qhat|: when both are inside for both views in
-      // every lane of the warp, every out test is false and the tests, selects and clamps are
-      // skipped with no change to any result.  The row coordinate (equal to qhat + wt within a
-      // few ulps, far below half a row) then lies inside the quad rows when rows_inside_ok.  A
-      // NaN fails the test.  (EXACT, 512^2 x 256 from 736 x 64 views: 69.4 ms with scalar code and
-      // no inside path on partial windows, 64.3 ms so.)
+      // when the first and last slices of the groups that run are inside for both views in every
+      // lane of the warp (rows_inside), every out test is false and the tests, selects and clamps are
+      // skipped with no change to any result; the row coordinate (equal to qhat + wt within a
+      // few ulps, far below half a row) then lies inside the quad rows when rows_inside_ok.
+      // (EXACT, 512^2 x 256 from 736 x 64 views: 69.4 ms with scalar code and no inside path on
+      // partial windows, 64.3 ms so.)
       const float jf = slice_j(jlo & ~(kQGroup - 1));
       const float jl = slice_j(((jhi + kQGroup - 1) & ~(kQGroup - 1)) - 1);
-      const bool inside = A.rows_inside_ok && fabsf(fmaf(jf, K.x, M.x)) <= wt &&
-                          fabsf(fmaf(jl, K.x, M.x)) <= wt && fabsf(fmaf(jf, K.y, M.y)) <= wt &&
-                          fabsf(fmaf(jl, K.y, M.y)) <= wt;
+      // (TEX8 takes its row coordinate from qhat itself)
+      constexpr bool kSingle = kQGroup == 1 && INTERP == LCT_INTERP_EXACT;
+      const bool inside = A.rows_inside_ok && rows_inside<kSingle>(jf, jl, K.x, M.x, wt) &&
+                          rows_inside<kSingle>(jf, jl, K.y, M.y, wt);
       if (__all_sync(0xffffffffu, inside)) {
         if (jlo == 0 && jhi == NZ) {  // straight code: every load of the chunk may be in flight
 #pragma unroll
