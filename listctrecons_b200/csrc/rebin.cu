@@ -298,11 +298,11 @@ __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* _
   bool ok[4], any = false;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    int ii = i + (k & 1), jj = j + (k >> 1);
+    int ii = (k & 1) ? next_texel(i) : i, jj = (k >> 1) ? next_texel(j) : j;
     ok[k] = w[k] != 0.0f;
     if (ADDR == LCT_ADDR_CLAMP) {
-      ii = min(max(ii, 0), a.ns - 1);
-      jj = min(max(jj, 0), a.nt - 1);
+      ii = (k & 1) ? next_clamped(i, a.ns) : min(max(i, 0), a.ns - 1);
+      jj = (k >> 1) ? next_clamped(j, a.nt) : min(max(j, 0), a.nt - 1);
     } else {
       ok[k] = ok[k] && ii >= 0 && ii < a.ns && jj >= 0 && jj < a.nt;
     }

@@ -29,6 +29,15 @@ __host__ __device__ __forceinline__ void tex_bilinear_weights(float a, float b, 
   w00 = (1.0f - a - b) + w11;
 }
 
+// Texel i + 1 of n with clamped addressing, in [0, n - 1].  i may be either end of int (a coordinate
+// beyond its range converts to them), so the step comes after the clamp: a sum that overflows first is
+// undefined, and compiled into a clamp of i it read far outside the views.
+__host__ __device__ __forceinline__ int next_clamped(int i, int n) {
+  return (i < -1 ? -1 : (i > n - 2 ? n - 2 : i)) + 1;
+}
+// and without clamping (the caller tests it against n)
+__host__ __device__ __forceinline__ int next_texel(int i) { return (int)((unsigned)i + 1u); }
+
 template <int INTERP>
 __device__ __forceinline__ void lin_axis(float coord, int& i, float& w) {
   // coord is a texture coordinate (texel centres at i + 0.5); coord - 0.5f is exact for
