@@ -270,13 +270,14 @@ __global__ void __launch_bounds__(256) rebin_null_kernel(const float* __restrict
 // output ran 1.63 ms).
 constexpr int kPiViews = 64, kPiThreads = 128;
 
-// grid (ceil(ns / 128), nt, ceil(n_angle / kPiViews)), block 128
+// grid (ceil(ns / 128), nt, walks of kPiViews views from walk0 on), block 128
 template <int ADDR>
 __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* __restrict__ fan,
-                                                                  float* __restrict__ par, RebinArgs a) {
+                                                                  float* __restrict__ par, RebinArgs a,
+                                                                  int walk0) {
   const int is = blockIdx.x * kPiThreads + threadIdx.x, it = blockIdx.y;
   if (is >= a.ns) return;
-  const int ia0 = blockIdx.z * kPiViews, ia1 = min(a.n_angle, ia0 + kPiViews);
+  const int ia0 = (walk0 + blockIdx.z) * kPiViews, ia1 = ia0 + min(a.n_angle - ia0, kPiViews);
   const double s = ((double)is - a.ws) * (double)a.ds;
   const double gamma = asin(s / a.dso);
   const double pidx = gamma * a.dso / a.ds + a.ws;
@@ -341,10 +342,11 @@ __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* _
 // (PI is a double literal there).  The weight is the same for every view: a thread evaluates it
 // once and scales kPiViews views.  Bound: HBM (1,833 views of 736 x 64: 0.14 ms; 0.45 ms with the
 // weight evaluated per output).
-__global__ void __launch_bounds__(kPiThreads) weight_pi_ori_kernel(float* __restrict__ par, RebinArgs a) {
+__global__ void __launch_bounds__(kPiThreads) weight_pi_ori_kernel(float* __restrict__ par, RebinArgs a,
+                                                                   int walk0) {
   const int is = blockIdx.x * kPiThreads + threadIdx.x, it = blockIdx.y;
   if (is >= a.ns) return;
-  const int ia0 = blockIdx.z * kPiViews, ia1 = min(a.n_angle, ia0 + kPiViews);
+  const int ia0 = (walk0 + blockIdx.z) * kPiViews, views = min(a.n_angle - ia0, kPiViews);
   float s = (is - a.ws) * a.ds;
   float t = (it - a.wt) * a.pitch / (float)(2 * a.nt);
   float gamma = asinf(s / a.dso);
@@ -353,13 +355,13 @@ __global__ void __launch_bounds__(kPiThreads) weight_pi_ori_kernel(float* __rest
   float weight = sqrtf(temp) / sqrtf(temp + temp2 * temp2);
   const long long plane = (long long)a.nt * a.ns;
   float* p = par + ((long long)ia0 * a.nt + it) * a.ns + is;
-  for (int ia = ia0; ia < ia1; ia += 8, p += 8 * plane) {  // eight loads in flight
+  for (int v = 0; v < views; v += 8, p += 8 * plane) {  // eight loads in flight
     float x[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = ia + k < ia1 ? p[k * plane] : 0.0f;
+    for (int k = 0; k < 8; ++k) x[k] = v + k < views ? p[k * plane] : 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      if (ia + k < ia1) p[k * plane] = x[k] * weight;
+      if (v + k < views) p[k * plane] = x[k] * weight;
   }
 }
 
@@ -405,9 +407,16 @@ int launch_rebin_fan2par_scan(const lct_geom& g, const float* d_fan, long long f
 
 using namespace lct;
 
-// grid of the kernels that walk kPiViews views per (row, column)
-static dim3 pi_grid(const lct_geom& g) {
-  return dim3((g.ns + kPiThreads - 1) / kPiThreads, g.nt, (g.n_angle + kPiViews - 1) / kPiViews);
+// The kernels that walk kPiViews views per (row, column): one launch for every 65,535 walks (grid.z),
+// launch(grid, first walk).
+template <class Launch>
+static int for_pi_walks(const lct_geom& g, Launch launch) {
+  const int walks = (g.n_angle - 1) / kPiViews + 1;
+  for (int w = 0; w < walks; w += 65535) {
+    launch(dim3((g.ns + kPiThreads - 1) / kPiThreads, g.nt, walks - w < 65535 ? walks - w : 65535), w);
+    if (const int st = launch_status()) return st;
+  }
+  return LCT_OK;
 }
 
 static int check_modes(int interp, int addr) {
@@ -516,7 +525,6 @@ LCT_API int lct_rebin_pi_ori(const lct_geom* g, const float* d_fan, float* d_par
   if ((st = check_modes(interp, addr))) return st;
   if (!d_fan || !d_par || g->nt < 2) return LCT_ERR_ARG;
   RebinArgs a = rebin_args(*g);
-  const dim3 grid = pi_grid(*g);
   cudaStream_t s = (cudaStream_t)stream;
   bool tex = interp == LCT_INTERP_TEX8, clamp = addr == LCT_ADDR_CLAMP;
   if (tex) {
@@ -529,11 +537,12 @@ LCT_API int lct_rebin_pi_ori(const lct_geom* g, const float* d_fan, float* d_par
     view_texture_destroy(t);
     return st ? st : st2;
   }
-  if (clamp)
-    rebin_pi_ori_kernel<LCT_ADDR_CLAMP><<<grid, kPiThreads, 0, s>>>(d_fan, d_par, a);
-  else
-    rebin_pi_ori_kernel<LCT_ADDR_BORDER><<<grid, kPiThreads, 0, s>>>(d_fan, d_par, a);
-  return launch_status();
+  return for_pi_walks(*g, [&](dim3 grid, int walk0) {
+    if (clamp)
+      rebin_pi_ori_kernel<LCT_ADDR_CLAMP><<<grid, kPiThreads, 0, s>>>(d_fan, d_par, a, walk0);
+    else
+      rebin_pi_ori_kernel<LCT_ADDR_BORDER><<<grid, kPiThreads, 0, s>>>(d_fan, d_par, a, walk0);
+  });
 }
 
 LCT_API int lct_weight_pi_ori(const lct_geom* g, float* d_par, lct_stream stream) {
@@ -541,6 +550,7 @@ LCT_API int lct_weight_pi_ori(const lct_geom* g, float* d_par, lct_stream stream
   if (st) return st;
   if (!d_par) return LCT_ERR_ARG;
   RebinArgs a = rebin_args(*g);
-  weight_pi_ori_kernel<<<pi_grid(*g), kPiThreads, 0, (cudaStream_t)stream>>>(d_par, a);
-  return launch_status();
+  return for_pi_walks(*g, [&](dim3 grid, int walk0) {
+    weight_pi_ori_kernel<<<grid, kPiThreads, 0, (cudaStream_t)stream>>>(d_par, a, walk0);
+  });
 }
