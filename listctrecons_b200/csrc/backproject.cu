@@ -63,14 +63,15 @@ __device__ __forceinline__ ColSetup col_setup(float p_idx, int ns) {
   int i;
   lin_axis<INTERP>(p_idx + 0.5f, i, c.a);
   if (ADDR == LCT_ADDR_CLAMP) {
+    i = below_max(i);
     c.c0 = min(max(i, 0), ns - 1);
-    c.c1 = next_clamped(i, ns);
+    c.c1 = min(max(i + 1, 0), ns - 1);
     c.ok0 = c.ok1 = true;
   } else {
     c.c0 = i;
-    c.c1 = next_texel(i);
+    c.c1 = i + 1;
     c.ok0 = (unsigned)i < (unsigned)ns;
-    c.ok1 = (unsigned)c.c1 < (unsigned)ns;
+    c.ok1 = (unsigned)(i + 1) < (unsigned)ns;
   }
   return c;
 }
@@ -96,11 +97,12 @@ __device__ __forceinline__ float sample_rows(const float* __restrict__ view, int
   int j;
   float b;
   lin_axis<INTERP>(q_idx + 0.5f, j, b);
+  if (ADDR == LCT_ADDR_CLAMP) j = below_max(j);
   int r0 = j, r1 = next_texel(j);
   bool rk0 = true, rk1 = true;
   if (ADDR == LCT_ADDR_CLAMP) {
     r0 = min(max(r0, 0), nt - 1);
-    r1 = next_clamped(j, nt);
+    r1 = min(max(r1, 0), nt - 1);
   } else {
     rk0 = (unsigned)r0 < (unsigned)nt;
     rk1 = (unsigned)r1 < (unsigned)nt;

@@ -289,29 +289,31 @@ __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* _
   float wx, wy;
   lin_axis<LCT_INTERP_EXACT>(pidx + 0.5, i, wx);
   lin_axis<LCT_INTERP_EXACT>(qidx + 0.5, j, wy);
+  i = below_max(i);  // near s = dso the row coordinate is huge
+  j = below_max(j);
   const double fk = floor(shift);
   float c = (float)(shift - fk);
   float w[4] = {(1.0f - wx) * (1.0f - wy), wx * (1.0f - wy), (1.0f - wx) * wy, wx * wy};
   // texels that count: on the detector (or clamped to it), weight not zero.  The others' weights are
   // zero, so that a column past the source's distance, whose coordinates and weights are NaN, reads the
   // border's 0 as any other column outside the detector does
-  int off[4];
+  unsigned off[4];
   bool ok[4], any = false;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    int ii = (k & 1) ? next_texel(i) : i, jj = (k >> 1) ? next_texel(j) : j;
+    int ii = i + (k & 1), jj = j + (k >> 1);
     ok[k] = w[k] != 0.0f;
     if (ADDR == LCT_ADDR_CLAMP) {
-      ii = (k & 1) ? next_clamped(i, a.ns) : min(max(i, 0), a.ns - 1);
-      jj = (k >> 1) ? next_clamped(j, a.nt) : min(max(j, 0), a.nt - 1);
+      ii = min(max(ii, 0), a.ns - 1);
+      jj = min(max(jj, 0), a.nt - 1);
     } else {
       ok[k] = ok[k] && ii >= 0 && ii < a.ns && jj >= 0 && jj < a.nt;
     }
-    off[k] = ok[k] ? jj * a.ns + ii : 0;
-    if (!ok[k]) w[k] = 0.0f;
+    off[k] = ok[k] ? (unsigned)jj * (unsigned)a.ns + (unsigned)ii : 0u;
+    if (ADDR == LCT_ADDR_BORDER && !ok[k]) w[k] = 0.0f;
     any = any || ok[k];
   }
-  if (!any) c = 0.0f;
+  if (ADDR == LCT_ADDR_BORDER && !any) c = 0.0f;
   const long long plane = (long long)a.nt * a.ns;
   auto sample = [&](long long v) {
     bool in = true;
@@ -331,7 +333,7 @@ __global__ void __launch_bounds__(kPiThreads) rebin_pi_ori_kernel(const float* _
   float* o = par + ((long long)ia0 * a.nt + it) * a.ns + is;
   float lo = sample(k0 + ia0);
 #pragma unroll 4
-  for (int ia = ia0; ia < ia1; ++ia, o += plane) {
+  for (int ia = ia0, n = ia1 - ia0; n > 0; --n, ++ia, o += plane) {
     const float hi = sample(k0 + ia + 1);
     *o = c == 0.0f ? lo : (c == 1.0f ? hi : fmaf(c, hi, (1.0f - c) * lo));
     lo = hi;

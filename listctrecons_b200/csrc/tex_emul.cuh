@@ -29,13 +29,11 @@ __host__ __device__ __forceinline__ void tex_bilinear_weights(float a, float b, 
   w00 = (1.0f - a - b) + w11;
 }
 
-// Texel i + 1 of n with clamped addressing, in [0, n - 1].  i may be either end of int (a coordinate
-// beyond its range converts to them), so the step comes after the clamp: a sum that overflows first is
-// undefined, and compiled into a clamp of i it read far outside the views.
-__host__ __device__ __forceinline__ int next_clamped(int i, int n) {
-  return (i < -1 ? -1 : (i > n - 2 ? n - 2 : i)) + 1;
-}
-// and without clamping (the caller tests it against n)
+// A coordinate beyond the range of int converts to one of its ends, and the texel after INT_MAX is a sum that
+// overflows: undefined, and with the clamp folded onto i it read far outside the views.  Clamped
+// addressing takes such an origin one texel down first (both clamp to the last texel); border addressing
+// steps in unsigned arithmetic, and the caller tests the result.
+__host__ __device__ __forceinline__ int below_max(int i) { return i < 0x7ffffffe ? i : 0x7ffffffe; }
 __host__ __device__ __forceinline__ int next_texel(int i) { return (int)((unsigned)i + 1u); }
 
 template <int INTERP>

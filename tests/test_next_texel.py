@@ -20,8 +20,9 @@ int main() {
   for (int n : {1, 2, 8})
     for (int i : v) {
       const long long want = std::min(std::max((long long)i + 1, 0LL), (long long)n - 1);
-      if (lct::next_clamped(i, n) != want) return 1;
-      if ((unsigned)lct::next_texel(i) != (unsigned)((long long)i + 1)) return 2;
+      if (std::min(std::max(lct::below_max(i) + 1, 0), n - 1) != want) return 1;
+      if (std::min(std::max(lct::below_max(i), 0), n - 1) != std::min(std::max(i, 0), n - 1)) return 2;
+      if ((unsigned)lct::next_texel(i) != (unsigned)((long long)i + 1)) return 3;
     }
   return 0;
 }
