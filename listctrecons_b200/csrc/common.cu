@@ -1,7 +1,11 @@
 // Status codes, CUDA error bookkeeping, the device status word and geometry checks.
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 #include <cmath>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "lct_internal.h"
 
@@ -19,57 +23,80 @@ int cuda_status(cudaError_t e) {
 
 int launch_status() { return cuda_status(cudaGetLastError()); }
 
+// cudaDeviceReset destroys a device's context with all that lives in it -- pools, module addresses,
+// kernel attributes -- and the next call starts another, so what the library keeps per device is kept
+// for the context's id.
+unsigned long long context_id() {
+  static std::once_flag once;
+  static PFN_cuCtxGetId_v12000 get = nullptr;
+  std::call_once(once, [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get = reinterpret_cast<PFN_cuCtxGetId_v12000>(p);
+  });
+  unsigned long long id = 0;
+  if (!get || get(nullptr, &id) == CUDA_SUCCESS) return id;
+  cudaFree(nullptr);  // no context yet: starts the device's
+  return get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 // One word per device, kept in the module's own global memory (no allocation).
 static __device__ int g_device_status = 0;
 
 int* device_status_ptr() {
   static std::mutex mu;
   static int* ptrs[64] = {nullptr};
+  static unsigned long long ctx[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  const unsigned long long id = context_id();
   std::lock_guard<std::mutex> lock(mu);
-  if (!ptrs[dev]) {
+  if (!ptrs[dev] || ctx[dev] != id) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_device_status) != cudaSuccess) return nullptr;
     ptrs[dev] = static_cast<int*>(p);
+    ctx[dev] = id;
   }
   return ptrs[dev];
 }
 
 // Scratch of the stage entry points.  The default pool unmaps what is freed at every
 // synchronisation, so a call that takes a gigabyte of scratch after each one paid for mapping it
-// again (a 3,600-view block of 735 x 31: 15-160 ms a call for a 5 ms kernel).  One pool per device
-// keeps up to kScratchKeep bytes (1/32 of the device's memory if that is less) mapped between calls.
+// again (a 3,600-view block of 735 x 31: 15-160 ms a call for a 5 ms kernel).  One pool per device and
+// context keeps up to kScratchKeep bytes (1/32 of the device's memory if that is less) mapped between calls.
 // The pool is stream-ordered and thread-safe like the default one; what exceeds the bound goes back
 // at the next synchronisation, the rest when the driver needs it for another allocation of the
 // process or lct_scratch_release asks.
 constexpr size_t kScratchKeep = 4ull << 30;
 static std::mutex g_scratch_mu;
-static cudaMemPool_t g_scratch_pool[64] = {nullptr};
+// by device and context; never destroyed, as calls may outlive static objects
+static auto& g_scratch_pool = *new std::map<std::pair<int, unsigned long long>, cudaMemPool_t>;
 
 static cudaMemPool_t scratch_pool() {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  const std::pair<int, unsigned long long> ctx{dev, context_id()};
   std::lock_guard<std::mutex> lock(g_scratch_mu);
-  if (!g_scratch_pool[dev]) {
-    cudaMemPoolProps p = {};
-    p.allocType = cudaMemAllocationTypePinned;
-    p.handleTypes = cudaMemHandleTypeNone;
-    p.location.type = cudaMemLocationTypeDevice;
-    p.location.id = dev;
-    cudaMemPool_t pool = nullptr;
-    size_t free_b = 0, total = 0;
-    uint64_t keep = kScratchKeep;
-    if (cudaMemGetInfo(&free_b, &total) == cudaSuccess) keep = std::min<uint64_t>(keep, total / 32);
-    if (cudaMemPoolCreate(&pool, &p) != cudaSuccess) {
-      cudaGetLastError();  // no pools on this device: the default one
-      return nullptr;
-    }
-    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
-      cudaGetLastError();
-    g_scratch_pool[dev] = pool;
+  const auto it = g_scratch_pool.find(ctx);
+  if (it != g_scratch_pool.end()) return it->second;
+  cudaMemPoolProps p = {};
+  p.allocType = cudaMemAllocationTypePinned;
+  p.handleTypes = cudaMemHandleTypeNone;
+  p.location.type = cudaMemLocationTypeDevice;
+  p.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  size_t free_b = 0, total = 0;
+  uint64_t keep = kScratchKeep;
+  if (cudaMemGetInfo(&free_b, &total) == cudaSuccess) keep = std::min<uint64_t>(keep, total / 32);
+  if (cudaMemPoolCreate(&pool, &p) != cudaSuccess) {
+    cudaGetLastError();  // no pools on this device: the default one
+    return nullptr;
   }
-  return g_scratch_pool[dev];
+  if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
+    cudaGetLastError();
+  return g_scratch_pool[ctx] = pool;
 }
 
 int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
@@ -140,9 +167,10 @@ LCT_API int lct_scratch_release(void) {
   int dev = 0;
   int st = cuda_status(cudaGetDevice(&dev));
   if (st) return st;
+  const std::pair<int, unsigned long long> ctx{dev, context_id()};
   std::lock_guard<std::mutex> lock(g_scratch_mu);
-  if (dev < 0 || dev >= 64 || !g_scratch_pool[dev]) return LCT_OK;
-  return cuda_status(cudaMemPoolTrimTo(g_scratch_pool[dev], 0));
+  const auto it = g_scratch_pool.find(ctx);
+  return it == g_scratch_pool.end() ? LCT_OK : cuda_status(cudaMemPoolTrimTo(it->second, 0));
 }
 
 LCT_API int lct_version(void) { return 100; }

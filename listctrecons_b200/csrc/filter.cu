@@ -219,18 +219,23 @@ int launch_filter_rows(int ns, const float* d_h, float* d_rows, long long nrows,
   if (mode == LCT_FILTER_BF16X3 || mode == LCT_FILTER_BF16X6)
     return launch_filter_tc(ns, d_h, d_rows, nrows, mode, s);
   static std::mutex mu;
-  static int sms_of[64] = {0};  // 0: attribute not set yet on that device
+  static int sms_of[64] = {0};                 // 0: attribute not set yet on that device
+  static unsigned long long ctx_of[64] = {0};  // and in that context
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
+  const unsigned long long ctx = context_id();
   {
     std::lock_guard<std::mutex> lock(mu);  // host threads may share a device
-    if (dev >= 64 || !sms_of[dev]) {
+    if (dev >= 64 || !sms_of[dev] || ctx_of[dev] != ctx) {
       int st = cuda_status(cudaFuncSetAttribute(filter_fp32_kernel,
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 200 * 1024));
       if (!st) st = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (st) return st;
-      if (dev < 64) sms_of[dev] = sms;
+      if (dev < 64) {
+        sms_of[dev] = sms;
+        ctx_of[dev] = ctx;
+      }
     } else {
       sms = sms_of[dev];
     }

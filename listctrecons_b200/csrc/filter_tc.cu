@@ -396,15 +396,20 @@ static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cu
   cudaGetDevice(&dev);
   {
     static std::mutex mu;  // host threads may share a device
-    static int sms_of[64] = {0};  // 0: attribute not set yet on that device
+    static int sms_of[64] = {0};                 // 0: attribute not set yet on that device
+    static unsigned long long ctx_of[64] = {0};  // and in that context
+    const unsigned long long ctx = context_id();
     std::lock_guard<std::mutex> lock(mu);
-    if (dev >= 64 || !sms_of[dev]) {
+    if (dev >= 64 || !sms_of[dev] || ctx_of[dev] != ctx) {
       if ((st = cuda_status(cudaFuncSetAttribute(filter_tc_kernel<P>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  kTcSmem))))
         return st;
       if ((st = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))) return st;
-      if (dev < 64) sms_of[dev] = sms;
+      if (dev < 64) {
+        sms_of[dev] = sms;
+        ctx_of[dev] = ctx;
+      }
     } else {
       sms = sms_of[dev];
     }

@@ -28,6 +28,8 @@ void set_cuda_error(cudaError_t e);
 int cuda_status(cudaError_t e);  // LCT_OK or LCT_ERR_CUDA (records e)
 int launch_status();             // cudaGetLastError() -> status
 
+unsigned long long context_id();  // of the current device's context: another one after a device reset
+
 // Stream-ordered scratch of a stage entry point (common.cu), from a bounded pool of the library's own.
 int scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 int scratch_free(void* p, cudaStream_t s);
