@@ -165,6 +165,11 @@ int lct_backproject_par(const lct_geom* g, const lct_img* ig, const float* d_bet
    full rotation, which the reference planner's blocks always have -- else 0 (the general
    kernel, which needs no scratch). */
 int lct_backproject_par_quad_path(const lct_geom* g, const lct_img* ig, int* out);
+/* Host-side query, no launch: the slices per thread that the quad path takes by default for n_slabs
+   slabs of ig->nz slices in one launch (n_slabs 1: lct_backproject_par of this block; a scan-mode recon
+   launches all of its slabs together): 8, or 4 where a view stays active for few slices, and 4, 2 or 1
+   where that would leave the chip's CTA slots empty.  A volume's values do not depend on it. */
+int lct_backproject_par_slices(const lct_geom* g, const lct_img* ig, int n_slabs, int* out);
 /* No counterpart in the reference.  lct_backproject_par for callers that cannot let the
    library allocate device memory (a host that budgets all device memory itself, an acquisition
    loop that must not stall or fail on an allocation, a plugin host with its own allocator): the

@@ -143,6 +143,7 @@ SIGNATURES: dict[str, tuple] = {
     "lct_backproject_par": (I32, [GP, IP, P, P, P, I32, I32, P]),
     "lct_backproject_par_noalloc": (I32, [GP, IP, P, P, P, I32, I32, P]),
     "lct_backproject_par_quad_path": (I32, [GP, IP, C.POINTER(I32)]),
+    "lct_backproject_par_slices": (I32, [GP, IP, I32, C.POINTER(I32)]),
     "lct_backproject_pi_ori": (I32, [GP, IP, P, P, P, I32, I32, P]),
     "lct_plan_create": (I32, [C.POINTER(ScanParams), P, P, C.POINTER(P)]),
     "lct_plan_adopt": (I32, [C.POINTER(PlanInfo), C.POINTER(BlockInfo), I32, P, P, C.POINTER(P)]),

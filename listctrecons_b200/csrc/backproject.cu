@@ -710,6 +710,15 @@ LCT_API int lct_backproject_par_quad_path(const lct_geom* g, const lct_img* ig, 
   return LCT_OK;
 }
 
+LCT_API int lct_backproject_par_slices(const lct_geom* g, const lct_img* ig, int n_slabs, int* out) {
+  int st = check_geom(g);
+  if (st) return st;
+  if ((st = check_img(ig))) return st;
+  if (n_slabs <= 0 || !out) return LCT_ERR_ARG;
+  *out = bp_nz_default(bp_z_base(*g, *ig), n_slabs * bp_tiles(*ig), ig->nz, device_sms());
+  return LCT_OK;
+}
+
 LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const float* d_betas,
                                 const float* d_proj, float* d_img, int interp, int addr,
                                 lct_stream stream) {
@@ -741,7 +750,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
       L.slab_z0[0] = 0;
       L.interp = interp;
       L.addr = addr;
-      L.nz_thread = bp_nz_default(*g, *ig);
+      L.nz_thread = bp_nz_default(bp_z_base(*g, *ig), bp_tiles(*ig), ig->nz, device_sms());
       L.z_base = 8;
       st = launch_bp_par_quads(*g, *ig, L, q, s);
     }

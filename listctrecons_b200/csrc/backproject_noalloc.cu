@@ -79,7 +79,7 @@ LCT_API int lct_backproject_par_noalloc(const lct_geom* g, const lct_img* ig,
   L.slab_z0[0] = 0;
   L.interp = interp;
   L.addr = addr;
-  L.nz_thread = bp_nz_default(*g, *ig);
+  L.nz_thread = bp_nz_default(bp_z_base(*g, *ig), bp_tiles(*ig), ig->nz, device_sms());
   L.z_base = 8;
   return launch_bp_par_quads(*g, *ig, L, q, s);
 }

@@ -2,7 +2,7 @@
 // volume): every buffer is owned per scan (one lct_recon each, allocated once), and a run is
 //   upload fans -> [graph] rebin all scans -> [graph] filter + quad pack all scans
 //               -> [graph] persistent work-list backprojection over every scan's tiles (one
-//                  launch per thread shape: each scan keeps the shape its own run would use)
+//                  launch per thread shape)
 //               -> download volumes.
 // The three stage graphs are captured once at create (after one eager warm-up run, which also
 // sets kernel attributes and loads modules).  The work-list kernel balances the uneven scans
@@ -129,14 +129,21 @@ LCT_API int lct_batch_create(const lct_plan* const* plans, int n, const lct_reco
       if (!recon_bp_quads_all(r) || r->o.interp != b->interp) b->worklist = false;
   }
   if (!st && b->worklist) {
-    // each scan keeps the thread shape its own run would use (the slices-per-thread heuristic,
-    // or the requested / autotuned shape); scans sharing a shape share a work list
+    // each scan takes the requested / autotuned thread shape, or the default for all scans' tiles
+    // together (its volume is the same bits in any); scans sharing a shape share a work list
     const int asz = bp_quad_args_size();
     std::map<std::tuple<int, int, bool>, std::vector<int>> by_shape;
+    long long tiles = 0;  // of all scans' slabs: they run together, and the default goes by that
+    for (auto* r : b->recs) tiles += r->info.n_blocks_run * bp_tiles(r->info.ig);
+    auto launch_of = [&](lct_recon* r, BpLaunch& L) {
+      recon_bp_launch(r, 0, r->info.n_blocks_run, r->d_img, L);
+      if (!bp_nz_requested(r->o.bp_nz))
+        L.nz_thread = bp_nz_default(bp_z_base(r->info.ctg, r->info.ig), tiles, kBlockSlices, device_sms());
+    };
     for (int i = 0; i < n; ++i) {
       lct_recon* r = b->recs[i];
       BpLaunch L;
-      recon_bp_launch(r, 0, r->info.n_blocks_run, r->d_img, L);
+      launch_of(r, L);
       r->o.bp_minb = L.minb > 0 ? L.minb : 4;
       by_shape[{L.nz_thread, r->o.bp_minb, L.z_base > L.nz_thread}].push_back(i);
     }
@@ -150,11 +157,11 @@ LCT_API int lct_batch_create(const lct_plan* const* plans, int n, const lct_reco
       for (int k = 0; k < gr.n && !st; ++k) {
         lct_recon* r = b->recs[kv.second[k]];
         BpLaunch L;
-        recon_bp_launch(r, 0, r->info.n_blocks_run, r->d_img, L);
-        int tiles = 0;
+        launch_of(r, L);
+        int ctas = 0;
         st = bp_quad_args_build(r->info.ctg, r->info.ig, L, r->d_quad,
-                                args.data() + (size_t)asz * k, &tiles);
-        prefix[k + 1] = prefix[k] + tiles;
+                                args.data() + (size_t)asz * k, &ctas);
+        prefix[k + 1] = prefix[k] + ctas;
       }
       b->groups.push_back(gr);
       BpGroup& g = b->groups.back();

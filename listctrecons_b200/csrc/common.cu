@@ -23,6 +23,15 @@ int cuda_status(cudaError_t e) {
 
 int launch_status() { return cuda_status(cudaGetLastError()); }
 
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+    return sms;
+  cudaGetLastError();
+  return 148;
+}
+
 // cudaDeviceReset destroys a device's context with all that lives in it -- pools, module addresses,
 // kernel attributes -- and the next call starts another, so what the library keeps per device is kept
 // for the context's id.

@@ -28,6 +28,7 @@ void set_cuda_error(cudaError_t e);
 int cuda_status(cudaError_t e);  // LCT_OK or LCT_ERR_CUDA (records e)
 int launch_status();             // cudaGetLastError() -> status
 
+int device_sms();                 // of the current device (a B200's where there is none)
 unsigned long long context_id();  // of the current device's context: another one after a device reset
 
 // Stream-ordered scratch of a stage entry point (common.cu), from a bounded pool of the library's own.
@@ -105,19 +106,36 @@ int launch_quad_pack(const float* rows, long long views, int ns, int nt, int add
 inline int bp_z_base(const lct_geom& g, const lct_img& ig) {
   return 0.5 * (double)g.pitch / (double)ig.dz < 6.0 ? 4 : 8;
 }
-// Slices per thread of the quad kernel by default: 8, which shares a view's terms among most slices;
-// 4 when a view stays active for fewer than 6 slices ((feed / 2) / dz); and fewer where one slab's
-// 16 x 16 tiles would leave most of the chip's 592 CTA slots empty and the views' latency in series
-// is what counts.  The line by tiles, on 736 x 64 views (ms at 1 / 2 / 4 / 8 slices): 32^2
-// 0.41 / 0.47 / 0.80 / 1.39, 64^2 0.48 / 0.47 / 0.77 / 1.25, 128^2 1.48 / 0.98 / 0.83 / 1.16, 192^2
-// 3.16 / 2.08 / 1.60 / 1.34, 256^2 5.41 / 3.54 / 2.70 / 2.32.  One slab's tiles, whatever the launch
-// holds: streamed, bounded and whole runs then sum alike.
-inline int bp_nz_default(const lct_geom& g, const lct_img& ig) {
-  const long long tiles = (long long)((ig.nx + 15) / 16) * ((ig.ny + 15) / 16);
-  if (tiles * 16 < 200) return 1;
-  if (tiles * 8 < 500) return 2;
-  if (tiles * 4 < 500) return 4;
-  return bp_z_base(g, ig);
+// 16 x 16 voxel tiles of a slice
+inline long long bp_tiles(const lct_img& ig) {
+  return (long long)((ig.nx + 15) / 16) * ((ig.ny + 15) / 16);
+}
+// Slices per thread of the quad kernel by default, for `tiles` voxel tiles of nz slices that run
+// together (the tiles of every slab of the launch, or of every scan of a batch; results do not depend on
+// it, bp_z_base): z_base, which shares a view's terms among most slices, where the launch fills the chip's
+// 4 CTA slots per SM at least twice; below that the shape whose last round leaves least of them idle.
+// A round takes a CTA's latency, hardly less with fewer CTAs on an SM.  CTA times in units of a z_base
+// thread's, fitted to 32^2 .. 192^2 images of 1 .. 16 slabs from 736 x 16, 32 and 64 views (every shape
+// timed in each: the choice costs 1% on average and at most 12% over the best).  ms at 1 / 2 / 4 / 8 slices, one
+// slab from 736 x 32: 32^2 0.47 / 0.53 / 0.94 / 1.77, 96^2 0.96 / 0.60 / 0.86 / 1.50, 128^2 1.53 / 0.98 /
+// 0.94 / 1.43, 192^2 3.02 / 1.98 / 1.73 / 1.58; sixteen slabs: 48^2 4.14 / 2.90 / 2.88 / 2.83, 96^2 12.7 /
+// 8.44 / 7.89 / 7.71.
+inline int bp_nz_default(int z_base, long long tiles, int nz, int sms) {
+  constexpr double kCta8[4] = {0.295, 0.32, 0.52, 1.0}, kCta4[3] = {0.42, 0.52, 1.0};
+  const double* cta = z_base == 4 ? kCta4 : kCta8;
+  auto ctas = [&](int k) { return tiles * ((nz + k - 1) / k); };
+  if (ctas(z_base) >= 8LL * sms) return z_base;
+  int best = z_base;
+  double best_time = 1e300;
+  for (int k = z_base, i = z_base == 4 ? 2 : 3; k >= 1; k /= 2, --i) {
+    const long long per_sm = (ctas(k) + sms - 1) / sms;
+    const double time = cta[i] * (1.1 * (double)(per_sm / 4) + (per_sm % 4 ? 1.0 : 0.0));
+    if (time < best_time * (1.0 - 1e-9)) {
+      best = k;
+      best_time = time;
+    }
+  }
+  return best;
 }
 // Backprojection from quad-layout views (full windows only; L.proj is ignored, L.quads used).
 int launch_bp_par_quads(const lct_geom& g, const lct_img& ig, const BpLaunch& L,

@@ -104,13 +104,17 @@ struct lct_recon {
 };
 
 namespace lct {
-// backprojection slices per thread: the requested 4 / 8 / 16, else bp_nz_default
-inline int pick_bp_nz(const lct_geom& g, const lct_img& ig, int requested) {
-  return requested == 4 || requested == 8 || requested == 16 ? requested : bp_nz_default(g, ig);
+inline bool bp_nz_requested(int bp_nz) { return bp_nz == 4 || bp_nz == 8 || bp_nz == 16; }
+// backprojection slices per thread: the requested 4 / 8 / 16, else the default of n_slabs slabs that run
+// together
+inline int pick_bp_nz(const lct_geom& g, const lct_img& ig, int requested, int n_slabs) {
+  return bp_nz_requested(requested)
+             ? requested
+             : bp_nz_default(bp_z_base(g, ig), n_slabs * bp_tiles(ig), kBlockSlices, device_sms());
 }
 // ... and the slices per base of their row coordinates: a requested thread shape has its own
 inline int pick_bp_z_base(const lct_geom& g, const lct_img& ig, int requested) {
-  return requested == 4 || requested == 8 || requested == 16 ? requested : bp_z_base(g, ig);
+  return bp_nz_requested(requested) ? requested : bp_z_base(g, ig);
 }
 // kernels one filter call launches
 inline int filter_launches(int mode) { return mode == LCT_FILTER_FP32 ? 1 : 2; }
