@@ -124,12 +124,18 @@ inline int bp_nz_default(int z_base, long long tiles, int nz, int sms) {
   constexpr double kCta8[4] = {0.295, 0.32, 0.52, 1.0}, kCta4[3] = {0.42, 0.52, 1.0};
   const double* cta = z_base == 4 ? kCta4 : kCta8;
   auto ctas = [&](int k) { return tiles * ((nz + k - 1) / k); };
-  if (ctas(z_base) >= 8LL * sms) return z_base;
-  int best = z_base;
+  int most = z_base, i = z_base == 4 ? 2 : 3;
+  for (; most / 2 >= nz; most /= 2) --i;  // no more slices than the call has
+  if (ctas(most) >= 8LL * sms) return most;
+  int best = most;
   double best_time = 1e300;
-  for (int k = z_base, i = z_base == 4 ? 2 : 3; k >= 1; k /= 2, --i) {
+  for (int k = most; k >= 1; k /= 2, --i) {
     const long long per_sm = (ctas(k) + sms - 1) / sms;
-    const double time = cta[i] * (1.1 * (double)(per_sm / 4) + (per_sm % 4 ? 1.0 : 0.0));
+    // a thread's slices that the call has, in groups of two; about a fifth of a CTA's time is per view
+    const int chunks = (nz + k - 1) / k;
+    const int used = k == 1 ? 1 : ((nz + chunks - 1) / chunks + 1) / 2 * 2;
+    const double time = cta[i] * (0.2 + 0.8 * used / k) *
+                        (1.1 * (double)(per_sm / 4) + (per_sm % 4 ? 1.0 : 0.0));
     if (time < best_time * (1.0 - 1e-9)) {
       best = k;
       best_time = time;

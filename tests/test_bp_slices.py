@@ -33,6 +33,11 @@ def test_few_active_slices(nx, slabs, want):
     assert _slices(nx, slabs, dz=1.5) == want  # 16 mm of feed: 5.3 slices of 1.5 mm active
 
 
+@pytest.mark.parametrize("nx,nz,want", [(512, 3, 4), (512, 5, 8), (512, 8, 8), (256, 5, 4), (33, 5, 1)])
+def test_few_slices(nx, nz, want):
+    assert _slices(nx, 1, nz=nz) == want  # 512^2 x 5: 1.61 ms in threads of 8, 1.84 ms in threads of 2
+
+
 @pytest.mark.parametrize("nx", [32, 128, 512])
 def test_never_more_threads_slices_than_a_few_slices_need(nx):
     assert _slices(nx, 1, nz=1) == 1
