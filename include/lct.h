@@ -349,9 +349,11 @@ int lct_recon_run_file(lct_recon* r, const char* fan_path, const char* image_pat
    reads (summed over threads), s3[1] = time the pipeline waited for fan chunks not yet read,
    s3[2] = time it waited for a free slab slot of the writer.  Zeros before the first call. */
 int lct_recon_io_times(const lct_recon* r, float* s3);
-/* Backprojection autotuner (no reference counterpart): times the kernel's slices-per-thread x
-   CTAs-per-SM variants on this recon's buffers, keeps the fastest in the recon, and caches it per
-   geometry class for the process.  Synchronous; returns the choice. */
+/* Backprojection autotuner (no reference counterpart): times the default thread shape and the kernel's
+   slices-per-thread (4, 8, 16) x CTAs-per-SM variants on this recon's buffers, keeps the fastest in the
+   recon, and caches it per geometry class for the process.  Synchronous; returns the choice -- for a
+   kept default, whose threads may take fewer slices, the 8 or 4 slices whose row coordinates share a
+   base (lct_backproject_par_slices tells the threads' number). */
 int lct_recon_autotune(lct_recon* r, int* nz, int* minb);
 /* Device-side per-stage time of the last run (ms): h2d, rebin, filter, backproject, d2h.  A
    streamed run reports its whole overlapped span as backprojection and 0 for the others. */

@@ -113,11 +113,15 @@ LCT_API int lct_batch_create(const lct_plan* const* plans, int n, const lct_reco
     lct_recon* big = b->recs[0];
     for (auto* r : b->recs)
       if (r->voxel_updates > big->voxel_updates) big = r;
-    int nz = 8, mb = 4;
-    st = lct_recon_autotune(big, &nz, &mb);
+    st = lct_recon_autotune(big, nullptr, nullptr);
+    // scans whose default is of the same kind run in one work list with it and take its shape; the others
+    // keep theirs
+    const int base = bp_z_base(big->info.ctg, big->info.ig);
     for (auto* r : b->recs) {
-      r->o.bp_nz = nz;
-      r->o.bp_minb = mb;
+      const bool same = bp_z_base(r->info.ctg, r->info.ig) == base;
+      r->bp_tuned = same;
+      r->o.bp_nz = same ? big->o.bp_nz : 0;
+      r->o.bp_minb = same ? big->o.bp_minb : 0;
     }
   }
   // work list: every scan on the quad kernel with one interpolation and thread shape (texture-

@@ -247,8 +247,9 @@ int recon_stage_bp(lct_recon* r, float* d_img, cudaStream_t s);
 }
 
 // Backprojection autotuner: times the quad kernel over slices per thread x CTAs per SM on this
-// recon's own buffers and keeps the fastest; results are cached per geometry class (detector,
-// volume, window, interpolation and views-per-slice), so a class is tuned once per process.
+// recon's own buffers, the default shape (which may have fewer slices per thread than can be requested)
+// first, and keeps the fastest; results are cached per geometry class (detector, volume, window,
+// interpolation and views-per-slice), so a class is tuned once per process.  A kept default stays one: bp_nz 0.
 LCT_API int lct_recon_autotune(lct_recon* r, int* nz_out, int* minb_out) {
   if (r && r->bounded) return LCT_ERR_UNSUPPORTED;  // no whole-scan buffers to time on
   if (!r) return LCT_ERR_ARG;
@@ -259,6 +260,14 @@ LCT_API int lct_recon_autotune(lct_recon* r, int* nz_out, int* minb_out) {
     if (minb_out) *minb_out = r->o.bp_minb > 0 ? r->o.bp_minb : 4;
     return LCT_OK;
   }
+  r->bp_tuned = true;
+  auto keep = [&](int nz, int minb) {
+    r->o.bp_nz = nz;
+    r->o.bp_minb = minb;
+    if (nz_out) *nz_out = nz ? nz : bp_z_base(g, ig);
+    if (minb_out) *minb_out = minb ? minb : 4;
+    return LCT_OK;
+  };
   static std::mutex mu;
   static std::map<std::vector<long long>, std::pair<int, int>> cache;
   const std::vector<long long> key = {g.ns, g.nt, ig.nx, ig.ny, g.n_angle, g.n_proj_turn,
@@ -268,13 +277,7 @@ LCT_API int lct_recon_autotune(lct_recon* r, int* nz_out, int* minb_out) {
   {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
-    if (it != cache.end()) {
-      r->o.bp_nz = it->second.first;
-      r->o.bp_minb = it->second.second;
-      if (nz_out) *nz_out = r->o.bp_nz;
-      if (minb_out) *minb_out = r->o.bp_minb;
-      return LCT_OK;
-    }
+    if (it != cache.end()) return keep(it->second.first, it->second.second);
   }
   cudaStream_t s;
   int st = cuda_status(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -285,37 +288,34 @@ LCT_API int lct_recon_autotune(lct_recon* r, int* nz_out, int* minb_out) {
   const size_t qbytes = sizeof(float4) * (size_t)r->g_count * quad_view_elems(g.ns, g.nt);
   if (!r->tex_bp) st = cuda_status(cudaMemsetAsync(r->d_quad, 0, qbytes, s));
   float best = 1e30f;
-  int bnz = 8, bmb = 4;
-  const int nzs[3] = {4, 8, 16}, mbs[3] = {2, 3, 4};
-  for (int i = 0; i < 3 && !st; ++i)
-    for (int j = 0; j < 3 && !st; ++j) {
-      r->o.bp_nz = nzs[i];
-      r->o.bp_minb = mbs[j];
-      if ((st = recon_stage_bp(r, r->d_img, s))) break;  // warm
-      cudaEventRecord(e0, s);
-      if ((st = recon_stage_bp(r, r->d_img, s))) break;
-      cudaEventRecord(e1, s);
-      if ((st = cuda_status(cudaEventSynchronize(e1)))) break;
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best) {
-        best = ms;
-        bnz = nzs[i];
-        bmb = mbs[j];
-      }
+  int bnz = 0, bmb = 0;
+  auto time_shape = [&](int nz, int minb) {
+    r->o.bp_nz = nz;
+    r->o.bp_minb = minb;
+    if ((st = recon_stage_bp(r, r->d_img, s))) return;  // warm
+    cudaEventRecord(e0, s);
+    if ((st = recon_stage_bp(r, r->d_img, s))) return;
+    cudaEventRecord(e1, s);
+    if ((st = cuda_status(cudaEventSynchronize(e1)))) return;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    if (ms < best) {
+      best = ms;
+      bnz = nz;
+      bmb = minb;
     }
+  };
+  if (!st) time_shape(0, 0);
+  for (int nz : {4, 8, 16})
+    for (int minb : {2, 3, 4})
+      if (!st) time_shape(nz, minb);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaStreamDestroy(s);
-  r->o.bp_nz = bnz;
-  r->o.bp_minb = bmb;
+  keep(bnz, bmb);
   if (st) return st;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    cache[key] = {bnz, bmb};
-  }
-  if (nz_out) *nz_out = bnz;
-  if (minb_out) *minb_out = bmb;
+  std::lock_guard<std::mutex> lock(mu);
+  cache[key] = {bnz, bmb};
   return LCT_OK;
 }
 
@@ -400,7 +400,7 @@ static int run_blocks(lct_recon* r, const float* d_fan, float* d_img, cudaStream
       L.interp = r->o.interp;
       L.addr = addr;
       L.nz_thread = bp_nz;
-      L.z_base = pick_bp_z_base(g, ig, r->o.bp_nz);
+      L.z_base = pick_bp_z_base(g, ig, r->o.bp_nz, r->bp_tuned);
       L.minb = r->o.bp_minb;
       if (r->quads) {
         if ((st = recon_pack(r, r->d_par, g.n_angle, 0, addr, s))) return st;
@@ -476,7 +476,7 @@ void recon_bp_launch(const lct_recon* r, int b0, int b1, float* d_img, BpLaunch&
   L.interp = r->o.interp;
   L.addr = block_addr(r, b0);
   L.nz_thread = pick_bp_nz(g, r->info.ig, r->o.bp_nz, b1 - b0);
-  L.z_base = pick_bp_z_base(g, r->info.ig, r->o.bp_nz);
+  L.z_base = pick_bp_z_base(g, r->info.ig, r->o.bp_nz, r->bp_tuned);
   L.minb = r->o.bp_minb;
   // betas are indexed by the same slab offset: shift the base by g_first
   L.betas = r->d_betas + r->g_first;

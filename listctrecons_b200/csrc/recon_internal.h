@@ -70,6 +70,7 @@ struct lct_recon {
   bool tex_bp = false;       // the pairs backprojection samples a 3-D texture (TEX8) instead
   lct::ViewTexture vtex;     // filtered views as that texture (scan: global views; block: one block)
   lct::ViewTexture pi_tex;   // PI-original rebin in TEX8: the fan block as a texture, reused per block
+  bool bp_tuned = false;     // o.bp_nz was chosen by lct_recon_autotune
   bool tma_bp = false;       // EXACT pairs backprojection with TMA-staged footprints (same quads)
   CUtensorMap tma_map;       // d_quad as the staged kernel's tensor
   cudaEvent_t ev[6] = {};
@@ -112,9 +113,11 @@ inline int pick_bp_nz(const lct_geom& g, const lct_img& ig, int requested, int n
              ? requested
              : bp_nz_default(bp_z_base(g, ig), n_slabs * bp_tiles(ig), kBlockSlices, device_sms());
 }
-// ... and the slices per base of their row coordinates: a requested thread shape has its own
-inline int pick_bp_z_base(const lct_geom& g, const lct_img& ig, int requested) {
-  return bp_nz_requested(requested) ? requested : bp_z_base(g, ig);
+// ... and the slices per base of their row coordinates: a requested thread shape has its own; a tuned one of
+// fewer slices keeps the default's, so that its values are the default's too
+inline int pick_bp_z_base(const lct_geom& g, const lct_img& ig, int requested, bool tuned) {
+  const int z_base = bp_z_base(g, ig);
+  return bp_nz_requested(requested) && !(tuned && requested < z_base) ? requested : z_base;
 }
 // kernels one filter call launches
 inline int filter_launches(int mode) { return mode == LCT_FILTER_FP32 ? 1 : 2; }
