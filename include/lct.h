@@ -271,7 +271,9 @@ void lct_plan_destroy(lct_plan* plan);
    TEXTURE  views in a 3-D texture, one hardware fetch per sample (TEX8 only: the reference's own
             fetch, CUDA/Backprojector.cu:85-86; QUADS otherwise);
    QUADS_TMA (EXACT only) the quads, with each view's tile footprint staged in shared memory by
-            TMA before the samples read it (the same values: bit-identical to QUADS);
+            TMA before the samples read it (the same values: bit-identical to QUADS); threads of 8
+            slices, whatever the image's size -- QUADS where bp_nz asks for others, where a view stays
+            active for few slices, and for the parts of a streamed run's first slab;
    AUTO     QUADS (on B200 the quad kernel's TEX8 path outruns the texture fetch: 89 against
             137 ms on a 512^2 x 256 volume of 736 x 64 views). */
 #define LCT_BP_SAMPLER_AUTO 0
@@ -290,9 +292,10 @@ typedef struct lct_recon_opts {
   int interp;        /* LCT_INTERP_* */
   int addr;          /* LCT_ADDR_* */
   int bp_nz;         /* backprojection slices per thread: 4, 8, 16; 0 = default (8; fewer when a
-                        view stays active for few slices or the image is small); -1 = autotune at
-                        create */
-  int bp_minb;       /* backprojection CTAs per SM the register budget targets: 1-4 (0 = 4) */
+                        view stays active for few slices or what runs together is small:
+                        lct_backproject_par_slices); -1 = autotune at create */
+  int bp_minb;       /* backprojection CTAs per SM the register budget targets: 1-4 (0 = 4); with
+                        1-3 the default bp_nz is 8 or 4 whatever the image's size */
   int bp_sampler;    /* LCT_BP_SAMPLER_*: how the backprojector samples the filtered views */
 } lct_recon_opts;
 
@@ -353,7 +356,8 @@ int lct_recon_io_times(const lct_recon* r, float* s3);
    slices-per-thread (4, 8, 16) x CTAs-per-SM variants on this recon's buffers, keeps the fastest in the
    recon, and caches it per geometry class for the process.  Synchronous; returns the choice -- for a
    kept default, whose threads may take fewer slices, the 8 or 4 slices whose row coordinates share a
-   base (lct_backproject_par_slices tells the threads' number). */
+   base (lct_backproject_par_slices tells the threads' number).  A recon that cannot be tuned (block mode,
+   LEGACY addressing, no quads) keeps its shape, which is returned. */
 int lct_recon_autotune(lct_recon* r, int* nz, int* minb);
 /* Device-side per-stage time of the last run (ms): h2d, rebin, filter, backproject, d2h.  A
    streamed run reports its whole overlapped span as backprojection and 0 for the others. */

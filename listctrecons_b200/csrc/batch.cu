@@ -141,7 +141,7 @@ LCT_API int lct_batch_create(const lct_plan* const* plans, int n, const lct_reco
     for (auto* r : b->recs) tiles += r->info.n_blocks_run * bp_tiles(r->info.ig);
     auto launch_of = [&](lct_recon* r, BpLaunch& L) {
       recon_bp_launch(r, 0, r->info.n_blocks_run, r->d_img, L);
-      if (!bp_nz_requested(r->o.bp_nz))
+      if (!bp_nz_requested(r->o.bp_nz) && !bp_minb_requested(r->o.bp_minb))
         L.nz_thread = bp_nz_default(bp_z_base(r->info.ctg, r->info.ig), tiles, kBlockSlices, device_sms());
     };
     for (int i = 0; i < n; ++i) {

@@ -256,7 +256,7 @@ LCT_API int lct_recon_autotune(lct_recon* r, int* nz_out, int* minb_out) {
   const lct_geom& g = r->info.ctg;
   const lct_img& ig = r->info.ig;
   if (r->o.mode != LCT_MODE_SCAN || !r->quads || r->o.addr == LCT_ADDR_LEGACY) {
-    if (nz_out) *nz_out = pick_bp_nz(g, ig, r->o.bp_nz, 1);
+    if (nz_out) *nz_out = pick_bp_nz(r, 1);
     if (minb_out) *minb_out = r->o.bp_minb > 0 ? r->o.bp_minb : 4;
     return LCT_OK;
   }
@@ -368,7 +368,7 @@ static int run_blocks(lct_recon* r, const float* d_fan, float* d_img, cudaStream
   const lct_geom& g = r->info.ctg;
   const lct_img& ig = r->info.ig;
   const long long slab = (long long)kBlockSlices * ig.nx * ig.ny;
-  const int bp_nz = pick_bp_nz(g, ig, r->o.bp_nz, 1);
+  const int bp_nz = pick_bp_nz(r, 1);
   int st;
   for (int b = 0; b < r->info.n_blocks_run; ++b) {
     const lct_block_info& bi = r->blocks[b];
@@ -475,7 +475,7 @@ void recon_bp_launch(const lct_recon* r, int b0, int b1, float* d_img, BpLaunch&
   }
   L.interp = r->o.interp;
   L.addr = block_addr(r, b0);
-  L.nz_thread = pick_bp_nz(g, r->info.ig, r->o.bp_nz, b1 - b0);
+  L.nz_thread = pick_bp_nz(r, b1 - b0);
   L.z_base = pick_bp_z_base(g, r->info.ig, r->o.bp_nz, r->bp_tuned);
   L.minb = r->o.bp_minb;
   // betas are indexed by the same slab offset: shift the base by g_first

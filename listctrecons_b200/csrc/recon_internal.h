@@ -106,12 +106,16 @@ struct lct_recon {
 
 namespace lct {
 inline bool bp_nz_requested(int bp_nz) { return bp_nz == 4 || bp_nz == 8 || bp_nz == 16; }
+inline bool bp_minb_requested(int bp_minb) { return bp_minb >= 1 && bp_minb <= 3; }
 // backprojection slices per thread: the requested 4 / 8 / 16, else the default of n_slabs slabs that run
-// together
-inline int pick_bp_nz(const lct_geom& g, const lct_img& ig, int requested, int n_slabs) {
-  return bp_nz_requested(requested)
-             ? requested
-             : bp_nz_default(bp_z_base(g, ig), n_slabs * bp_tiles(ig), kBlockSlices, device_sms());
+// together.  The TMA-staged kernel has 8 slices per thread, and the smaller shapes have no other register
+// budget than 4 CTAs per SM: where either is asked for, the base's slices.
+inline int pick_bp_nz(const lct_recon* r, int n_slabs) {
+  const lct_geom& g = r->info.ctg;
+  const lct_img& ig = r->info.ig;
+  if (bp_nz_requested(r->o.bp_nz)) return r->o.bp_nz;
+  if (r->tma_bp || bp_minb_requested(r->o.bp_minb)) return bp_z_base(g, ig);
+  return bp_nz_default(bp_z_base(g, ig), n_slabs * bp_tiles(ig), kBlockSlices, device_sms());
 }
 // ... and the slices per base of their row coordinates: a requested thread shape has its own; a tuned one of
 // fewer slices keeps the default's, so that its values are the default's too
