@@ -68,14 +68,19 @@ __device__ double noisy_integral(double p, double i0, uint64_t seed, uint64_t id
 // Bound: the FP64 pipe.  With M = the ellipsoid's frame scaled to a unit sphere, the ray S + l D
 // meets it where |M (S - c) + l M D| = 1, a quadratic with coefficients A = |M D|^2, B and C.  D is
 // (Dx, Dy) of the column and tz of the row, so A is a quadratic and B a line in tz whose
-// coefficients need the column only: a thread makes kSimRows rows of one column and pays, per
+// coefficients need the column only: a thread makes up to 16 rows of one column and pays, per
 // ellipsoid, about 20 operations for the column and 2 per row (the discriminant B^2 - A C, a quadratic
 // in the row), where the products with the rotation and six divisions per ray took about 100.  The
 // chord sqrt(disc) / A, where there is one, is one rsqrt.
 // 600 views x 64 x 736, 40 ellipsoids, I0 = 1e5: 1.1 ms, one ray per thread with everything
 // evaluated per ray 8.4 ms.
-constexpr int kSimRows = 16;     // rows per thread and pass
+// A launch that leaves the chip's CTA slots empty is bound by one thread's time instead: it takes ROWS = 4
+// rows per thread, or 1.  One view x 16 x 736: 67 us with 16 rows per thread, 20 with 1 (one ray per thread
+// with everything evaluated per ray 39).  A row is a step
+// from its 16's first row in any of them, so its value does not depend on the launch.
+constexpr int kSimRows = 16;     // rows whose quadratics share a base
 constexpr int kSimThreads = 128; // columns per CTA
+constexpr int kSimCtas = 5;      // CTAs per SM
 
 struct SimEllipsoid {            // one ellipsoid seen from one view
   double xx, xy2, yy, xz2, yz2, zz;  // M^T M, off-diagonal terms doubled
@@ -84,7 +89,8 @@ struct SimEllipsoid {            // one ellipsoid seen from one view
 };
 
 // grid (ceil(ns / 128), row chunks, views); CTA: 128 columns x rows_per_cta rows of one view
-__global__ void __launch_bounds__(kSimThreads, 5) sim_project_kernel(
+template <int ROWS>
+__global__ void __launch_bounds__(kSimThreads, kSimCtas) sim_project_kernel(
     const double* __restrict__ ell, int ne, int ns, int nt, int rows_per_cta, float ds, float dt,
     float ws, float wt, float dso, const double* __restrict__ angles,
     const double* __restrict__ zpos, long long v0, double i0, uint64_t seed,
@@ -127,14 +133,17 @@ __global__ void __launch_bounds__(kSimThreads, 5) sim_project_kernel(
   const double dxx = dx * dx, dxy = dx * dy, dyy = dy * dy;
   const double step = (double)dt / R;  // tz from one row to the next
   const int row1 = min(nt, (int)(blockIdx.y + 1) * rows_per_cta);
-  for (int it0 = blockIdx.y * rows_per_cta; it0 < row1; it0 += kSimRows) {
-    const double t0 = ((double)it0 - wt) * dt / R;
-    double p[kSimRows];
+  for (int it0 = blockIdx.y * rows_per_cta; it0 < row1; it0 += ROWS) {
+    const int base = it0 / kSimRows * kSimRows;
+    const double t0 = ((double)base - wt) * dt / R;
+    const double r0 = ROWS == kSimRows ? 0.0 : (double)(it0 - base);  // steps from the base to the first row
+    const unsigned rows = (1u << min(ROWS, row1 - it0)) - 1u;         // of this pass
+    double p[ROWS];
 #pragma unroll
-    for (int r = 0; r < kSimRows; ++r) p[r] = 0.0;
+    for (int r = 0; r < ROWS; ++r) p[r] = 0.0;
     for (int m = 0; m < ne; ++m) {
       const SimEllipsoid& e = s_e[m];
-      // A and B at row it0 + r: A0 + r (A1 + r A2), B0 + r B1; the discriminant B^2 - A c is a
+      // A and B at row base + r: A0 + r (A1 + r A2), B0 + r B1; the discriminant B^2 - A c is a
       // quadratic in r too, and A is needed where it is positive only
       const double ul = fma(dx, e.xz2, dy * e.yz2), tl = fma(t0, e.zz, ul);
       const double A0 = fma(t0, tl, fma(dxx, e.xx, fma(dxy, e.xy2, dyy * e.yy)));
@@ -144,24 +153,25 @@ __global__ void __launch_bounds__(kSimThreads, 5) sim_project_kernel(
       const double d0 = fma(B0, B0, -(A0 * c)), d1 = fma(2.0 * B0, B1, -(A1 * c)), d2 = fma(B1, B1, -(A2 * c));
       unsigned hit = 0;
 #pragma unroll
-      for (int r = 0; r < kSimRows; ++r)
-        if (fma((double)r, fma((double)r, d2, d1), d0) > 0.0) hit |= 1u << r;
+      for (int r = 0; r < ROWS; ++r)
+        if (fma(r0 + r, fma(r0 + r, d2, d1), d0) > 0.0) hit |= 1u << r;
+      hit &= rows;
       if (!hit) continue;
 #pragma unroll
-      for (int r = 0; r < kSimRows; ++r)
+      for (int r = 0; r < ROWS; ++r)
         if ((hit >> r) & 1u) {
-          const double disc = fma((double)r, fma((double)r, d2, d1), d0);
-          const double A = fma((double)r, fma((double)r, A2, A1), A0);
+          const double disc = fma(r0 + r, fma(r0 + r, d2, d1), d0);
+          const double A = fma(r0 + r, fma(r0 + r, A2, A1), A0);
           p[r] = fma(mu2 * disc, rsqrt(disc * A * A), p[r]);  // sqrt(disc) / A
         }
     }
 #pragma unroll 2
-    for (int r = 0; r < kSimRows; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
       const int it = it0 + r;
       if (it >= row1) break;
       double pr = p[0];
 #pragma unroll
-      for (int k = 1; k < kSimRows; ++k) pr = r == k ? p[k] : pr;
+      for (int k = 1; k < ROWS; ++k) pr = r == k ? p[k] : pr;
       const double tz = ((double)it - wt) * dt / R;
       const uint64_t idx = ((uint64_t)v * nt + it) * ns + is;
       fan[((long long)blockIdx.z * nt + it) * ns + is] =
@@ -226,20 +236,22 @@ LCT_API int lct_sim_project(const double* d_ellipsoids, int n_ellipsoids, int ns
   const long long nv = v1 - v0;
   cudaStream_t s = (cudaStream_t)stream;
   // a CTA makes all rows of its columns (the ellipsoids' view terms once) unless that leaves fewer
-  // CTAs than 8 per SM; then one pass of rows each
+  // CTAs than 8 per SM; then one pass of rows each, and of as few rows as one round of CTA slots holds
+  const int sms = device_sms();
   const int cols = (ns + kSimThreads - 1) / kSimThreads;
-  const int passes = (nt + kSimRows - 1) / kSimRows;
-  const int chunks = (long long)cols * nv >= 8 * 148 ? (passes + 15) / 16 : passes;
-  const int rows_per_cta = (passes + chunks - 1) / chunks * kSimRows;
+  const long long slots = (long long)kSimCtas * sms;
+  const int rows = cols * nv * nt <= slots ? 1 : (cols * nv * ((nt + 3) / 4) <= slots ? 4 : kSimRows);
+  const int passes = (nt + rows - 1) / rows;
+  const int chunks = cols * nv >= 8LL * sms ? (passes + 15) / 16 : passes;
+  const int rows_per_cta = (passes + chunks - 1) / chunks * rows;
   const unsigned gy = (unsigned)((nt + rows_per_cta - 1) / rows_per_cta);
   if (gy > 65535) return LCT_ERR_ARG;
+  auto kernel = rows == 1 ? sim_project_kernel<1> : (rows == 4 ? sim_project_kernel<4> : sim_project_kernel<kSimRows>);
   for (long long c = 0; c < nv; c += 65535) {
     const long long cnt = nv - c < 65535 ? nv - c : 65535;
     dim3 grid(cols, gy, (unsigned)cnt);
-    sim_project_kernel<<<grid, kSimThreads, 0, s>>>(d_ellipsoids, n_ellipsoids, ns, nt,
-                                                    rows_per_cta, ds, dt, ws, wt, dso, d_angles,
-                                                    d_zpos, v0 + c, i0, seed,
-                                                    d_fan + c * (long long)nt * ns);
+    kernel<<<grid, kSimThreads, 0, s>>>(d_ellipsoids, n_ellipsoids, ns, nt, rows_per_cta, ds, dt, ws, wt, dso,
+                                        d_angles, d_zpos, v0 + c, i0, seed, d_fan + c * (long long)nt * ns);
     int st = launch_status();
     if (st) return st;
   }

@@ -1,0 +1,74 @@
+"""The scan simulator's rows per thread (16, and 4 or 1 where a launch would leave the chip empty): a view's
+values do not depend on how many views a call makes, with and without noise, on detectors whose rows end
+inside a thread's; and they are the FP64 chord lengths (tolerance 1e-6: FP32 results of FP64 sums)."""
+import numpy as np
+import pytest
+
+from listctrecons_b200.scan import Phantom, ScanGeometry, simulate_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+def _chords(geo, ph, v):
+    """Line integrals of view v in numpy, [nt][ns]."""
+    b, z = geo.angles64()[v], geo.zpos64()[v]
+    S = np.array([-geo.dso * np.sin(b), geo.dso * np.cos(b), z])
+    a = b - (np.arange(geo.ns) - geo.central_channel) * geo.ds / geo.dso
+    t = (np.arange(geo.nt) - (geo.nt - 1) / 2.0) * geo.dt / geo.dso
+    D = np.stack(np.broadcast_arrays(np.sin(a)[None, :], -np.cos(a)[None, :], t[:, None]), axis=-1)
+    out = np.zeros((geo.nt, geo.ns))
+    for e in np.asarray(ph.records, dtype=np.float64):
+        c, ax, rot, mu = e[:3], e[3:6], e[6:15].reshape(3, 3), e[15]
+        s, d = ((S - c) @ rot) / ax, (D @ rot) / ax
+        A, B, C = (d * d).sum(-1), d @ s, s @ s - 1.0
+        disc = np.maximum(B * B - A * C, 0.0)
+        out += 2.0 * mu * np.sqrt(disc) / A * np.sqrt((D * D).sum(-1))
+    return out
+
+
+@pytest.mark.parametrize("nt", [1, 3, 16, 17, 37])
+def test_views_do_not_depend_on_the_launch(cuda, nt):
+    geo = ScanGeometry(ns=300, nt=nt, ds=0.8, dt=0.9, npt=1000, pitch=0.9, nx=64, ny=64, dx=3.0,
+                       dz=1.0).with_blocks(1)
+    z = geo.zpos64()
+    ph = Phantom.random(12, seed=5, fov_radius=90.0, z_lo=float(z.min()), z_hi=float(z.max()))
+    many = simulate_gpu(geo, ph, i0=0.0, seed=3, v0=0, v1=400).cpu().numpy()   # 16 rows per thread
+    noisy = simulate_gpu(geo, ph, i0=1e5, seed=3, v0=0, v1=400).cpu().numpy()
+    for n in (1, 4, 16, 60):                                                    # 1, 4 or 16 rows
+        assert np.array_equal(simulate_gpu(geo, ph, i0=0.0, seed=3, v0=7, v1=7 + n).cpu().numpy(), many[7:7 + n])
+        assert np.array_equal(simulate_gpu(geo, ph, i0=1e5, seed=3, v0=7, v1=7 + n).cpu().numpy(), noisy[7:7 + n])
+    for v in (0, 123):
+        ref = _chords(geo, ph, v)
+        assert np.linalg.norm(many[v] - ref) < 1e-6 * np.linalg.norm(ref)
+
+
+def test_one_view_is_not_slow(cuda):
+    """One view of 16 rows leaves most of the chip empty, forty do not: it takes less than 0.8 of their time
+    (0.9 with one thread's 16 rows in series).  The best of twenty runs each."""
+    import torch
+
+    from listctrecons_b200 import capi
+
+    geo = ScanGeometry(ns=736, nt=16, ds=0.6, dt=0.6, npt=1152, pitch=0.9, nx=64, ny=64, dx=3.0,
+                       dz=1.0).with_blocks(1)
+    z = geo.zpos64()
+    ph = Phantom.random(40, seed=3, fov_radius=110.0, z_lo=float(z.min()), z_hi=float(z.max()))
+    ell = torch.as_tensor(np.ascontiguousarray(ph.records), dtype=torch.float64, device="cuda")
+    ang, zp = (torch.as_tensor(a, device="cuda") for a in (geo.angles64(), z))
+    out = torch.empty((40, 16, 736), device="cuda")
+
+    def best(views):
+        ts = []
+        for _ in range(20):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            capi.check(capi.lib().lct_sim_project(
+                ell.data_ptr(), 40, 736, 16, 0.6, 0.6, 367.5, 7.5, geo.dso, ang.data_ptr(), zp.data_ptr(), 0,
+                views, 1e5, 3, out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+            b.record()
+            torch.cuda.synchronize()
+            ts.append(a.elapsed_time(b))
+        return min(ts)
+
+    one, forty = best(1), best(40)
+    assert one < 0.8 * forty, (one, forty)
