@@ -19,7 +19,9 @@
 // accumulators of output rows r - 2, r - 1 and r, 32 columns apart in tensor memory, so a pixel's
 // channels are read from shared memory 3 x 10 / 8 times instead of 9 (N64 and N32 at the tile's edges).
 // Two buffers of 8 x 32 columns fill tensor memory; the packed weights sit in shared memory for the
-// CTA's lifetime.  Per output the taps add in the order (dx, dy, channel half).
+// CTA's lifetime.  Per output the taps add in the order (dx, dy, channel half).  Launches of few tiles take
+// lower ones (conv_height).  The first tiles' boxes load while the CTA stages its weights and zeroes its
+// accumulators (64^2 x 16 slices: 83 us a forward pass, 93 with the loads after that).
 // Bound: shared-memory operand reads (7 KB per MMA), then HBM.  512 x 512, 32 slices: 190 us per
 // hidden layer; one tap per MMA (M128 x N32, three boxes per tile) 308 us.
 // Fused epilogues: bias + ReLU -> bf16 (forward), ReLU mask of the previous activation -> bf16 delta
@@ -32,6 +34,7 @@
 #include <cmath>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "lct_internal.h"
@@ -42,8 +45,8 @@ namespace lct {
 constexpr int kCnnLayers = 8, kCnnC = 32, kCnnTaps = 9, kCnnK = kCnnTaps * kCnnC;  // K = 288
 constexpr int kCnnParams = 57249;     // sum over layers of cin*cout*9 + cout
 constexpr int kWSlot = kCnnC * kCnnK;  // packed weights of one layer, elements
-constexpr int kConvRows = 8;      // output rows of a tile
-constexpr int kConvIn = kConvRows + 2;
+constexpr int kConvHeights = 3;   // output rows of a tile: 8, 4 or 2 (conv_height)
+LCT_HD constexpr int conv_rows(int height) { return 8 >> height; }
 constexpr int kConvMaxN = 128;    // pixels of a tile, a multiple of 8 (its box starts on a block)
 constexpr int kConvThreads = 320; // warp 0 copies, warp 1 MMA + TMEM, warps 2-9 epilogue
 constexpr int kConvMaxStages = 8;
@@ -97,15 +100,17 @@ LCT_HD constexpr uint32_t dw_plane(int n_px) { return (uint32_t)(n_px + 2) * 16;
 
 // PLANES: planes of the input (1: the network input, whose channels 8..15 read a zeroed plane of
 // shared memory and whose second half of 16 channels does not exist; 4: an activation).
+// ROWS: output rows of a tile.
 // Every wait is bounded; on a timeout the CTA drains its copies and MMAs, raises the device status
 // word and leaves its remaining tiles unwritten.
-template <int EPI, int PLANES>
+template <int EPI, int PLANES, int ROWS>
 __global__ void __launch_bounds__(kConvThreads, 1)
     conv_tc_kernel(const __grid_constant__ CUtensorMap mbox, const ConvArgs a) {
   constexpr bool kLast = EPI == kEpiResid || EPI == kEpiGate;
   constexpr int kHalves = PLANES == 1 ? 1 : 2;  // K16 steps per tap
   constexpr int kCo = kLast ? 16 : 32;          // accumulator columns of an output row
-  constexpr uint32_t kBuf = kConvRows * kCo;    // columns of a buffer
+  constexpr int kIn = ROWS + 2;                 // input rows of a tile
+  constexpr uint32_t kBuf = ROWS * kCo;         // columns of a buffer
   constexpr uint32_t kTmem = 2 * kBuf;
   constexpr uint32_t kWPlane = 3 * kCo * 16, kWBlock = 2 * kWPlane;  // weights of (dx, half), [2][3 kCo][8]
   extern __shared__ __align__(128) uint8_t smem[];
@@ -123,6 +128,15 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   const uint32_t stage0 = smem_u32(smem), zero0 = stage0 + (uint32_t)S * a.stage_bytes;
   const uint32_t w0 = zero0 + (PLANES == 1 ? kConvZero : 0u);
 
+  // tile t as the k-th of this CTA: one box (rows and columns outside the padded image read as zero)
+  auto load = [&](long long t, long long k) {
+    int x0, y0, b;
+    conv_tile(a, t, x0, y0, b);
+    const int s = (int)(k % S);
+    mbar_expect_tx(full0 + 8 * s, kIn * rs);
+    tma_load_5d(stage0 + s * a.stage_bytes, &mbox, 0, x0 / 8, 0, y0, b, full0 + 8 * s);
+  };
+  long long issued = 0;  // thread 0: tiles loaded
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int s = 0; s < S; ++s) {
@@ -135,6 +149,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     }
     mbar_init(mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // the first tiles' loads under the set-up that follows
+    for (; issued < S && blockIdx.x + issued * gridDim.x < a.n_tiles; ++issued)
+      load(blockIdx.x + issued * gridDim.x, issued);
   }
   if (PLANES == 1)
     for (uint32_t i = threadIdx.x * 16; i < kConvZero; i += kConvThreads * 16)
@@ -168,20 +185,16 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   tc_fence_after();
 
   if (warp == 0) {
-    // producer: one box per tile (rows and columns outside the padded image read as zero)
+    // producer: the tiles past the first S
     if (lane == 0) {
-      long long k = 0;
-      for (long long t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++k) {
-        int x0, y0, b;
-        conv_tile(a, t, x0, y0, b);
-        const int s = (int)(k % S);
-        if (k >= S && !mbar_wait(empty0 + 8 * s, (uint32_t)(((k / S) - 1) & 1))) {
+      long long k = issued;
+      for (long long t = blockIdx.x + k * gridDim.x; t < a.n_tiles; t += gridDim.x, ++k) {
+        if (!mbar_wait(empty0 + 8 * (int)(k % S), (uint32_t)(((k / S) - 1) & 1))) {
           atomicExch(&s_abort, 1);
           break;
         }
         if (conv_aborted(&s_abort)) break;
-        mbar_expect_tx(full0 + 8 * s, kConvIn * rs);
-        tma_load_5d(stage0 + s * a.stage_bytes, &mbox, 0, x0 / 8, 0, y0, b, full0 + 8 * s);
+        load(t, k);
       }
       if (conv_aborted(&s_abort))  // let copies in flight land before the CTA exits
         for (long long q = (k > S ? k - S : 0); q < k; ++q)
@@ -204,9 +217,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 #pragma unroll
         for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-          for (int r = 0; r < kConvIn; ++r) {
+          for (int r = 0; r < kIn; ++r) {
             // output rows j0 .. j1 take tap r - j of input row r
-            const int j0 = r < 2 ? 0 : r - 2, j1 = r < kConvRows ? r : kConvRows - 1, n = (j1 - j0 + 1) * kCo;
+            const int j0 = r < 2 ? 0 : r - 2, j1 = r < ROWS ? r : ROWS - 1, n = (j1 - j0 + 1) * kCo;
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
 #pragma unroll
             for (int h = 0; h < kHalves; ++h) {
@@ -225,9 +238,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     __syncwarp();
     if (!mbar_wait(mdone, 0)) atomicExch(&s_abort, 1);
   } else {
-    // epilogue: the two warps of quadrant q hold pixels 32 q .. + 31, a lane one pixel, four of the
+    // epilogue: the two warps of quadrant q hold pixels 32 q .. + 31, a lane one pixel, half of the
     // output rows each
-    constexpr int kRows = kConvRows / 2;
+    constexpr int kRows = ROWS / 2;
     const int px = (warp & 3) * 32 + lane, j0 = warp < 6 ? 0 : kRows;
     const uint32_t tl = (uint32_t)((warp & 3) * 32) << 16;
     float bias[EPI == kEpiRelu ? 32 : 1];
@@ -646,8 +659,8 @@ struct lct_cnn {
   __nv_bfloat16* d_wb = nullptr;  // 8 backward slots (slot 0 unused)
   // boxes of the convolutions' inputs and of the weight gradients; activations: [0] the network input,
   // [1 + i] buffer i
-  CUtensorMap m_in[kCnnLayers], m_dwa[kCnnLayers];
-  CUtensorMap m_zin[3], m_dwz[3];  // the same for the deltas
+  CUtensorMap m_in[kConvHeights][kCnnLayers], m_dwa[kCnnLayers];
+  CUtensorMap m_zin[kConvHeights][3], m_dwz[3];  // the same for the deltas
   __nv_bfloat16* d_in = nullptr;  // network input
   __nv_bfloat16* d_act = nullptr; // n_act activation buffers
   __nv_bfloat16* d_dz = nullptr;  // training: 3 delta buffers
@@ -670,13 +683,13 @@ static int in_map(const lct_cnn* c, int l) { return l == 0 ? 0 : 1 + out_buf(c, 
 
 // Boxes of the convolutions: bf16 [cap][H + 2][planes][wp / 8][8 pixels] as 8-byte elements, box
 // {8 pixels, px / 8 + 1 blocks, planes, rows, 1}.
-static int conv_map(CUtensorMap* m, __nv_bfloat16* base, const lct_cnn* c, int planes) {
+static int conv_map(CUtensorMap* m, __nv_bfloat16* base, const lct_cnn* c, int planes, int rows) {
   auto fn = tensor_map_encoder();
   if (!fn) return LCT_ERR_UNSUPPORTED;
   const size_t plane = (size_t)16 * c->wp, row = plane * planes, slice = row * (c->H + 2);
   cuuint64_t dims[5] = {16, (cuuint64_t)c->wp / 8, (cuuint64_t)planes, (cuuint64_t)(c->H + 2), (cuuint64_t)c->cap};
   cuuint64_t strides[4] = {128, plane, row, slice};
-  cuuint32_t box[5] = {16, (cuuint32_t)(c->n_px / 8 + 1), (cuuint32_t)planes, (cuuint32_t)kConvIn, 1};
+  cuuint32_t box[5] = {16, (cuuint32_t)(c->n_px / 8 + 1), (cuuint32_t)planes, (cuuint32_t)(rows + 2), 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, base, dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -720,30 +733,60 @@ static int conv_prepare(int dev) {
     return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
   };
   int st;
-  if ((st = attr(conv_tc_kernel<kEpiRelu, 1>))) return st;
-  if ((st = attr(conv_tc_kernel<kEpiRelu, 4>))) return st;
-  if ((st = attr(conv_tc_kernel<kEpiMask, 4>))) return st;
-  if ((st = attr(conv_tc_kernel<kEpiResid, 4>))) return st;
-  if ((st = attr(conv_tc_kernel<kEpiGate, 4>))) return st;
+  auto convs = [&](auto rows) {
+    constexpr int kRows = decltype(rows)::value;
+    if ((st = attr(conv_tc_kernel<kEpiRelu, 1, kRows>))) return st;
+    if ((st = attr(conv_tc_kernel<kEpiRelu, 4, kRows>))) return st;
+    if ((st = attr(conv_tc_kernel<kEpiMask, 4, kRows>))) return st;
+    if ((st = attr(conv_tc_kernel<kEpiResid, 4, kRows>))) return st;
+    return st = attr(conv_tc_kernel<kEpiGate, 4, kRows>);
+  };
+  if (convs(std::integral_constant<int, conv_rows(0)>{})) return st;
+  if (convs(std::integral_constant<int, conv_rows(1)>{})) return st;
+  if (convs(std::integral_constant<int, conv_rows(2)>{})) return st;
   if ((st = attr(cnn_dw_tc_kernel<1>))) return st;
   if ((st = attr(cnn_dw_tc_kernel<4>))) return st;
   done[dev] = true;
   return LCT_OK;
 }
 
-template <int EPI, int PLANES>
-static int launch_conv(const CUtensorMap& in, ConvArgs a, int B, int sms, cudaStream_t s) {
+template <int EPI, int PLANES, int ROWS>
+static int launch_conv_rows(const CUtensorMap& in, ConvArgs a, int B, int sms, cudaStream_t s) {
+  a.rows = ROWS;
+  a.tiles_y = (a.H + ROWS - 1) / ROWS;
   a.n_tiles = (long long)B * a.tiles_x * a.tiles_y;
   if (a.n_tiles <= 0) return LCT_OK;
-  a.stage_bytes = (kConvIn * PLANES * conv_plane(a.n_px) + 127) / 128 * 128;
+  a.stage_bytes = ((ROWS + 2) * PLANES * conv_plane(a.n_px) + 127) / 128 * 128;
   const bool last = EPI == kEpiResid || EPI == kEpiGate;
   const uint32_t fixed = (PLANES == 1 ? kConvZero : 0u) + 3u * (PLANES == 1 ? 1u : 2u) * 2u * 3u * (last ? 16u : 32u) * 16u;
   const uint32_t tail = 128 * 16;  // an operand of the last plane may read this far past it
   a.stages = std::min<int>(kConvMaxStages, (int)((kSmemMax - fixed - tail) / a.stage_bytes));
   const size_t smem = (size_t)a.stages * a.stage_bytes + fixed + tail;
   const unsigned grid = (unsigned)std::min<long long>(a.n_tiles, sms);  // tensor memory: one CTA per SM
-  conv_tc_kernel<EPI, PLANES><<<grid, kConvThreads, smem, s>>>(in, a);
+  conv_tc_kernel<EPI, PLANES, ROWS><<<grid, kConvThreads, smem, s>>>(in, a);
   return launch_status();
+}
+
+// Height of the tiles: the fewest rows whose tiles are still one for each SM.  Such a launch is bound by one
+// tile's MMAs (60 in series for eight rows, 3.3 us; 36 for four; 24 of fewer columns for two, 1 us), not by
+// operand reads or the rows that neighbouring tiles both load; a second tile for some SMs costs more than it
+// saves (96^2 x 4 slices, 192 tiles of two rows: 84 us a forward pass, 80 with eight rows; two CTAs per SM no
+// better).  Forward pass of 8 layers, us, eight rows / the fewest: 64^2 x 4 slices 79 / 65, 128^2 80 / 66,
+// 96^2 x 4 80 / 72.  The same values: a pixel's taps add in the same order.
+static int conv_height(const ConvArgs& a, int B, int sms) {
+  int h = kConvHeights - 1;
+  while (h > 0 && (long long)B * a.tiles_x * ((a.H + conv_rows(h) - 1) / conv_rows(h)) > sms) --h;
+  return h;
+}
+
+// in(height): the input's boxes for tiles of that height
+template <int EPI, int PLANES, class Boxes>
+static int launch_conv(Boxes in, const ConvArgs& a, int B, int sms, cudaStream_t s) {
+  switch (conv_height(a, B, sms)) {
+    case 2: return launch_conv_rows<EPI, PLANES, conv_rows(2)>(in(2), a, B, sms, s);
+    case 1: return launch_conv_rows<EPI, PLANES, conv_rows(1)>(in(1), a, B, sms, s);
+    default: return launch_conv_rows<EPI, PLANES, conv_rows(0)>(in(0), a, B, sms, s);
+  }
 }
 
 static ConvArgs conv_args(const lct_cnn* c) {
@@ -752,9 +795,7 @@ static ConvArgs conv_args(const lct_cnn* c) {
   a.W = c->W;
   a.wp = c->wp;
   a.n_px = c->n_px;
-  a.rows = kConvRows;
   a.tiles_x = (c->W + a.n_px - 1) / a.n_px;
-  a.tiles_y = (c->H + kConvRows - 1) / kConvRows;
   a.status = device_status_ptr();
   return a;
 }
@@ -781,7 +822,7 @@ static int run_hidden(lct_cnn* c, int B, cudaStream_t s) {
     a.bias = c->d_p + cnn_off(l) + cnn_cin(l) * cnn_cout(l) * 9;
     a.w = c->d_wf + (size_t)l * kWSlot;
     a.out_act = act_buf(c, out_buf(c, l));
-    const CUtensorMap& in = c->m_in[in_map(c, l)];
+    auto in = [&, m = in_map(c, l)](int h) -> const CUtensorMap& { return c->m_in[h][m]; };
     st = l == 0 ? launch_conv<kEpiRelu, 1>(in, a, B, c->sms, s) : launch_conv<kEpiRelu, 4>(in, a, B, c->sms, s);
     if (st) return st;
   }
@@ -803,7 +844,7 @@ static int cnn_forward_impl(lct_cnn* c, const float* d_in5, int B, cudaStream_t 
   ConvArgs a;
   last_bias_and_args(c, a);
   a.out_f = c->d_r;
-  const CUtensorMap& in = c->m_in[in_map(c, kCnnLayers - 1)];
+  auto in = [&, m = in_map(c, kCnnLayers - 1)](int h) -> const CUtensorMap& { return c->m_in[h][m]; };
   return launch_conv<kEpiResid, 4>(in, a, B, c->sms, s);
 }
 
@@ -846,7 +887,8 @@ static int cnn_backward_impl(lct_cnn* c, const float* d_in5, const float* d_targ
     a.w = c->d_wb + (size_t)l * kWSlot;
     a.out_act = dz_buf(c, nxt);
     a.mask_act = act_buf(c, out_buf(c, l - 1));
-    if ((st = launch_conv<kEpiMask, 4>(c->m_zin[cur], a, B, c->sms, s))) return st;
+    auto in = [&](int h) -> const CUtensorMap& { return c->m_zin[h][cur]; };
+    if ((st = launch_conv<kEpiMask, 4>(in, a, B, c->sms, s))) return st;
     cur = nxt;
   }
   return LCT_OK;
@@ -951,11 +993,11 @@ LCT_API int lct_cnn_create(int max_slices, int ny, int nx, int flags, uint64_t s
   for (int i = 0; i <= c->n_act && !st; ++i) {  // i = 0: the network input
     __nv_bfloat16* p = i == 0 ? c->d_in : act_buf(c, i - 1);
     const int planes = i == 0 ? 1 : 4;
-    st = conv_map(&c->m_in[i], p, c, planes);
+    for (int h = 0; h < kConvHeights && !st; ++h) st = conv_map(&c->m_in[h][i], p, c, planes, conv_rows(h));
     if (!st && c->train) st = act_map(&c->m_dwa[i], p, c, planes, c->dw_px + 2, kDwRows + 2, false);
   }
   for (int i = 0; i < 3 && !st && c->train; ++i) {
-    st = conv_map(&c->m_zin[i], dz_buf(c, i), c, 4);
+    for (int h = 0; h < kConvHeights && !st; ++h) st = conv_map(&c->m_zin[h][i], dz_buf(c, i), c, 4, conv_rows(h));
     if (!st) st = act_map(&c->m_dwz[i], dz_buf(c, i), c, 4, c->dw_px, kDwRows, true);
   }
   if (!st) {
@@ -1091,7 +1133,7 @@ int cnn_infer_range(lct_cnn* c, const float* d_vol, float* d_out, int nz, int z0
     a.inv_scale = 1.f / c->in_scale;
     a.bound = bound;
     a.n_reject = c->d_rej;
-    const CUtensorMap& in = c->m_in[in_map(c, kCnnLayers - 1)];
+    auto in = [&, m = in_map(c, kCnnLayers - 1)](int h) -> const CUtensorMap& { return c->m_in[h][m]; };
     st = launch_conv<kEpiGate, 4>(in, a, B, c->sms, s);
   }
   return st;
