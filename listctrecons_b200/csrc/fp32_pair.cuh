@@ -35,12 +35,13 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
   return r;
 }
 
-// x / d rounded to nearest for a launch-constant d with r = RN(1 / d): the quotient estimate's
-// remainder is exact in an FMA and one more FMA rounds correctly (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34(1), 1990), except
-// that a divisor whose fraction bits are all ones may leave a power of two one ulp off; 3
-// operations where a division by a variable is a subroutine.  tests/test_div_by.py compares every
-// fraction of x with the division.
+// x / d rounded to nearest where r = RN(1 / d) is at hand (a constant of the launch, or one per view): the
+// quotient estimate's remainder is exact in an FMA and one more FMA rounds correctly (Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34(1), 1990), except that
+// a divisor whose fraction bits are all ones may leave a power of two one ulp off; 3 operations where a
+// division by a variable is a subroutine.  For normal numbers: d = 0 and an infinite quotient give NaN.
+// tests/test_div_by_kernel.py compiles these functions and compares every fraction of x, constant divisors and
+// varying ones, with the division.
 __device__ __forceinline__ float div_by(float x, float d, float r) {
   const float q = __fmul_rn(x, r);
   return fmaf(fmaf(-q, d, x), r, q);
