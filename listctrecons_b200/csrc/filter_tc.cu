@@ -383,7 +383,7 @@ static int tc_filter_p(int ns, float* d_rows, long long nrows, void* scratch, cu
   const long long mt = (nrows + kTcM - 1) / kTcM;
   if (mt > 65535) return LCT_ERR_ARG;
   __nv_bfloat16* b = static_cast<__nv_bfloat16*>(scratch);
-  __nv_bfloat16* a = b + (size_t)P * kp * kp;  // 16-byte aligned: kp is a multiple of 8
+  __nv_bfloat16* a = b + (size_t)P * kp * kp;  // 64-byte aligned: kp is a multiple of 32
   if (ns % 4 == 0 && reinterpret_cast<uintptr_t>(d_rows) % 16 == 0 &&
       reinterpret_cast<uintptr_t>(a) % 8 == 0)
     split_rows4_kernel<P><<<(unsigned)((nrows + kSplitRows - 1) / kSplitRows), 256, 0, s>>>(

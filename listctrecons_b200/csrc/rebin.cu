@@ -493,7 +493,7 @@ LCT_API int lct_rebin_null(const lct_geom* g, const float* d_fan, float* d_par, 
 // TEX8 PI-original rebin through the texture unit, as the reference samples it
 // (CUDA/Rebiner.cu:156-179): all three coordinates off texel centres, so the unit's trilinear
 // filter -- which register emulation matches only to within two 8-bit weight steps -- is used
-// itself.  Coordinates as in rebin_pi_ori_kernel's TEX8 branch.
+// itself.  Coordinates: the reference's FP32 expressions.
 __global__ void __launch_bounds__(256) rebin_pi_ori_tex_kernel(cudaTextureObject_t tex,
                                                                float* __restrict__ par, RebinArgs a) {
   const int ia = blockIdx.x, it = blockIdx.y;

@@ -76,8 +76,8 @@ __device__ double noisy_integral(double p, double i0, uint64_t seed, uint64_t id
 // evaluated per ray 8.4 ms.
 // A launch that leaves the chip's CTA slots empty is bound by one thread's time instead: it takes ROWS = 4
 // rows per thread, or 1.  One view x 16 x 736: 67 us with 16 rows per thread, 20 with 1 (one ray per thread
-// with everything evaluated per ray 39).  A row is a step
-// from its 16's first row in any of them, so its value does not depend on the launch.
+// with everything evaluated per ray 39).  A row is a step from its 16's first row in any of them, so its
+// value does not depend on the launch.
 constexpr int kSimRows = 16;     // rows whose quadratics share a base
 constexpr int kSimThreads = 128; // columns per CTA
 constexpr int kSimCtas = 5;      // CTAs per SM
