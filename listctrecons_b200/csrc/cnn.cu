@@ -723,33 +723,6 @@ static int tile_px(int W, int most, int step) {
   return ((W + tiles - 1) / tiles + step - 1) / step * step;
 }
 
-static int conv_prepare(int dev) {
-  static std::mutex mu;  // host threads may create workspaces on one device together
-  static bool done[64] = {false};
-  if (dev < 0 || dev >= 64) return LCT_ERR_UNSUPPORTED;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done[dev]) return LCT_OK;
-  auto attr = [](auto kernel) {
-    return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
-  };
-  int st;
-  auto convs = [&](auto rows) {
-    constexpr int kRows = decltype(rows)::value;
-    if ((st = attr(conv_tc_kernel<kEpiRelu, 1, kRows>))) return st;
-    if ((st = attr(conv_tc_kernel<kEpiRelu, 4, kRows>))) return st;
-    if ((st = attr(conv_tc_kernel<kEpiMask, 4, kRows>))) return st;
-    if ((st = attr(conv_tc_kernel<kEpiResid, 4, kRows>))) return st;
-    return st = attr(conv_tc_kernel<kEpiGate, 4, kRows>);
-  };
-  if (convs(std::integral_constant<int, conv_rows(0)>{})) return st;
-  if (convs(std::integral_constant<int, conv_rows(1)>{})) return st;
-  if (convs(std::integral_constant<int, conv_rows(2)>{})) return st;
-  if ((st = attr(cnn_dw_tc_kernel<1>))) return st;
-  if ((st = attr(cnn_dw_tc_kernel<4>))) return st;
-  done[dev] = true;
-  return LCT_OK;
-}
-
 template <int EPI, int PLANES, int ROWS>
 static int launch_conv_rows(const CUtensorMap& in, ConvArgs a, int B, int sms, cudaStream_t s) {
   a.rows = ROWS;
@@ -771,8 +744,8 @@ static int launch_conv_rows(const CUtensorMap& in, ConvArgs a, int B, int sms, c
 // tile's MMAs (60 in series for eight rows, 3.3 us; 36 for four; 24 of fewer columns for two, 1 us), not by
 // operand reads or the rows that neighbouring tiles both load; a second tile for some SMs costs more than it
 // saves (96^2 x 4 slices, 192 tiles of two rows: 84 us a forward pass, 80 with eight rows; two CTAs per SM no
-// better).  Forward pass of 8 layers, us, eight rows / the fewest: 64^2 x 4 slices 79 / 65, 128^2 80 / 66,
-// 96^2 x 4 80 / 72.  The same values: a pixel's taps add in the same order.
+// better).  Forward pass of 8 layers as a program calls it, us, eight rows / the fewest: 64^2 x 4 slices
+// 79 / 65, 128^2 80 / 66 (in a graph 58 / 39, the loads' overlap included), 96^2 x 4 80 / 72.  The same values: a pixel's taps add in the same order.
 static int conv_height(const ConvArgs& a, int B, int sms) {
   int h = kConvHeights - 1;
   while (h > 0 && (long long)B * a.tiles_x * ((a.H + conv_rows(h) - 1) / conv_rows(h)) > sms) --h;
@@ -798,6 +771,40 @@ static ConvArgs conv_args(const lct_cnn* c) {
   a.tiles_x = (c->W + a.n_px - 1) / a.n_px;
   a.status = device_status_ptr();
   return a;
+}
+
+template <int ROWS>
+static int conv_attributes() {
+  auto attr = [](auto kernel) {
+    return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+  };
+  int st;
+  if ((st = attr(conv_tc_kernel<kEpiRelu, 1, ROWS>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiRelu, 4, ROWS>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiMask, 4, ROWS>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiResid, 4, ROWS>))) return st;
+  if ((st = attr(conv_tc_kernel<kEpiGate, 4, ROWS>))) return st;
+  if ((st = attr(cnn_dw_tc_kernel<1>))) return st;
+  return attr(cnn_dw_tc_kernel<4>);
+}
+
+// attributes (which load a kernel) of the tile heights that passes of 1 .. cap slices take
+static int conv_prepare(const lct_cnn* c) {
+  static std::mutex mu;  // host threads may create workspaces on one device together
+  static unsigned long long done[64][kConvHeights] = {};  // the context they are set in, plus one
+  if (c->device < 0 || c->device >= 64) return LCT_ERR_UNSUPPORTED;
+  const unsigned long long ctx = context_id() + 1;
+  const ConvArgs a = conv_args(c);
+  std::lock_guard<std::mutex> lock(mu);
+  for (int h = conv_height(a, c->cap, c->sms); h <= conv_height(a, 1, c->sms); ++h) {
+    if (done[c->device][h] == ctx) continue;
+    const int st = h == 0   ? conv_attributes<conv_rows(0)>()
+                   : h == 1 ? conv_attributes<conv_rows(1)>()
+                            : conv_attributes<conv_rows(2)>();
+    if (st) return st;
+    done[c->device][h] = ctx;
+  }
+  return LCT_OK;
 }
 
 static int run_pack(lct_cnn* c, cudaStream_t s) {
@@ -968,7 +975,7 @@ LCT_API int lct_cnn_create(int max_slices, int ny, int nx, int flags, uint64_t s
   c->act_elems = (long long)max_slices * (ny + 2) * wp * kCnnC;
   int st = cuda_status(cudaGetDevice(&c->device));
   if (!st) st = cuda_status(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device));
-  if (!st) st = conv_prepare(c->device);
+  if (!st) st = conv_prepare(c);
   if (!st) st = cuda_status(cudaMalloc(&c->d_p, sizeof(float) * 4 * kCnnParams));
   if (!st) {
     c->d_g = c->d_p + kCnnParams;
