@@ -736,7 +736,7 @@ LCT_API int lct_backproject_par(const lct_geom* g, const lct_img* ig, const floa
     float4* q = nullptr;
     const size_t bytes = sizeof(float4) * (size_t)g->n_angle * quad_view_elems(g->ns, g->nt);
     if ((st = scratch_alloc((void**)&q, bytes, s))) return LCT_ERR_ALLOC;
-    st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, interp, q, s);
+    st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, q, s);
     if (!st) {
       BpLaunch L;
       L.proj = d_proj;

@@ -66,7 +66,7 @@ LCT_API int lct_backproject_par_noalloc(const lct_geom* g, const lct_img* ig,
   float4* q = nullptr;
   if ((st = noalloc_scratch(&q))) return st;
   cudaStream_t s = (cudaStream_t)stream;
-  if ((st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, interp, q, s))) return st;
+  if ((st = launch_quad_pack(d_proj, g->n_angle, g->ns, g->nt, addr, q, s))) return st;
   BpLaunch L;
   L.proj = d_proj;
   L.betas = d_betas;

@@ -13,8 +13,8 @@
 //   * views whose window covers every slice of the thread's chunk run an unpredicated loop.
 // EXACT keeps FP64 view trigonometry and full FP32 weights; TEX8 keeps the reference's order
 // for the sample column (phat/dso, theta*dso/ds) and the texture unit's 8-bit weight rules, bit
-// for bit, in the same packed path: divisions by launch constants as three FMAs, 8-bit weights as
-// whole numbers from round-down adds (256^2 x 32 from 672 x 16 views: 4.05 ms, 5.13 ms in scalar
+// for bit, in the same packed path: divisions by launch constants as three FMAs, 8-bit weights on
+// their own grid from round-down adds (256^2 x 32 from 672 x 16 views: 4.05 ms, 5.13 ms in scalar
 // code with IEEE divisions, FRND and F2I).
 // Both: floor, fraction and index of a sample from one round-down add (no conversions)
 // and one wide multiply-add for its address; per-view terms staged in shared memory 128 views
@@ -93,9 +93,7 @@ struct BpQuadArgs {
 
 // quad pack: grid (views, nt + 3), block 256 over the ns + 3 quad columns; view v goes to slot
 // (vbase + v) mod ring of a ring of quads (ring > 0), else to view v
-// TEX8: the row differences carry a factor 2^-8 (exact), so the samples' 8-bit row weights stay
-// whole numbers
-template <int ADDR, int INTERP>
+template <int ADDR>
 __global__ void __launch_bounds__(256) quad_pack_kernel(const float* __restrict__ rows, int ns,
                                                         int nt, float4* __restrict__ quads,
                                                         long long vbase, long long ring) {
@@ -119,26 +117,20 @@ __global__ void __launch_bounds__(256) quad_pack_kernel(const float* __restrict_
                 t11 = texel(j + 1, i + 1);
     // differences {T00, dy, dx, dxy}: a bilinear sample is then T00 + a dx + b (dy + a dxy), the
     // pair (T00, dy) + a (dx, dxy) one packed FMA
-    constexpr float kRow = INTERP == LCT_INTERP_TEX8 ? 1.0f / 256.0f : 1.0f;
-    out[q] = make_float4(t00, kRow * (t10 - t00), t01 - t00, kRow * ((t11 - t10) - (t01 - t00)));
+    out[q] = make_float4(t00, t10 - t00, t01 - t00, (t11 - t10) - (t01 - t00));
   }
 }
 
-int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, int interp,
-                     float4* quads, cudaStream_t s, long long vbase, long long ring) {
+int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, float4* quads,
+                     cudaStream_t s, long long vbase, long long ring) {
   if (views <= 0) return LCT_OK;
   if (views > 0x7fffffffLL || nt + 3 > 65535 || vbase < 0 || ring < 0) return LCT_ERR_ARG;
   if (ring > 0 && views > ring) return LCT_ERR_ARG;  // a piece would overwrite itself
   dim3 grid((unsigned)views, nt + 3);
-  const bool tex = interp == LCT_INTERP_TEX8, clamp = addr == LCT_ADDR_CLAMP;
-  if (tex && clamp)
-    quad_pack_kernel<LCT_ADDR_CLAMP, LCT_INTERP_TEX8><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
-  else if (tex)
-    quad_pack_kernel<LCT_ADDR_BORDER, LCT_INTERP_TEX8><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
-  else if (clamp)
-    quad_pack_kernel<LCT_ADDR_CLAMP, LCT_INTERP_EXACT><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
+  if (addr == LCT_ADDR_CLAMP)
+    quad_pack_kernel<LCT_ADDR_CLAMP><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
   else
-    quad_pack_kernel<LCT_ADDR_BORDER, LCT_INTERP_EXACT><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
+    quad_pack_kernel<LCT_ADDR_BORDER><<<grid, 256, 0, s>>>(rows, ns, nt, quads, vbase, ring);
   return launch_status();
 }
 
@@ -437,10 +429,10 @@ __device__ __forceinline__ void bp_quad_tile(const BpQuadArgs& A, int bx, int by
           }
           // texture unit: w01 = a - w11, w10 = b - w11, w00 = 1 - a - b + w11, so the sample is
           // T00 + a dx + b dy + w11 dxy with b = round-half-up of the fraction and w11 =
-          // round-half-up(a b), both on the 1/256 grid: B = 256 b and W = 256 w11 are the whole
-          // parts of exact sums (the quads' row differences carry the 1/256)
-          const float2 B = __fadd2_rn(__fadd2_rd(__ffma2_rn(b, f2(256.0f), f2(0.5f)), f2(kFloorMagic)), f2(-kFloorMagic));
-          const float2 W = __fadd2_rn(__fadd2_rd(__ffma2_rn(make_float2(a1, a2), B, f2(0.5f)), f2(kFloorMagic)), f2(-kFloorMagic));
+          // round-half-up(a b), both on the 1/256 grid, which is where a round-down add of
+          // 1.5 * 2^15 leaves an exact sum
+          const float2 B = __fadd2_rn(__fadd2_rd(__fadd2_rn(b, f2(kHalfStep8)), f2(kFloorMagic8)), f2(-kFloorMagic8));
+          const float2 W = __fadd2_rn(__fadd2_rd(__ffma2_rn(make_float2(a1, a2), B, f2(kHalfStep8)), f2(kFloorMagic8)), f2(-kFloorMagic8));
           const float s1 = fmaf(W.x, v0.w, fmaf(B.x, v0.y, fmaf(a1, v0.z, v0.x)));
           const float s2 = fmaf(W.y, v1.w, fmaf(B.y, v1.y, fmaf(a2, v1.z, v1.x)));
           sum = fmaf(w1, s1, fmaf(w2, s2, acc[j]));

@@ -20,6 +20,9 @@ __device__ __forceinline__ float2 f2sub(float2 x, float2 y) {
 // range the bit pattern still orders like x, so a clamp on it clamps floor(x).
 constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kFloorBits = 0x4B400000;
+// the same for the 1/256 grid of 8-bit weights, |x| < 2^14, and half a step of it
+constexpr float kFloorMagic8 = 49152.0f;  // 1.5 * 2^15
+constexpr float kHalfStep8 = 1.0f / 512.0f;
 
 // The hardware's approximate reciprocal and reciprocal square root without the scaling that the
 // general forms wrap around them for subnormal and huge arguments (distances and row differences are

@@ -97,9 +97,8 @@ LCT_HD inline long long quad_cols(int ns) { return (long long)ns + 3; }
 LCT_HD inline long long quad_view_elems(int ns, int nt) { return (long long)(nt + 3) * (ns + 3); }
 // ring > 0: quads is a ring of `ring` views and rows view v is packed into slot
 // (vbase + v) mod ring; 0: into view v.
-// interp: TEX8 quads hold their row differences (dy, dxy) times 2^-8.
-int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, int interp,
-                     float4* quads, cudaStream_t s, long long vbase = 0, long long ring = 0);
+int launch_quad_pack(const float* rows, long long views, int ns, int nt, int addr, float4* quads,
+                     cudaStream_t s, long long vbase = 0, long long ring = 0);
 // Slices whose EXACT row coordinates are steps from one base (the first of them): 8, or 4 where few are
 // active together, however few a thread takes -- a slice's rounding then depends on neither the image's
 // size nor the split.

@@ -486,8 +486,8 @@ int recon_pack(lct_recon* r, const float* par, long long nv, long long v0, int a
   const lct_geom& g = r->info.ctg;
   if (r->tex_bp) return view_texture_fill(r->vtex, par, nv, v0, s);
   if (r->quad_ring > 0)
-    return launch_quad_pack(par, nv, g.ns, g.nt, addr, r->o.interp, r->d_quad, s, v0, r->quad_ring);
-  return launch_quad_pack(par, nv, g.ns, g.nt, addr, r->o.interp, r->d_quad + v0 * quad_view_elems(g.ns, g.nt), s);
+    return launch_quad_pack(par, nv, g.ns, g.nt, addr, r->d_quad, s, v0, r->quad_ring);
+  return launch_quad_pack(par, nv, g.ns, g.nt, addr, r->d_quad + v0 * quad_view_elems(g.ns, g.nt), s);
 }
 
 int recon_bp_pairs(lct_recon* r, BpLaunch& L, cudaStream_t s) {
