@@ -494,9 +494,7 @@ __global__ void __launch_bounds__(kPiTX* kPiTY, 4) bp_pi_ori_z_kernel(const __gr
       const float* p = w.p0 + (long long)(__float_as_int(row) - kFloorBits) * A.ns;
       const float* q = p + A.ns;
       const float v00 = __ldg(p), v01 = __ldg(p + 1), v10 = __ldg(q), v11 = __ldg(q + 1);
-      if (INTERP == LCT_INTERP_TEX8) return blend<INTERP>(w.c.a, bb, v00, v01, v10, v11);
-      const float top = fmaf(w.c.a, v01 - v00, v00), bot = fmaf(w.c.a, v11 - v10, v10);
-      return fmaf(bb, bot - top, top);
+      return blend<INTERP>(w.c.a, bb, v00, v01, v10, v11);
     };
     sum[j] += sample(m.x, b.x);
     sum[j + 1] += sample(m.y, b.y);
